@@ -37,6 +37,7 @@ struct CountParams {
     int nidx;
     const float4* mpts[kMaxFused];
     const uint32_t* mcs[kMaxFused];
+    uint32_t mn[kMaxFused];  // particles of each index
 };
 
 __device__ __forceinline__ float edge_margin(float v) { return 1e-3f + 2e-6f * fabsf(v); }
@@ -100,16 +101,17 @@ __device__ __forceinline__ Image make_image(const CountParams& p, float cx, floa
     return im;
 }
 
-template <int BIN, bool BIG>
+// ZONE: only distances >= zone_lo are counted.
+template <int BIN, bool BIG, bool ZONE = false>
 __device__ __forceinline__ void test_candidate(const CountParams& p, const Image& im, const float4 pp, bool live,
                                                uint32_t* __restrict__ sink, const float* __restrict__ tab,
-                                               const uint32_t* __restrict__ lut) {
+                                               const uint32_t* __restrict__ lut, float zone_lo = 0.0f) {
     const bool inb = !(pp.x < im.lox) & !(im.hix < pp.x) & !(pp.y < im.loy) & !(im.hiy < pp.y) &
                      !(pp.z < im.loz) & !(im.hiz < pp.z);
     const float dx = __fsub_rn(pp.x, im.cx), dy = __fsub_rn(pp.y, im.cy), dz = __fsub_rn(pp.z, im.cz);
     const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
     if (BIN != BIN_FIRST_MATCH) {
-        if (live && inb && dist < p.r2max) atomicAdd(sink + bin_of<BIN>(p, tab, lut, dist), 1u);
+        if (live && inb && dist < p.r2max && (!ZONE || dist >= zone_lo)) atomicAdd(sink + bin_of<BIN>(p, tab, lut, dist), 1u);
     } else if (live && inb) {
         for (int i = 0; i < p.nrads; ++i) {
             if (dist < tab[i]) {
@@ -160,11 +162,11 @@ __device__ __forceinline__ void run_rows(const CountParams& p, const Image& im, 
 // contiguous share [total*part/nparts, total*(part+1)/nparts) of the
 // flattened candidate sequence, so nparts warps sharing a halo split every
 // row set evenly and together test each candidate once.
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool ZONE = false>
 __device__ __forceinline__ void run_rows_part(const CountParams& p, const Image& im, uint32_t start, uint32_t end,
                                               uint32_t* __restrict__ sink, const float* __restrict__ tab,
                                               const uint32_t* __restrict__ lut, int lane, uint32_t part,
-                                              uint32_t nparts) {
+                                              uint32_t nparts, float zone_lo = 0.0f) {
     const uint32_t len = end - start;
     uint32_t incl = len;
 #pragma unroll
@@ -191,8 +193,8 @@ __device__ __forceinline__ void run_rows_part(const CountParams& p, const Image&
         const bool l0 = t0 < te, l1 = t1 < te;
         const float4 p0 = l0 ? __ldg(p.pts + (t0 + o0)) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 p1 = l1 ? __ldg(p.pts + (t1 + o1)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        test_candidate<BIN, BIG>(p, im, p0, l0, sink, tab, lut);
-        test_candidate<BIN, BIG>(p, im, p1, l1, sink, tab, lut);
+        test_candidate<BIN, BIG, ZONE>(p, im, p0, l0, sink, tab, lut, zone_lo);
+        test_candidate<BIN, BIG, ZONE>(p, im, p1, l1, sink, tab, lut, zone_lo);
     }
 }
 

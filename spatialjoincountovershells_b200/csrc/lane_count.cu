@@ -1,0 +1,626 @@
+// Periodic multi-shell count of grid indexes with one lane per halo.
+//
+// k_lane_count   32 halos of the Morton order per warp, one per lane.  A lane
+//                plans its box's rows of cells (at most 5 x 5), clips each in x
+//                to the sphere, fetches the rows' slot ranges and then walks
+//                its own candidates one by one; its counts go to a private
+//                column of 16-bit counters in shared memory (no atomics) and
+//                from there to the halo's row.  Shifted periodic images wait
+//                in a per-warp list until there are 32 of them and are then
+//                walked the same way.
+// k_listed_count what does not suit a lane: images of more than 25 rows, and
+//                lanes with so many candidates that the rest of the warp
+//                would wait.  k_lane_count lists them; here a warp takes an
+//                item (or a part of a large one), reads its rows in windows
+//                of 32 slots and counts in 32-bit columns, one per lane.
+//
+// A candidate costs one float4 load, the eight fp32 operations of the
+// reference's distance, one lookup and one counter update; the box test and
+// the compare with r2max are gone from the loop.  The lookup word of the
+// distance's bit pattern (sjcs_query::LaneTable) carries into the shell index
+// exactly when the distance has reached the slot's threshold, everything from
+// safe2 on lands in one spare counter, and below safe2 the box test cannot
+// fail.  The few candidates between safe2 and r2max (about 0.4 % of halos at
+// R = 5 meet one) are tested literally: the walk keeps the least key -
+// zone0, and a halo that met the zone is listed again for it alone.
+//
+// Why lanes walk their own rows: mapping 32 lanes onto one halo's ~21 rows of
+// ~5 candidates cost a five-step shuffle search per window and shared-memory
+// atomics on the few shells that hold most of the volume, 484-559 warp
+// instructions per halo and file; this form takes about 235.  The price is a
+// gather of 32 addresses per load, but an L1 gather of 32 x 16 bytes takes
+// 11.0 cycles per SM against 5.2 coalesced and 9.2 from shared memory (random
+// slots, measured), so staging the candidates would not pay.  What bounds it:
+// the L1/shared data pipe (81 % of its peak, 47 % issue active).
+//
+// Measured (B200, count kernels of one call, before -> after): 1e7 uniform
+// halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.32 ms; 1e6 on 1e7 0.42 ->
+// 0.21; 1e6 clustered halos on 3e7 clustered particles 9.2 (static schedule)
+// and 7.1 (queue) -> 4.3; 1e6 on 5e7, R = 20, 64 shells 55 and 40.8 -> 24.6;
+// 1e5 on 2e7, R = 10 2.14 and 1.45 -> 0.94.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "grid_rows.cuh"
+#include "lane_count.cuh"
+
+namespace sjcs {
+namespace {
+
+using namespace count;
+
+// One block of 16 warps per SM: its warps take neighbouring batches and share
+// their particle lines in L1 (4.32 ms at 1e8 x 1e7; two blocks of 8 warps 4.68,
+// four of 4 5.08; 14 warps 4.46, 20 warps 4.84: more counters, less L1).
+constexpr int LN_WARPS = 16;
+constexpr int LN_ROWS = 25;       // rows of cells a lane walks
+constexpr uint32_t LN_PEND = 96;  // shifted images waiting per warp
+constexpr int LN_DEPTH = 4;       // candidates in flight per lane (2: 4.42 ms, 3: 4.35, 6: 4.34)
+constexpr int HV_WARPS = 4, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 6;
+// Items above this many candidates (in the box's rows) are split into at
+// least 8 parts: one warp would need longer than the rest of the pass.
+// 16384 and 32768 were slower (clustered R = 20: 32.3 and 30.7 against 29.9 ms).
+constexpr uint32_t kHuge = 65536;
+constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles on this path
+// Mean row length from which listed rows are read one by one; shorter rows
+// are flattened first (14: 3 % slower, 24 and 64: within 1 %).
+constexpr uint32_t kLongRow = 40;
+// Work of a lane's step for the whole warp, of 32 listed candidates and of a
+// listed item, in cycles of the data pipe: decides which lanes are listed.
+constexpr uint32_t kStepCost = 26, kWindowCost = 9, kItemCost = 100;
+
+struct LaneParams {
+    const uint32_t* __restrict__ slots;  // the fields of sjcs_query::LaneTable
+    int nslots, kbase, shift, ncol;
+    float safe2, cmax;
+    int khi;               // last key of the slots less kbase
+    uint32_t mask;         // (1 << shift) - 1
+    uint32_t zone0, zone;  // bit pattern of safe2; that of r2max less it
+    // Items: the huge ones from the front of the list, the others from its end.
+    uint2* __restrict__ list;  // (halo, flags)
+    uint32_t cap;
+    uint32_t* __restrict__ ctl;  // [0] items asked for, [1] huge, [2] others, [3] claims
+};
+
+// An item's flags: bits 0-2 the shifted axes, bits 3-6 the indexes to count.
+constexpr uint32_t kItemZone = 1u << 7;  // only distances from safe2 on
+constexpr uint32_t kItemFar = 1u << 8;   // centre beyond cmax: literal test throughout
+
+// Shared memory of one warp beside its counters.
+struct LaneRows {
+    uint32_t s0[LN_ROWS + 2][32];   // first slot of a lane's row
+    uint16_t len[LN_ROWS + 2][32];  // its candidates
+    uint32_t pend[LN_PEND];         // halo | shifted axes << 29
+};
+
+// A coordinate's periodic image: lo < 0 takes precedence (MultiRangeCount.c:38-43).
+__device__ __forceinline__ float shifted(float v, float half) {
+    return (__fsub_rn(v, half) < kBoxLow) ? __fadd_rn(v, kBoxUpp) : __fsub_rn(v, kBoxUpp);
+}
+
+// Axes on which the halo's box crosses a face.
+__device__ __forceinline__ uint32_t oob_flags(const CountParams& p, const float4 c) {
+    return ((__fsub_rn(c.x, p.half) < kBoxLow) | (__fadd_rn(c.x, p.half) > kBoxUpp) ? 1u : 0u) |
+           ((__fsub_rn(c.y, p.half) < kBoxLow) | (__fadd_rn(c.y, p.half) > kBoxUpp) ? 2u : 0u) |
+           ((__fsub_rn(c.z, p.half) < kBoxLow) | (__fadd_rn(c.z, p.half) > kBoxUpp) ? 4u : 0u);
+}
+
+// One lane counts one image by itself, straight into the count row: the way
+// out when the item list is full.
+__device__ __noinline__ void serial_count(const CountParams& p, float4 c, uint32_t flags, float safe2) {
+    const Image im = make_image(p, c.x, c.y, c.z);
+    uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
+    for (int f = 0; f < p.nidx; ++f) {
+        if (!((flags >> (3 + f)) & 1u)) continue;
+        for (int zz = im.z0; zz <= im.z1; ++zz)
+            for (int yy = im.y0; yy <= im.y1; ++yy) {
+                const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
+                const uint32_t e = p.mcs[f][rc + im.x1 + 1];
+                for (uint32_t j = p.mcs[f][rc + im.x0]; j < e; ++j) {
+                    const float4 v = p.mpts[f][j];
+                    if (flags & kItemZone)
+                        test_candidate<BIN_LUT, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
+                    else
+                        test_candidate<BIN_LUT, true>(p, im, v, true, row, p.r2, p.lut);
+                }
+            }
+    }
+}
+
+// Lanes with `push` add an item (h, flags) to the list; c is its centre.
+__device__ __forceinline__ void push_items(const CountParams& p, const LaneParams& q, bool push, bool huge, uint32_t h,
+                                           uint32_t flags, float4 c, int lane) {
+    const uint32_t all = __ballot_sync(0xffffffffu, push);
+    if (!all) return;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(q.ctl, (uint32_t)__popc(all));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const bool fits = push && base + (uint32_t)__popc(all & lt) < q.cap;
+    const uint32_t hb = __ballot_sync(0xffffffffu, fits && huge), ob = __ballot_sync(0xffffffffu, fits && !huge);
+    uint32_t at = 0;
+    if (lane < 2) {
+        const uint32_t k = (uint32_t)__popc(lane == 0 ? hb : ob);
+        if (k) at = atomicAdd(q.ctl + 1 + lane, k);
+    }
+    const uint32_t ah = __shfl_sync(0xffffffffu, at, 0), ao = __shfl_sync(0xffffffffu, at, 1);
+    if (fits) {
+        const uint32_t i = huge ? ah + (uint32_t)__popc(hb & lt) : q.cap - 1u - (ao + (uint32_t)__popc(ob & lt));
+        q.list[i] = make_uint2(h, flags);
+    }
+    if (push && !fits) serial_count(p, c, flags, q.safe2);
+}
+
+__global__ void __launch_bounds__(LN_WARPS * 32, 1)
+k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
+    extern __shared__ uint32_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    LaneRows* rows = reinterpret_cast<LaneRows*>(smem) + warp;
+    const int nwarps = (int)(blockDim.x >> 5);
+    uint32_t* cols32 = reinterpret_cast<uint32_t*>(reinterpret_cast<LaneRows*>(smem) + nwarps);
+    const int colwords = (q.ncol + 1) * 16;
+    uint32_t* slots = cols32 + nwarps * colwords;
+    cols32 += warp * colwords;
+    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols32) + 2 * lane;
+    for (int i = tid; i < q.nslots; i += (int)blockDim.x) slots[i] = q.slots[i];
+    for (int i = lane; i < colwords; i += 32) cols32[i] = 0u;
+    __syncthreads();
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t nbatch = (uint32_t)((p.nhalos + 31) / 32);
+    const uint32_t W = gridDim.x * (uint32_t)nwarps;
+    uint32_t b = blockIdx.x * (uint32_t)nwarps + (uint32_t)warp;
+    uint32_t npend = 0;
+    const float hmy = 0.5f * p.h[1] + 3e-3f, hmz = 0.5f * p.h[2] + 3e-3f;
+    const uint32_t plane_cells = (uint32_t)p.g.G[1] * (uint32_t)p.g.G[0];
+    const uint32_t files = ((1u << p.nidx) - 1u) << 3;
+    for (;;) {
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t h = 0, S = 0;
+        bool valid;
+        if (npend >= 32u || (b >= nbatch && npend)) {
+            // a batch of shifted images
+            const uint32_t take = min(npend, 32u);
+            npend -= take;
+            valid = (uint32_t)lane < take;
+            if (valid) {
+                const uint32_t it = rows->pend[npend + lane];
+                h = it & 0x1fffffffu;
+                S = it >> 29;
+                c = p.halos[h];
+                if (S & 1u) c.x = shifted(c.x, p.half);
+                if (S & 2u) c.y = shifted(c.y, p.half);
+                if (S & 4u) c.z = shifted(c.z, p.half);
+            }
+            __syncwarp();
+        } else if (b < nbatch) {
+            h = b * 32u + (uint32_t)lane;
+            b += W;
+            valid = h < p.nhalos;
+            if (valid) c = p.halos[h];
+            if (p.periodic) {
+                uint32_t F = valid ? oob_flags(p, c) : 0u;
+                uint32_t T = F;
+                for (;;) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, T != 0u);
+                    if (!bal) break;
+                    if (npend + (uint32_t)__popc(bal) <= LN_PEND) {
+                        if (T) rows->pend[npend + __popc(bal & lt)] = h | (T << 29);
+                        npend += __popc(bal);
+                    } else {
+                        float4 ci = c;
+                        if (T & 1u) ci.x = shifted(c.x, p.half);
+                        if (T & 2u) ci.y = shifted(c.y, p.half);
+                        if (T & 4u) ci.z = shifted(c.z, p.half);
+                        push_items(p, q, T != 0u, false, h, T | files, ci, lane);
+                    }
+                    T = T ? (T - 1u) & F : 0u;
+                }
+                __syncwarp();
+            }
+        } else {
+            break;
+        }
+        // a centre that is not finite has no finite distance: nothing to count
+        const bool fin = (c.x - c.x == 0.0f) & (c.y - c.y == 0.0f) & (c.z - c.z == 0.0f);
+        const bool far = !(fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)) <= q.cmax);
+        const Image im = make_image(p, c.x, c.y, c.z);
+        const bool mine = valid & fin & !far & (im.ny <= 5) & (im.nz <= 5);
+        uint32_t heavy = valid & fin & !mine ? files : 0u;  // files counted from the list
+        uint32_t hflag = far ? kItemFar : 0u, zoned = 0u;
+        uint32_t Tsum = 0u;
+        if (__any_sync(0xffffffffu, heavy != 0u)) {
+            // candidates of the box, to tell the items that must be split
+            if (heavy && im.nrows <= 400u) {
+                for (int zz = im.z0; zz <= im.z1; ++zz)
+                    for (int yy = im.y0; yy <= im.y1; ++yy) {
+                        const uint32_t rc = ((uint32_t)zz * (uint32_t)p.g.G[1] + (uint32_t)yy) * (uint32_t)p.g.G[0];
+                        Tsum += __ldg(p.mcs[0] + (rc + (uint32_t)im.x1 + 1u)) - __ldg(p.mcs[0] + (rc + (uint32_t)im.x0));
+                    }
+            } else if (heavy) {
+                Tsum = kHuge + 1u;
+            }
+            __syncwarp();
+        }
+        const int ny = mine ? im.ny : 0, nz = mine ? im.nz : 0;
+        const int nymax = __reduce_max_sync(0xffffffffu, ny), nzmax = __reduce_max_sync(0xffffffffu, nz);
+        // Row gaps as max(0, |cell middle - centre| - half a cell - margin), the
+        // centre clamped into the box (edge cells also hold what lies outside
+        // it).  The margin of 3e-3 is that of cell_gap at the far face.
+        const float ccy = fminf(fmaxf(c.y, 0.0f), kBoxUpp), ccz = fminf(fmaxf(c.z, 0.0f), kBoxUpp);
+        const float ybase = ((float)im.y0 + 0.5f) * p.h[1] - ccy, zbase = ((float)im.z0 + 0.5f) * p.h[2] - ccz;
+        constexpr int kMagicI = 0x4b400000;  // bits of 1.5 * 2^23: adding it rounds to an integer in the low bits
+        constexpr float kMagic = 12582912.0f;
+        const int ra = im.x0 + kMagicI, rz = im.x1 + kMagicI;
+        const float r2q = p.r2p + p.r2slack;
+        const float cxh = c.x - 0.5f * p.h[0];  // half a cell lower: rounding to nearest gives the end point's cell
+        const float xpad = 1e-3f + 1e-6f * fabsf(c.x);
+        const uint32_t rowc0 = ((uint32_t)im.z0 * (uint32_t)p.g.G[1] + (uint32_t)im.y0) * (uint32_t)p.g.G[0] - (uint32_t)kMagicI;
+        uint32_t walked = 0;  // candidates in the lane's 16-bit counters
+        for (int f = 0; f < p.nidx; ++f) {
+            const float4* __restrict__ pts = p.mpts[f];
+            const uint32_t* __restrict__ cs = p.mcs[f];
+            const uint32_t np = p.mn[f];
+            uint32_t T = 0, m = 0, win = 0;
+            bool wide = false;
+            for (int zi = 0; zi < nzmax; ++zi) {
+                const float gz = fmaxf(fabsf(__fmaf_rn((float)zi, p.h[2], zbase)) - hmz, 0.0f);
+                const float rz2 = r2q - gz * gz;
+                const uint32_t rowz = rowc0 + (uint32_t)zi * plane_cells;
+                uint32_t a[5], e[5];
+#pragma unroll
+                for (int u = 0; u < 5; ++u) {
+                    const float gy = fmaxf(fabsf(__fmaf_rn((float)u, p.h[1], ybase)) - hmy, 0.0f);
+                    const float rem = rz2 - gy * gy;
+                    a[u] = e[u] = 0u;
+                    if (rem >= 0.0f && u < ny && zi < nz) {
+                        // approximate square root: its error (< 1e-6 relative) is far inside the margin
+                        const float sq = rem * rsqrtf(fmaxf(rem, 1e-35f));
+                        const float xr = __fmaf_rn(sq, 1.0f + 2e-6f, xpad);
+                        const int xa = min(max(__float_as_int(__fmaf_rn(cxh - xr, p.g.inv_h[0], kMagic)), ra), rz);
+                        const int xb = min(max(__float_as_int(__fmaf_rn(cxh + xr, p.g.inv_h[0], kMagic)), ra), rz);
+                        const uint32_t row = rowz + (uint32_t)u * (uint32_t)p.g.G[0];
+                        a[u] = __ldg(cs + (row + (uint32_t)xa));
+                        e[u] = __ldg(cs + (row + (uint32_t)xb + 1u));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 5; ++u) {
+                    const uint32_t l = e[u] - a[u];
+                    if (l) {
+                        rows->s0[m][lane] = a[u];
+                        rows->len[m][lane] = (uint16_t)l;
+                        ++m;
+                        T += l;
+                        win += (l + 31u) >> 5;
+                        wide |= l > 65535u;
+                    }
+                }
+            }
+            // which lanes walk their own rows: the threshold with the least work
+            bool coop = wide | (T > 60000u) | (walked + T > 65000u);
+            uint32_t steps = __reduce_max_sync(0xffffffffu, coop ? 0u : T);
+            if (steps > 160u) {
+                const uint32_t mxT = steps;
+                const uint32_t hc = min(kWindowCost * win, T >> 1) + kItemCost;  // the lane's rows from the list
+                uint32_t best = kStepCost * mxT, tau = mxT;
+#pragma unroll
+                for (int k = 1; k < 5; ++k) {
+                    const uint32_t t = k == 4 ? 0u : mxT >> k;
+                    const bool over = !coop && T > t;
+                    const uint32_t st = __reduce_max_sync(0xffffffffu, (!coop && !over) ? T : 0u);
+                    const uint32_t cost = __reduce_add_sync(0xffffffffu, over ? hc : 0u) + kStepCost * st;
+                    if (cost < best) {
+                        best = cost;
+                        tau = t;
+                        steps = st;
+                    }
+                }
+                coop |= T > tau;
+            }
+            if (coop) {
+                heavy |= 8u << f;
+                Tsum += T;
+            } else {
+                walked += T;
+            }
+            if (steps) {
+                // the list ends in a row of slots past the particles, which load nothing
+                const uint32_t mm = coop ? 0u : m;
+                rows->s0[mm][lane] = kEndSlot;
+                rows->len[mm][lane] = 0xffffu;
+                uint32_t j = rows->s0[0][lane], e = j + rows->len[0][lane];
+                const uint32_t* rs = &rows->s0[1][lane];
+                const uint16_t* rl = &rows->len[1][lane];
+                uint32_t ns = *rs, nl = *rl;
+                uint32_t z = 0xffffffffu;  // least key - zone0 met
+                float4 buf[LN_DEPTH];
+                auto next = [&](float4& v) {
+                    v.x = INFINITY;
+                    if (j < np) v = __ldg(pts + j);
+                    ++j;
+                    if (j == e) {
+                        j = ns;
+                        e = ns + nl;
+                        rs += 32;
+                        rl += 32;
+                        ns = *rs;
+                        nl = *rl;
+                    }
+                };
+                auto test = [&](const float4& v) {
+                    const float dx = __fsub_rn(v.x, c.x), dy = __fsub_rn(v.y, c.y), dz = __fsub_rn(v.z, c.z);
+                    const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                    const uint32_t key = __float_as_uint(dist);
+                    z = __viaddmin_u32(key, 0u - q.zone0, z);
+                    const uint32_t t = (uint32_t)__viaddmin_s32_relu((int)key, -q.kbase, q.khi);
+                    const uint32_t w = slots[t >> q.shift] + (t & q.mask);
+                    uint16_t* cnt = reinterpret_cast<uint16_t*>(mycol + (w >> q.shift) * 64u);
+                    *cnt = (uint16_t)(*cnt + 1);
+                };
+#pragma unroll
+                for (int u = 0; u < LN_DEPTH; ++u) next(buf[u]);
+                for (uint32_t it = 0; it < steps; it += LN_DEPTH) {
+#pragma unroll
+                    for (int u = 0; u < LN_DEPTH; ++u) {
+                        test(buf[u]);
+                        next(buf[u]);
+                    }
+                }
+                if (z < q.zone) zoned |= 8u << f;
+            }
+        }
+        push_items(p, q, heavy != 0u, Tsum > kHuge, h, heavy | S | hflag, c, lane);
+        push_items(p, q, zoned != 0u, false, h, zoned | S | kItemZone, c, lane);
+        // the lanes' counters to their halos' rows
+        if (__any_sync(0xffffffffu, walked != 0u)) {
+            uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
+#pragma unroll 4
+            for (int sh = 0; sh < q.ncol; ++sh) {
+                const uint32_t v = *reinterpret_cast<uint16_t*>(mycol + sh * 64);
+                if (v) atomicAdd(row + sh, v);
+            }
+            __syncwarp();
+            for (int i = lane; i < colwords; i += 32) cols32[i] = 0u;
+            __syncwarp();
+        }
+    }
+}
+
+// Part `part` of `nparts` of a listed item (an even share of every 32 rows'
+// candidates).
+__device__ __forceinline__ void count_item(const CountParams& p, const LaneParams& q, const uint2 it, uint32_t part,
+                                           uint32_t nparts, uint32_t* __restrict__ cols, const uint32_t* __restrict__ slots,
+                                           int lane) {
+    const uint32_t S = it.y & 7u;
+    float4 c = p.halos[it.x];
+    if (S & 1u) c.x = shifted(c.x, p.half);
+    if (S & 2u) c.y = shifted(c.y, p.half);
+    if (S & 4u) c.z = shifted(c.z, p.half);
+    uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
+    const Image im = make_image(p, c.x, c.y, c.z);
+    float gy, gz;
+    gap_tables(p, im, lane, &gy, &gz);
+    const bool exactly = (it.y & (kItemZone | kItemFar)) != 0u;
+    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols) + 4 * lane;
+    bool any = false;
+    for (int f = 0; f < p.nidx; ++f) {
+        if (!((it.y >> (3 + f)) & 1u)) continue;
+        CountParams pf = p;
+        pf.pts = p.mpts[f];
+        pf.cs = p.mcs[f];
+        for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
+            uint32_t a, e;
+            row_issue(pf, im, rb, lane, gy, gz, &a, &e);
+            if (exactly) {
+                if (it.y & kItemZone)
+                    run_rows_part<BIN_LUT, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
+                else
+                    run_rows_part<BIN_LUT, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
+                continue;
+            }
+            // this warp's share of the rows' candidates, [tb, te) of the flattened sequence
+            const uint32_t len = e - a;
+            uint32_t incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            uint32_t tb = 0, te = total;
+            if (nparts > 1) {
+                tb = (uint32_t)(((uint64_t)total * part) / nparts);
+                te = (uint32_t)(((uint64_t)total * (part + 1u)) / nparts);
+            }
+            if (tb == te) continue;
+            any = true;
+            uint32_t z = 0xffffffffu;
+            auto test = [&](const float4& v) {
+                const float dx = __fsub_rn(v.x, c.x), dy = __fsub_rn(v.y, c.y), dz = __fsub_rn(v.z, c.z);
+                const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                const uint32_t key = __float_as_uint(dist);
+                z = __viaddmin_u32(key, 0u - q.zone0, z);
+                const uint32_t t = (uint32_t)__viaddmin_s32_relu((int)key, -q.kbase, q.khi);
+                const uint32_t w = slots[t >> q.shift] + (t & q.mask);
+                uint32_t* cnt = reinterpret_cast<uint32_t*>(mycol + (w >> q.shift) * 128u);
+                *cnt += 1u;
+            };
+            // distances from safe2 on, which the slots leave out
+            auto zone_test = [&](const float4& v) {
+                if (v.x != INFINITY) test_candidate<BIN_LUT, true, true>(pf, im, v, true, row, p.r2, p.lut, q.safe2);
+            };
+            const uint32_t excl = incl - len;
+            const uint32_t lo = max(excl, tb), hi = min(incl, te);
+            uint32_t bal = __ballot_sync(0xffffffffu, lo < hi);
+            if (te - tb >= kLongRow * (uint32_t)__popc(bal)) {
+                // long rows: each in windows of 32 slots
+                const uint32_t rs = a + (lo - excl), re = a + (hi - excl);
+                while (bal) {
+                    const int r = __ffs(bal) - 1;
+                    bal &= bal - 1;
+                    const uint32_t s0 = __shfl_sync(0xffffffffu, rs, r), s1 = __shfl_sync(0xffffffffu, re, r);
+                    const float4* src = pf.pts + s0 + lane;
+                    uint32_t left = s1 - s0;
+                    for (; left >= 128u; left -= 128u, src += 128) {
+                        const float4 v0 = __ldg(src), v1 = __ldg(src + 32), v2 = __ldg(src + 64), v3 = __ldg(src + 96);
+                        test(v0);
+                        test(v1);
+                        test(v2);
+                        test(v3);
+                        if (__any_sync(0xffffffffu, z < q.zone)) {
+                            zone_test(v0);
+                            zone_test(v1);
+                            zone_test(v2);
+                            zone_test(v3);
+                            z = 0xffffffffu;
+                        }
+                    }
+                    if (left) {
+                        float4 v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            v[u].x = INFINITY;
+                            if ((uint32_t)lane + 32u * (uint32_t)u < left) v[u] = __ldg(src + 32 * u);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (32u * (uint32_t)u < left) test(v[u]);
+                        if (__any_sync(0xffffffffu, z < q.zone)) {
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) zone_test(v[u]);
+                            z = 0xffffffffu;
+                        }
+                    }
+                }
+            } else {
+                // short rows: windows over the flattened sequence
+                const uint32_t off = a - excl;
+                for (uint32_t wb = tb; wb < te; wb += 64) {
+                    const uint32_t t0 = wb + (uint32_t)lane, t1 = t0 + 32u;
+                    int r0 = 0, r1 = 0;
+#pragma unroll
+                    for (int k = 16; k >= 1; k >>= 1) {
+                        const uint32_t v0 = __shfl_sync(0xffffffffu, incl, r0 + k - 1);
+                        const uint32_t v1 = __shfl_sync(0xffffffffu, incl, r1 + k - 1);
+                        r0 += (v0 <= t0) ? k : 0;
+                        r1 += (v1 <= t1) ? k : 0;
+                    }
+                    const uint32_t o0 = __shfl_sync(0xffffffffu, off, r0);
+                    const uint32_t o1 = __shfl_sync(0xffffffffu, off, r1);
+                    float4 v0, v1;
+                    v0.x = v1.x = INFINITY;
+                    if (t0 < te) v0 = __ldg(pf.pts + (t0 + o0));
+                    if (t1 < te) v1 = __ldg(pf.pts + (t1 + o1));
+                    test(v0);
+                    if (wb + 32u < te) test(v1);
+                    if (__any_sync(0xffffffffu, z < q.zone)) {
+                        zone_test(v0);
+                        zone_test(v1);
+                        z = 0xffffffffu;
+                    }
+                }
+            }
+        }
+    }
+    if (any) {
+        __syncwarp();
+        for (int s0 = 0; s0 < q.ncol; s0 += 32) {
+            const int s = s0 + lane;
+            if (s < q.ncol) {
+                uint32_t sum = 0;
+                const uint32_t* r = cols + s * 32;
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) sum += r[(k + lane) & 31];
+                if (sum) atomicAdd(row + s, sum);
+            }
+        }
+        __syncwarp();
+        for (int i = lane; i < q.ncol * 32; i += 32) cols[i] = 0u;
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(HV_THREADS, HV_BLOCKS)
+k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
+    extern __shared__ uint32_t smem[];
+    const uint32_t nhuge = min(q.ctl[1], q.cap), nother = min(q.ctl[2], q.cap);
+    if (nhuge + nother == 0u) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int colwords = (q.ncol + 1) * 32;
+    uint32_t* slots = smem + HV_WARPS * colwords;
+    uint32_t* cols = smem + warp * colwords;
+    for (int i = tid; i < q.nslots; i += HV_THREADS) slots[i] = q.slots[i];
+    for (int i = lane; i < colwords; i += 32) cols[i] = 0u;
+    __syncthreads();
+    // Warps claim (item, part) pairs.  Items of more than kHuge candidates
+    // are always split; all items are when there are too few of them.
+    const uint32_t warps = gridDim.x * HV_WARPS;
+    const uint32_t ph = nhuge >= (1u << 28) ? 1u : max(8u, min(64u, 4u * warps / max(nhuge, 1u)));
+    const uint32_t po = max(1u, min(32u, 4u * warps / max(nother, 1u)));
+    const uint32_t ch = nhuge * ph, co = nother * po;
+    for (;;) {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(q.ctl + 3, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= ch + co) break;
+        if (i < ch) count_item(p, q, q.list[i / ph], i % ph, ph, cols, slots, lane);
+        else count_item(p, q, q.list[q.cap - 1u - (i - ch) / po], (i - ch) % po, po, cols, slots, lane);
+    }
+}
+
+}  // namespace
+
+bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
+    if (!q->lane.nslots || q->nlut == 0 || !p.prune || p.nhalos >= (1ull << 29)) return false;
+    for (int i = 0; i < p.nidx; ++i)
+        if (p.mn[i] >= kEndSlot) return false;
+    return true;
+}
+
+int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s) {
+    const auto& L = qq->lane;
+    LaneParams q{};
+    q.slots = L.slots;
+    q.nslots = L.nslots;
+    q.kbase = L.kbase;
+    q.shift = L.shift;
+    q.khi = (L.nslots << L.shift) - 1;
+    q.mask = (1u << L.shift) - 1u;
+    q.ncol = L.ncol;
+    q.safe2 = L.safe2;
+    uint32_t km;
+    std::memcpy(&q.zone0, &L.safe2, 4);
+    std::memcpy(&km, &p.r2max, 4);
+    q.zone = km - q.zone0;
+    q.cmax = L.cmax;
+    q.cap = (uint32_t)std::min<uint64_t>(p.nhalos + p.nhalos / 2 + 4096, 0xffffffffull);
+    StreamScratch scr(s);
+    uint32_t* ctl = nullptr;
+    SJCS_CUDA_TRY(scr.alloc(&ctl, 32 + (uint64_t)q.cap * sizeof(uint2)));
+    SJCS_CUDA_TRY(cudaMemsetAsync(ctl, 0, 32, s));
+    q.ctl = ctl;
+    q.list = reinterpret_cast<uint2*>(ctl + 8);
+    // one block per SM (neighbouring batches share its L1); blocks of fewer
+    // warps when there are not enough batches for every SM
+    const uint64_t nbatch = (p.nhalos + 31) / 32;
+    const size_t warp_a = sizeof(LaneRows) + (size_t)(L.ncol + 1) * 64, table = (size_t)L.nslots * 4;
+    constexpr size_t kMaxSmem = 227 * 1024;
+    const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxSmem - table) / warp_a);  // >= 15 for any table
+    const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + (uint64_t)ctx->num_sms - 1) / (uint64_t)ctx->num_sms);
+    const size_t smem_a = nw * warp_a + table;
+    const size_t smem_b = HV_WARPS * (size_t)(L.ncol + 1) * 128 + (size_t)L.nslots * 4;
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
+    k_lane_count<<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
+    SJCS_LAUNCH_CHECK();
+    int per_sm = 0;
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_listed_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+    SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_listed_count, HV_THREADS, smem_b));
+    if (per_sm < 1) per_sm = 1;
+    k_listed_count<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
+    SJCS_LAUNCH_CHECK();
+    return SJCS_OK;
+}
+
+}  // namespace sjcs

@@ -167,7 +167,6 @@ int enqueue(sjcs_server* srv, Slot& sl) {
     cudaFreeAsync(sl.q.halos, s);
     cudaFreeAsync(sl.q.counts, s);
     cudaFreeAsync(sl.q.d_r2, s);
-    if (sl.q.d_lut) cudaFreeAsync(sl.q.d_lut, s);
     SJCS_CUDA_TRY(cudaEventRecord(sl.ev_done, s));
     return SJCS_OK;
 }
@@ -179,7 +178,6 @@ void release_partial(Slot& sl) {
     if (sl.q.halos) cudaFreeAsync(sl.q.halos, s);
     if (sl.q.counts) cudaFreeAsync(sl.q.counts, s);
     if (sl.q.d_r2) cudaFreeAsync(sl.q.d_r2, s);
-    if (sl.q.d_lut) cudaFreeAsync(sl.q.d_lut, s);
     cudaGetLastError();
 }
 

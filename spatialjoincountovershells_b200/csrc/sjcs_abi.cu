@@ -62,11 +62,6 @@ __global__ void k_fold_counts(uint32_t* __restrict__ c32, uint64_t m, unsigned l
     }
 }
 
-__global__ void k_fill_f32(float* __restrict__ p, uint64_t m, float v) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) p[i] = v;
-}
-
 bool valid_ctx(const sjcs_ctx* c) { return c && c->magic == kCtxMagic; }
 bool valid_index(const sjcs_index* i) { return i && i->magic == kIndexMagic; }
 bool valid_query(const sjcs_query* q) { return q && q->magic == kQueryMagic; }
@@ -145,6 +140,59 @@ void build_shell_lut(const float* r2, int nrads, std::vector<uint32_t>* lut, uin
     *shift_out = shift;
 }
 
+// Slots of the lane-per-halo count over the bit patterns of squared distances
+// (see lane_count.cu).  Shells are counted by the lanes for distances below
+// safe2: with d = p - c rounded per axis and the box bounds rounded from c -+
+// half, a particle outside the box on some axis has |d| >= (half - 2^-24 (|c|
+// + half)) (1 - 2^-24), so its fp32 distance is at least safe2 as computed
+// here for |c| <= cmax.  Slot j covers the keys [kbase + (j << shift), ... +
+// (1 << shift)) and holds at most one of the thresholds (r2 below safe2, then
+// safe2); word j is (thresholds before the slot << shift) + (1 << shift) - low
+// bits of its threshold, so adding a key's low bits carries into the index
+// exactly when the key has reached the threshold.
+void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32_t>* slots,
+                      sjcs_query::LaneTable* t) {
+    constexpr int kMaxSlots = 2048, kMaxCols = 128;
+    const float r2max = r2[nrads - 1];
+    if (!std::isfinite(r2max) || !std::isfinite(half)) return;
+    t->cmax = 1000.0f + 2.0f * half;  // every image of a halo in the box
+    const float sf = half - 1.2e-7f * (t->cmax + half);
+    if (!(sf > 0.0f)) return;
+    t->safe2 = std::min(sf * sf * (1.0f - 1e-6f), r2max);
+    if (!(t->safe2 >= 0.98f * r2max)) return;  // distances from safe2 on are counted one by one
+    std::vector<int> th;
+    for (int i = 0; i < nrads; ++i) {
+        int b;
+        std::memcpy(&b, &r2[i], 4);
+        if (b < 0 || (i > 0 && !(r2[i] > r2[i - 1]))) return;
+        if (r2[i] < t->safe2) th.push_back(b);
+    }
+    int b;
+    std::memcpy(&b, &t->safe2, 4);
+    th.push_back(b);
+    if (th[0] < 1 || th.size() > (size_t)kMaxCols) return;
+    int gap = th[0];
+    for (size_t i = 1; i < th.size(); ++i) gap = std::min(gap, th[i] - th[i - 1]);
+    int shift = 0;
+    while (shift < 24 && (2 << shift) <= gap && (th.size() + 2) < (1ull << (31 - shift))) ++shift;
+    const int kbase = th[0] - (1 << shift);  // >= 0
+    const int n = ((th.back() - kbase) >> shift) + 1;
+    if (n > kMaxSlots) return;
+    slots->resize(n);
+    size_t before = 0;
+    for (int j = 0; j < n; ++j) {
+        const int k = kbase + (j << shift);
+        while (before < th.size() && th[before] < k) ++before;
+        uint32_t low = 1u << shift;  // no threshold in this slot
+        if (before < th.size() && th[before] - k < (1 << shift)) low = (uint32_t)(th[before] - k);
+        (*slots)[j] = ((uint32_t)before << shift) + (1u << shift) - low;
+    }
+    t->nslots = n;
+    t->kbase = kbase;
+    t->shift = shift;
+    t->ncol = (int)th.size();
+}
+
 }  // namespace
 
 constexpr uint32_t kParamSlots = 8;
@@ -192,19 +240,23 @@ int query_prepare(sjcs_ctx* ctx, const float* d_halo_xyz, size_t stride, uint64_
     q->r2max = r2[nrads - 1];
     q->R = (float)std::sqrt((double)r2[nrads - 1]);
     q->half = (flags & SJCS_QUERY_PERIODIC) ? q->R : r2[nrads - 1];
-    SJCS_CUDA_TRY(cudaMallocAsync(&q->d_r2, (size_t)pad * sizeof(float), s));
-    k_fill_f32<<<(pad + 255) / 256, 256, 0, s>>>(q->d_r2, (uint64_t)pad, INFINITY);
-    SJCS_LAUNCH_CHECK();
-    int rc = upload_params(ctx, q->d_r2, r2, (size_t)nrads * sizeof(float), s);
-    if (rc) return rc;
-    std::vector<uint32_t> lut;
+    // radius table (padded with +inf), shell lookup and lane slots: one
+    // allocation, one upload
+    std::vector<uint32_t> lut, lane;
     if (mono) build_shell_lut(r2, nrads, &lut, &q->lut_k0, &q->lut_shift);
     q->nlut = (int)lut.size();
-    if (!lut.empty()) {
-        SJCS_CUDA_TRY(cudaMallocAsync(&q->d_lut, lut.size() * sizeof(uint32_t), s));
-        rc = upload_params(ctx, q->d_lut, lut.data(), lut.size() * sizeof(uint32_t), s);
-        if (rc) return rc;
-    }
+    q->lane = {};
+    if (mono) build_lane_table(r2, nrads, q->half, &lane, &q->lane);
+    std::vector<uint32_t> block((size_t)pad + lut.size() + lane.size());
+    const float inf = INFINITY;
+    for (int i = 0; i < pad; ++i) std::memcpy(&block[i], i < nrads ? &r2[i] : &inf, sizeof(float));
+    std::copy(lut.begin(), lut.end(), block.begin() + pad);
+    std::copy(lane.begin(), lane.end(), block.begin() + pad + lut.size());
+    SJCS_CUDA_TRY(cudaMallocAsync(&q->d_r2, block.size() * sizeof(uint32_t), s));
+    int rc = upload_params(ctx, q->d_r2, block.data(), block.size() * sizeof(uint32_t), s);
+    if (rc) return rc;
+    q->d_lut = lut.empty() ? nullptr : reinterpret_cast<uint32_t*>(q->d_r2) + pad;
+    q->lane.slots = reinterpret_cast<uint32_t*>(q->d_r2) + pad + lut.size();
     const uint64_t ncnt = nhalos * (uint64_t)nrads;
     SJCS_CUDA_TRY(cudaMallocAsync(&q->counts, (ncnt ? ncnt : 1) * sizeof(uint32_t), s));
     if (ncnt) SJCS_CUDA_TRY(cudaMemsetAsync(q->counts, 0, ncnt * sizeof(uint32_t), s));
@@ -285,7 +337,6 @@ void free_query(sjcs_query* q) {
     if (q->counts) cudaFreeAsync(q->counts, s);
     if (q->counts64) cudaFreeAsync(q->counts64, s);
     if (q->d_r2) cudaFreeAsync(q->d_r2, s);
-    if (q->d_lut) cudaFreeAsync(q->d_lut, s);
     cudaStreamSynchronize(s);
     if (q->h_stage) cudaFreeHost(q->h_stage);
     clear_count_events(q);

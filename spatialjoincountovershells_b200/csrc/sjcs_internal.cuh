@@ -184,6 +184,17 @@ struct sjcs_query {
     int nlut;
     uint32_t lut_k0;
     int lut_shift;
+    // Lane-per-halo count (lane_count.cu): shells as slots of the distance's
+    // bit pattern.  nslots == 0: the table does not fit that form.
+    struct LaneTable {
+        uint32_t* slots;  // [nslots], device (part of the d_r2 allocation)
+        int nslots;
+        int kbase;        // bit pattern where slot 0 starts
+        int shift;        // bits of a slot
+        int ncol;         // shells below safe2
+        float safe2;      // a distance below it lies inside the query box
+        float cmax;       // for centres up to this far from the origin on every axis
+    } lane;
     uint32_t* h_stage;  // pinned staging for count read-back
     size_t h_stage_elems;
     std::vector<cudaEvent_t> count_events;  // (start, end) pairs, one per count call since reset
