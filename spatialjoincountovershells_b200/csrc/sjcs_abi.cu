@@ -80,25 +80,82 @@ bool is_pinned(const void* p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// Parallel host copy/add of a widened chunk into the caller's array.
-void host_store(uint64_t* dst, const uint64_t* src, uint64_t m, bool add) {
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const unsigned nt = (m < (1u << 20)) ? 1u : hw;
-    auto work = [&](unsigned t) {
-        const uint64_t lo = m * t / nt, hi = m * (t + 1) / nt;
-        if (add)
-            for (uint64_t i = lo; i < hi; ++i) dst[i] += src[i];
-        else
-            std::memcpy(dst + lo, src + lo, (hi - lo) * sizeof(uint64_t));
-    };
-    if (nt == 1) {
-        work(0);
-        return;
+// Read-back of counts into pageable memory: each of up to kReadThreads host
+// threads takes chunks t, t + T, ... of the m counts through two page-locked
+// slots of its own, the copy of its next chunk queued before it widens and
+// stores (or adds) the current one.  The slots belong to the context and are
+// made once: page-locking per query cost about 50 ms, and the counts cross
+// the link as 32-bit values when no fold has happened (200 000 x 40 counts
+// into pageable memory: 53 ms before).  Called with ctx->mu held.
+constexpr unsigned kReadThreads = 8;
+constexpr size_t kReadSlotBytes = 1 << 20;
+
+int ensure_read_slots(sjcs_ctx* ctx) {
+    if (ctx->read_slots) return SJCS_OK;
+    std::vector<cudaEvent_t> ev(2 * kReadThreads, nullptr);
+    for (auto& e : ev) SJCS_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (cudaMallocHost(&ctx->read_slots, 2 * kReadThreads * kReadSlotBytes) != cudaSuccess) {
+        ctx->read_slots = nullptr;
+        cudaGetLastError();
+        for (auto e : ev) cudaEventDestroy(e);
+        return fail(SJCS_ERR_NOMEM, "page-locked staging for the count read-back could not be allocated");
     }
+    ctx->read_ev = std::move(ev);
+    return SJCS_OK;
+}
+
+template <class T>
+int read_pageable(sjcs_ctx* ctx, const T* d_src, uint64_t m, uint64_t* dst, bool add, cudaStream_t s) {
+    int rc = ensure_read_slots(ctx);
+    if (rc) return rc;
+    constexpr uint64_t kChunk = kReadSlotBytes / sizeof(T);
+    const uint64_t nchunks = (m + kChunk - 1) / kChunk;
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    const unsigned nt = (unsigned)std::min<uint64_t>(std::min(kReadThreads, hw), nchunks);
+    std::atomic<int> err{(int)cudaSuccess};
+    auto work = [&](unsigned t) {
+        auto check = [&](cudaError_t e) {
+            if (e != cudaSuccess) err = (int)e;
+            return e == cudaSuccess;
+        };
+        T* slot[2];
+        for (unsigned k = 0; k < 2; ++k)
+            slot[k] = reinterpret_cast<T*>(ctx->read_slots + (2 * t + k) * kReadSlotBytes);
+        auto queue = [&](uint64_t c, unsigned k) {
+            const uint64_t off = c * kChunk, len = std::min(kChunk, m - off);
+            return check(cudaMemcpyAsync(slot[k], d_src + off, len * sizeof(T), cudaMemcpyDeviceToHost, s)) &&
+                   check(cudaEventRecord(ctx->read_ev[2 * t + k], s));
+        };
+        if (!check(cudaSetDevice(ctx->device)) || !queue(t, 0)) return;
+        unsigned k = 0;
+        for (uint64_t c = t; c < nchunks && err == (int)cudaSuccess; c += nt, k ^= 1u) {
+            if (c + nt < nchunks && !queue(c + nt, k ^ 1u)) return;
+            if (!check(cudaEventSynchronize(ctx->read_ev[2 * t + k]))) return;
+            const uint64_t off = c * kChunk, len = std::min(kChunk, m - off);
+            const T* v = slot[k];
+            uint64_t* o = dst + off;
+            if (add)
+                for (uint64_t i = 0; i < len; ++i) o[i] += v[i];
+            else
+                for (uint64_t i = 0; i < len; ++i) o[i] = v[i];
+        }
+    };
     std::vector<std::thread> th;
     th.reserve(nt);
-    for (unsigned t = 0; t < nt; ++t) th.emplace_back(work, t);
+    unsigned started = 1;
+    try {
+        for (; started < nt; ++started) th.emplace_back(work, started);
+    } catch (const std::exception&) {
+        // no more threads: this one takes the missing threads' chunks below
+    }
+    work(0);
+    for (unsigned t = started; t < nt; ++t) work(t);
     for (auto& x : th) x.join();
+    const cudaError_t e = cudaStreamSynchronize(s);  // no copy into the slots is left in flight
+    if (err == (int)cudaSuccess) err = (int)e;
+    if (err != (int)cudaSuccess)
+        return fail(SJCS_ERR_CUDA, "count read-back failed: %s", cudaGetErrorString((cudaError_t)(int)err));
+    return SJCS_OK;
 }
 
 // Shell lookup table over the bit patterns of squared distances (see
@@ -338,7 +395,6 @@ void free_query(sjcs_query* q) {
     if (q->counts64) cudaFreeAsync(q->counts64, s);
     if (q->d_r2) cudaFreeAsync(q->d_r2, s);
     cudaStreamSynchronize(s);
-    if (q->h_stage) cudaFreeHost(q->h_stage);
     clear_count_events(q);
     cudaEventDestroy(q->ev_last);
     cudaEventDestroy(q->ev_d0);
@@ -640,6 +696,9 @@ int sjcs_ctx_destroy(sjcs_ctx* ctx) {
     for (cudaEvent_t e : ctx->param_ev)
         if (e) cudaEventDestroy(e);
     if (ctx->param_ring) cudaFreeHost(ctx->param_ring);
+    for (cudaEvent_t e : ctx->read_ev)
+        if (e) cudaEventDestroy(e);
+    if (ctx->read_slots) cudaFreeHost(ctx->read_slots);
     if (ctx->ev_counts) cudaEventDestroy(ctx->ev_counts);
     ctx->magic = 0;
     delete ctx;
@@ -1432,50 +1491,25 @@ int sjcs_query_read_counts(sjcs_ctx* ctx, sjcs_query* q, uint64_t* counts, int a
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaStream_t s = ctx->s_count;
     if (m == 0) return SJCS_OK;
+    const bool direct = !accumulate && is_pinned(counts);
     StreamScratch scr(s);
     unsigned long long* wide = nullptr;
-    SJCS_CUDA_TRY(scr.alloc(&wide, m * sizeof(uint64_t)));
+    if (direct || q->counts64) SJCS_CUDA_TRY(scr.alloc(&wide, m * sizeof(uint64_t)));
     cudaEventRecord(q->ev_d0, s);
-    k_widen_u32_u64<<<ctx->num_sms * 8, 256, 0, s>>>(q->counts, m, q->counts64, wide);
-    SJCS_LAUNCH_CHECK();
-    if (!accumulate && is_pinned(counts)) {
+    if (wide) {
+        k_widen_u32_u64<<<ctx->num_sms * 8, 256, 0, s>>>(q->counts, m, q->counts64, wide);
+        SJCS_LAUNCH_CHECK();
+    }
+    if (direct) {
         SJCS_CUDA_TRY(cudaMemcpyAsync(counts, wide, m * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         cudaEventRecord(q->ev_d1, s);
         SJCS_CUDA_TRY(cudaStreamSynchronize(s));
     } else {
-        // Double-buffered pinned staging; host threads store (or add) chunk
-        // k while the copy engine brings chunk k+1.
-        const uint64_t chunk = 8ull << 20;  // elements (64 MB)
-        if (!q->h_stage) {
-            SJCS_CUDA_TRY(cudaMallocHost(&q->h_stage, 2 * chunk * sizeof(uint64_t)));
-            q->h_stage_elems = 2 * chunk;
-        }
-        uint64_t* stage = reinterpret_cast<uint64_t*>(q->h_stage);
-        cudaEvent_t done[2];
-        cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming);
-        cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming);
-        const uint64_t nchunks = (m + chunk - 1) / chunk;
-        int err = SJCS_OK;
-        for (uint64_t c = 0; c <= nchunks && !err; ++c) {
-            if (c < nchunks) {
-                const uint64_t off = c * chunk, len = std::min(chunk, m - off);
-                cudaError_t e = cudaMemcpyAsync(stage + (c & 1) * chunk, wide + off, len * sizeof(uint64_t),
-                                                cudaMemcpyDeviceToHost, s);
-                if (e == cudaSuccess) e = cudaEventRecord(done[c & 1], s);
-                if (e != cudaSuccess) err = fail(SJCS_ERR_CUDA, "count read-back failed: %s", cudaGetErrorString(e));
-            }
-            if (c > 0 && !err) {
-                const uint64_t p = c - 1, off = p * chunk, len = std::min(chunk, m - off);
-                cudaError_t e = cudaEventSynchronize(done[p & 1]);
-                if (e != cudaSuccess) err = fail(SJCS_ERR_CUDA, "count read-back failed: %s", cudaGetErrorString(e));
-                else host_store(counts + off, stage + (p & 1) * chunk, len, accumulate != 0);
-            }
-        }
+        rc = wide ? read_pageable(ctx, wide, m, counts, accumulate != 0, s)
+                  : read_pageable(ctx, q->counts, m, counts, accumulate != 0, s);
         cudaEventRecord(q->ev_d1, s);
         cudaStreamSynchronize(s);
-        cudaEventDestroy(done[0]);
-        cudaEventDestroy(done[1]);
-        if (err) return err;
+        if (rc) return rc;
     }
     float ms = 0.f;
     q->last_d2h_ms = (cudaEventElapsedTime(&ms, q->ev_d0, q->ev_d1) == cudaSuccess) ? ms : 0.f;

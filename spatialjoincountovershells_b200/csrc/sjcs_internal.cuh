@@ -139,6 +139,10 @@ struct sjcs_ctx {
     char* param_ring = nullptr;
     std::vector<cudaEvent_t> param_ev;
     uint32_t param_next = 0;
+    // Read-back into pageable memory: page-locked slots with their events
+    // (used with mu held; released with the context).
+    char* read_slots = nullptr;
+    std::vector<cudaEvent_t> read_ev;
 };
 
 namespace sjcs {
@@ -195,8 +199,6 @@ struct sjcs_query {
         float safe2;      // a distance below it lies inside the query box
         float cmax;       // for centres up to this far from the origin on every axis
     } lane;
-    uint32_t* h_stage;  // pinned staging for count read-back
-    size_t h_stage_elems;
     std::vector<cudaEvent_t> count_events;  // (start, end) pairs, one per count call since reset
     cudaEvent_t ev_last;                    // end of the last count call
     cudaEvent_t ev_d0, ev_d1;
