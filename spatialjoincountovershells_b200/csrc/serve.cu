@@ -135,7 +135,7 @@ int enqueue(sjcs_server* srv, Slot& sl) {
             fuse = b->kind == SJCS_INDEX_GRID && b->geom.ncells == a->geom.ncells && b->geom.G[0] == a->geom.G[0] &&
                    b->geom.G[1] == a->geom.G[1] && b->geom.G[2] == a->geom.G[2];
         }
-        if (fuse) fuse = schedule_for(srv->ctx, &sl.q, srv->idx[0]).mode != SJCS_SCHED_QUEUE;
+        if (fuse) fuse = may_fuse(&sl.q, srv->idx[0], schedule_for(srv->ctx, &sl.q, srv->idx[0]));
         if (fuse) {
             rc = launch_shell_count_multi(srv->ctx, &sl.q, srv->idx.data(), (int)k, s);
             if (rc) return rc;

@@ -588,11 +588,24 @@ int launch_static(sjcs_ctx* ctx, const CountParams& p, int bin, bool big, size_t
 
 }  // namespace
 
+namespace {
+// Sizes the queue schedule refuses, whichever kernel counts.
+bool queue_too_large(const sjcs_query* q, const Schedule& sc) {
+    return q->nhalos * (uint64_t)sc.max_pieces >= (1ull << 32);
+}
+}  // namespace
+
+bool may_fuse(const sjcs_query* q, const sjcs_index* idx, const Schedule& sc) {
+    if (idx->kind != SJCS_INDEX_GRID) return false;
+    if (sc.mode != SJCS_SCHED_QUEUE) return true;
+    return !queue_too_large(q, sc) && lane_count_applies(q, count_params(q, idx));
+}
+
 int launch_shell_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx, cudaStream_t s,
                        const Schedule* sc) {
     if (q->nhalos == 0 || idx->n == 0) return SJCS_OK;
     const CountParams p = count_params(q, idx);
-    if (sc && sc->mode == SJCS_SCHED_QUEUE && p.nhalos * (uint64_t)sc->max_pieces >= (1ull << 32))
+    if (sc && sc->mode == SJCS_SCHED_QUEUE && queue_too_large(q, *sc))
         return fail(SJCS_ERR_INVALID, "queue schedule: nhalos * max_pieces must stay below 2^32");
     // Either schedule: the lane count lists heavy halos itself and splits them.
     if (lane_count_applies(q, p)) return launch_lane_count(ctx, q, p, s);

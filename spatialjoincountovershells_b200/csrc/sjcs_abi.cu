@@ -1207,7 +1207,7 @@ int sjcs_query_count_many(sjcs_ctx* ctx, sjcs_query* q, const sjcs_index* const*
     int rc = set_device(ctx);
     if (rc) return rc;
     // Fused: runs of up to kMaxFused grid indexes of one geometry under the
-    // static schedule whose counts fit the accumulators together; anything
+    // static schedule (or counted by lanes, which ignores it) whose counts fit the accumulators together; anything
     // else is counted index by index.
     for (int i = 0; i < k;) {
         int j = i + 1;
@@ -1215,7 +1215,7 @@ int sjcs_query_count_many(sjcs_ctx* ctx, sjcs_query* q, const sjcs_index* const*
         bool fuse = a->kind == SJCS_INDEX_GRID;
         if (fuse) {
             std::lock_guard<std::mutex> lk(ctx->mu);
-            fuse = schedule_for(ctx, q, a).mode != SJCS_SCHED_QUEUE;
+            fuse = may_fuse(q, a, schedule_for(ctx, q, a));
         }
         uint64_t add = count_call_bound(q->flags, q->r2max, a->n);
         while (fuse && j < k && j - i < kMaxFusedIndexes) {

@@ -288,6 +288,11 @@ constexpr int kMaxFusedIndexes = 4;
 int launch_shell_count_multi(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* const* idx, int k,
                              cudaStream_t s);
 
+// Whether a count under schedule sc may be one pass over several grid
+// indexes: the static schedule, or a query counted by lanes (lane_count.cu),
+// which the queue would count index by index for nothing.
+bool may_fuse(const sjcs_query* q, const sjcs_index* idx, const Schedule& sc);
+
 // scan.cu: exclusive prefix sum of m u32 values, in place.  `partials`
 // (scan_partials_needed(m) u32) may be given; otherwise it is allocated.
 int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* partials = nullptr);
