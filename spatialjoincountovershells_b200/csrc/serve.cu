@@ -102,9 +102,10 @@ constexpr uint32_t kServerMagic = 0x534a5653u;  // "SJVS"
 bool valid_server(const sjcs_server* s) { return s && s->magic == kServerMagic; }
 
 uint64_t request_bytes(uint64_t nhalos, size_t stride, int nrads) {
-    // per halo: raw halo + sorted halo + Morton sort records (2 x (4 + 16) B)
-    // + counts + queue-schedule scratch (12 B) + sort histogram (1 B);
-    // fixed: radius table, shell lookup table, scan partials
+    // per halo: raw halo + ordered halo + counts, and 53 bytes of scratch: its
+    // rank and share of the bucket counters (6 B) and the count's item list
+    // (12 B per index of a fused pass, up to 4), or the queue schedule's keys
+    // and order (13 B); fixed: radius and lookup tables, scan partials
     return nhalos * (uint64_t)(stride + 16 + 40 + 4 * (uint64_t)nrads + 13) + 65536 + 8 * (uint64_t)nrads;
 }
 
