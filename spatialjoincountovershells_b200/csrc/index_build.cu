@@ -511,7 +511,10 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         return SJCS_OK;
     }
     const int kb = grid_key_bits(g);
-    const int sb = kb > PB_MIN_SEG_BITS + 18 ? kb - 18 : PB_MIN_SEG_BITS;  // segment bits, <= PB_GROUP_BITS
+    // Segment bits, <= PB_GROUP_BITS.  Keys of up to 21 bits take segments
+    // wide enough for one digit above them: one partition pass instead of two.
+    const int sb = kb <= PB_GROUP_BITS + 9 ? std::max(PB_MIN_SEG_BITS, kb - 9)
+                                           : std::max(PB_MIN_SEG_BITS, kb - 18);
     const int upper = kb > sb ? kb - sb : 0;  // bits above the segment
     const int bits_mid = upper > 9 ? upper - 9 : 0;
     const int bits_top = upper - bits_mid;
@@ -530,11 +533,11 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
     // top digit counts and starts (ntop + 1 entries); without a middle pass
     // the top digit is the segment and these are the segment starts too
     SJCS_CUDA_TRY(scr.alloc(&top, ((uint64_t)ntop + 1) * sizeof(uint32_t)));
-    SJCS_CUDA_TRY(scr.alloc(&cur_top, (uint64_t)ntop * sizeof(uint32_t)));
+    SJCS_CUDA_TRY(scr.alloc(&cur_top, ((uint64_t)ntop + 1) * sizeof(uint32_t)));
     SJCS_CUDA_TRY(scr.alloc(&tmp, n * sizeof(float4)));
     if (bits_mid) {
         SJCS_CUDA_TRY(scr.alloc(&seg, (nseg + 1) * sizeof(uint32_t)));
-        SJCS_CUDA_TRY(scr.alloc(&cur_seg, nseg * sizeof(uint32_t)));
+        SJCS_CUDA_TRY(scr.alloc(&cur_seg, (nseg + 1) * sizeof(uint32_t)));
         SJCS_CUDA_TRY(scr.alloc(&tiles, ntiles_mid * sizeof(PbTile)));
         SJCS_CUDA_TRY(scr.alloc(&ntiles, sizeof(uint32_t)));
         SJCS_CUDA_TRY(scr.alloc(&mid, n * sizeof(uint16_t)));
@@ -549,9 +552,8 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
     k_pb_top_hist<<<(unsigned)((ntiles_in + PB_TOP_TILES - 1) / PB_TOP_TILES), PB_THREADS, PB_STAGE_SMEM, s>>>(
         d_xyz, aligned, n, g, top_shift, top);
     SJCS_LAUNCH_CHECK();
-    int rc = exclusive_scan_u32(top, (uint64_t)ntop + 1, s);
+    int rc = exclusive_scan_u32(top, (uint64_t)ntop + 1, s, nullptr, cur_top);
     if (rc) return rc;
-    SJCS_CUDA_TRY(cudaMemcpyAsync(cur_top, top, (uint64_t)ntop * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)PB_SMEM));
     SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -571,9 +573,8 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         k_pb_mid_hist<<<(unsigned)((ntiles_mid + PB_MID_TILES - 1) / PB_MID_TILES), PB_THREADS, 0, s>>>(
             mid, tiles, ntiles, bits_mid, nseg, seg);
         SJCS_LAUNCH_CHECK();
-        rc = exclusive_scan_u32(seg, nseg + 1, s);
+        rc = exclusive_scan_u32(seg, nseg + 1, s, nullptr, cur_seg);
         if (rc) return rc;
-        SJCS_CUDA_TRY(cudaMemcpyAsync(cur_seg, seg, nseg * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
         k_pb_partition<true><<<(unsigned)ntiles_mid, PB_THREADS, PB_SMEM, s>>>(
             nullptr, 0, pts, tiles, ntiles, n, g, sb, bits_mid, bits_mid, cur_seg, tmp, nullptr, sb, 0u);
         SJCS_LAUNCH_CHECK();

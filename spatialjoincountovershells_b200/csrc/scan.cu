@@ -1,5 +1,6 @@
-// Device-wide exclusive prefix sum of u32 values (reduce, scan of partials,
-// apply).  Used for the radix sort's digit-major tile histograms.
+// Device-wide exclusive prefix sum of u32 values: one block for short arrays,
+// else reduce, scan of partials, apply.  `copy` (optional) receives the sums
+// too (a build's starts and the cursors that begin there).
 #include "sjcs_internal.cuh"
 
 namespace sjcs {
@@ -65,9 +66,38 @@ __global__ void __launch_bounds__(SC_THREADS) k_scan_partials(uint32_t* __restri
     }
 }
 
+// Up to kOneBlock values: one block, SC_CHUNK at a time, carrying the total.
+constexpr uint64_t kOneBlock = 4 * SC_CHUNK;
+__global__ void __launch_bounds__(SC_THREADS) k_scan_one(uint32_t* __restrict__ data, uint32_t m,
+                                                         uint32_t* __restrict__ copy) {
+    __shared__ uint32_t tot;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < m; base += SC_CHUNK) {
+        const uint32_t at = base + threadIdx.x * SC_ITEMS;
+        uint32_t v[SC_ITEMS], s = 0;
+#pragma unroll
+        for (int i = 0; i < SC_ITEMS; ++i) {
+            v[i] = at + i < m ? data[at + i] : 0u;
+            s += v[i];
+        }
+        uint32_t run = block_excl_scan(s, &tot) + carry;
+        carry += tot;
+#pragma unroll
+        for (int i = 0; i < SC_ITEMS; ++i) {
+            if (at + i < m) {
+                data[at + i] = run;
+                if (copy) copy[at + i] = run;
+            }
+            run += v[i];
+        }
+        __syncthreads();
+    }
+}
+
 // Each thread owns SC_ITEMS consecutive values (blocked layout).
 __global__ void __launch_bounds__(SC_THREADS) k_scan_apply(uint32_t* __restrict__ data, uint64_t m,
-                                                           const uint32_t* __restrict__ partials) {
+                                                           const uint32_t* __restrict__ partials,
+                                                           uint32_t* __restrict__ copy) {
     const uint64_t base = (uint64_t)blockIdx.x * SC_CHUNK + (uint64_t)threadIdx.x * SC_ITEMS;
     uint32_t v[SC_ITEMS];
     uint32_t s = 0;
@@ -80,7 +110,10 @@ __global__ void __launch_bounds__(SC_THREADS) k_scan_apply(uint32_t* __restrict_
     uint32_t run = block_excl_scan(s, &tot) + partials[blockIdx.x];
 #pragma unroll
     for (int i = 0; i < SC_ITEMS; ++i) {
-        if (base + i < m) data[base + i] = run;
+        if (base + i < m) {
+            data[base + i] = run;
+            if (copy) copy[base + i] = run;
+        }
         run += v[i];
     }
 }
@@ -89,8 +122,13 @@ __global__ void __launch_bounds__(SC_THREADS) k_scan_apply(uint32_t* __restrict_
 
 uint64_t scan_partials_needed(uint64_t m) { return (m + SC_CHUNK - 1) / SC_CHUNK; }
 
-int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* partials) {
+int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* partials, uint32_t* copy) {
     if (m == 0) return SJCS_OK;
+    if (m <= kOneBlock) {
+        k_scan_one<<<1, SC_THREADS, 0, s>>>(d_data, (uint32_t)m, copy);
+        SJCS_LAUNCH_CHECK();
+        return SJCS_OK;
+    }
     const uint64_t nb = (m + SC_CHUNK - 1) / SC_CHUNK;
     if (nb > 0xffffffffull) return fail(SJCS_ERR_INVALID, "scan too large (%llu)", (unsigned long long)m);
     StreamScratch scr(s);
@@ -99,7 +137,7 @@ int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* p
     SJCS_LAUNCH_CHECK();
     k_scan_partials<<<1, SC_THREADS, 0, s>>>(partials, (uint32_t)nb);
     SJCS_LAUNCH_CHECK();
-    k_scan_apply<<<(unsigned)nb, SC_THREADS, 0, s>>>(d_data, m, partials);
+    k_scan_apply<<<(unsigned)nb, SC_THREADS, 0, s>>>(d_data, m, partials, copy);
     SJCS_LAUNCH_CHECK();
     return SJCS_OK;
 }

@@ -294,8 +294,10 @@ int launch_shell_count_multi(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_inde
 bool may_fuse(const sjcs_query* q, const sjcs_index* idx, const Schedule& sc);
 
 // scan.cu: exclusive prefix sum of m u32 values, in place.  `partials`
-// (scan_partials_needed(m) u32) may be given; otherwise it is allocated.
-int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* partials = nullptr);
+// (scan_partials_needed(m) u32) may be given; otherwise it is allocated when
+// the scan needs more than one block.  `copy` receives the sums too.
+int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* partials = nullptr,
+                       uint32_t* copy = nullptr);
 uint64_t scan_partials_needed(uint64_t m);
 
 // index_build.cu: the stable LSD grid build on caller-provided buffers (no
