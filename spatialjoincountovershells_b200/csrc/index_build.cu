@@ -9,11 +9,10 @@
 // -- so any index that returns a superset of the in-box points gives the same
 // counts.  Here the index is a uniform cell grid.  Cell keys of up to 30 bits
 // (every automatic grid) are built by the partition build further down; wider
-// keys, and the fixed-buffer build, by a stable LSD radix sort:
+// keys by a stable LSD radix sort:
 //   pass 0   key = cell of (x,y,z) and payload = (x,y,z), read from the AoS input
 //            (staged in shared memory a tile at a time when 16-byte aligned)
-//   passes   stable LSD radix sort of (key, payload), 8 bits per pass (9 for
-//            25-27-bit cell keys: three passes instead of four)
+//   passes   stable LSD radix sort of (key, payload), 8 bits per pass
 //   last     writes the sorted particles as float4 and the sorted keys
 //   offsets  cell_start[c] = first sorted slot of cell c (boundary fill)
 #include <algorithm>
@@ -185,21 +184,21 @@ __device__ __forceinline__ uint32_t pb_block_scan(uint32_t v, uint32_t* ws, uint
 __device__ __forceinline__ uint32_t pb_key(const float4& r) { return __float_as_uint(r.w); }
 
 // top_hist[cell >> shift] += 1 for every particle (at most PB_THREADS bins,
-// counted in shared memory first).  Block b takes tiles PB_TOP_TILES*b ..
+// counted in shared memory first).  Block b takes tiles `tiles`*b ..
 // (one reduction per bin for all of them); each tile's x,y,z are staged in
 // shared memory with coalesced 16-byte copies (cp.async when the array is
 // 16-byte aligned) and the keys taken from there.
 constexpr uint32_t PB_TOP_TILES = 4;
 __global__ void __launch_bounds__(PB_THREADS)
 k_pb_top_hist(const float* __restrict__ xyz, int aligned, uint64_t n, GridGeom g, int shift,
-              uint32_t* __restrict__ top_hist) {
+              uint32_t* __restrict__ top_hist, uint32_t tiles) {
     __shared__ uint32_t sh[PB_THREADS];
     extern __shared__ float4 stage4[];
     float* sx = reinterpret_cast<float*>(stage4);
     const int tid = threadIdx.x;
     sh[tid] = 0u;
-    for (uint32_t t = 0; t < PB_TOP_TILES; ++t) {
-        const uint64_t start = ((uint64_t)blockIdx.x * PB_TOP_TILES + t) * PB_TILE;
+    for (uint32_t t = 0; t < tiles; ++t) {
+        const uint64_t start = ((uint64_t)blockIdx.x * tiles + t) * PB_TILE;
         if (start >= n) break;  // uniform across the block
         const uint64_t rem = n - start;
         const uint32_t len = rem < PB_TILE ? (uint32_t)rem : PB_TILE;
@@ -503,6 +502,24 @@ k_pb_cells(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start
     }
 }
 
+// Segment bits of a key, <= PB_GROUP_BITS.  Keys of up to 21 bits take
+// segments wide enough for one digit above them: one partition pass instead
+// of two.
+int segment_bits(int kb) {
+    return kb <= PB_GROUP_BITS + 9 ? std::max(PB_MIN_SEG_BITS, kb - 9) : std::max(PB_MIN_SEG_BITS, kb - 18);
+}
+
+int set_partition_smem() {
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_top_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)PB_STAGE_SMEM));
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)PB_SMEM));
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)PB_SMEM));
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
+    return SJCS_OK;
+}
+
 // The partition build into pts (n records) and cs (ncells + 1 entries).
 int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, float4* pts, uint32_t* cs,
                            cudaStream_t s) {
@@ -511,10 +528,7 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         return SJCS_OK;
     }
     const int kb = grid_key_bits(g);
-    // Segment bits, <= PB_GROUP_BITS.  Keys of up to 21 bits take segments
-    // wide enough for one digit above them: one partition pass instead of two.
-    const int sb = kb <= PB_GROUP_BITS + 9 ? std::max(PB_MIN_SEG_BITS, kb - 9)
-                                           : std::max(PB_MIN_SEG_BITS, kb - 18);
+    const int sb = segment_bits(kb);
     const int upper = kb > sb ? kb - sb : 0;  // bits above the segment
     const int bits_mid = upper > 9 ? upper - 9 : 0;
     const int bits_top = upper - bits_mid;
@@ -546,19 +560,16 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         seg = top;
     }
     const int top_shift = sb + bits_mid;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_top_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)PB_STAGE_SMEM));
-    SJCS_CUDA_TRY(cudaMemsetAsync(top, 0, ((uint64_t)ntop + 1) * sizeof(uint32_t), s));
-    k_pb_top_hist<<<(unsigned)((ntiles_in + PB_TOP_TILES - 1) / PB_TOP_TILES), PB_THREADS, PB_STAGE_SMEM, s>>>(
-        d_xyz, aligned, n, g, top_shift, top);
-    SJCS_LAUNCH_CHECK();
-    int rc = exclusive_scan_u32(top, (uint64_t)ntop + 1, s, nullptr, cur_top);
+    int rc = set_partition_smem();
     if (rc) return rc;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)PB_SMEM));
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)PB_SMEM));
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
+    SJCS_CUDA_TRY(cudaMemsetAsync(top, 0, ((uint64_t)ntop + 1) * sizeof(uint32_t), s));
+    // four tiles a block once every SM has blocks enough
+    const uint32_t per = ntiles_in >= 148ull * 4 * PB_TOP_TILES ? PB_TOP_TILES : 1u;
+    k_pb_top_hist<<<(unsigned)((ntiles_in + per - 1) / per), PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, g,
+                                                                                          top_shift, top, per);
+    SJCS_LAUNCH_CHECK();
+    rc = exclusive_scan_u32(top, (uint64_t)ntop + 1, s, nullptr, cur_top);
+    if (rc) return rc;
     // pass A writes pts when a middle pass follows (pts is free until the
     // last pass), else tmp; with a middle pass it also writes the middle digits
     float4* a_out = bits_mid ? pts : tmp;
@@ -585,6 +596,33 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
 }
 
 }  // namespace
+
+int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s) {
+    if (n == 0) {
+        SJCS_CUDA_TRY(cudaMemsetAsync(b.cell_start, 0, (g.ncells + 1) * sizeof(uint32_t), s));
+        return SJCS_OK;
+    }
+    const int kb = grid_key_bits(g);
+    if (kb > kGridMaxDirectBits) return fail(SJCS_ERR_INVALID, "grid of %d key bits needs two partition passes", kb);
+    const int sb = segment_bits(kb), bits_top = std::max(0, kb - sb);
+    const uint64_t nseg = (g.ncells + (1ull << sb) - 1) >> sb;  // <= 512
+    const uint64_t ntiles = (n + PB_TILE - 1) / PB_TILE;
+    const int aligned = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
+    int rc = set_partition_smem();
+    if (rc) return rc;
+    k_pb_top_hist<<<(unsigned)ntiles, PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, g, sb, b.top, 1u);
+    SJCS_LAUNCH_CHECK();
+    rc = exclusive_scan_u32(b.top, nseg + 1, s, nullptr, b.cursors);
+    if (rc) return rc;
+    k_pb_partition<false><<<(unsigned)ntiles, PB_THREADS, PB_SMEM, s>>>(d_xyz, aligned, nullptr, nullptr, nullptr, n, g,
+                                                                        sb, bits_top, 0, b.cursors, b.tmp, nullptr, sb,
+                                                                        0u);
+    SJCS_LAUNCH_CHECK();
+    k_pb_cells<<<(unsigned)(g.ncells / PB_GROUP_CELLS + 1), PB_THREADS, PB_SMEM, s>>>(b.tmp, b.top, nseg, sb, g.ncells,
+                                                                                      b.cell_start, b.pts);
+    SJCS_LAUNCH_CHECK();
+    return SJCS_OK;
+}
 
 GridGeom auto_grid(uint64_t n, float radius_hint, const uint32_t* grid_req) {
     GridGeom g{};
@@ -632,34 +670,23 @@ int grid_key_bits(const GridGeom& g) {
     return key_bits;
 }
 
-int grid_digit_bits(const GridGeom& g) {
-    const int kb = grid_key_bits(g);
-    return (kb > 24 && kb <= 27) ? 9 : 8;  // three passes instead of four
-}
+namespace {
+// Buffers of the stable LSD sort (cell keys of more than 30 bits).
+struct LsdBuffers {
+    float4* pts;       // n sorted particles (output)
+    uint32_t* kfinal;  // n sorted keys
+    uint32_t *kx, *ky; // n
+    uint4 *px, *py;    // n
+    uint32_t* hist;    // RS_BINS * ceil(n / 4096)
+};
 
-template <int BITS, class PayOp0>
-int sort_particles(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, PayOp0 pop0,
-                   cudaStream_t s) {
-    return radix_sort_records<BITS>(n, grid_key_bits(g), KeysFromParticles{d_xyz, g}, pop0,
-                                    SinkParticles{b.kfinal, reinterpret_cast<uint4*>(b.pts)}, b.kx, b.px, b.ky,
-                                    b.py, b.hist, s, b.partials);
+template <class PayOp0>
+int sort_particles(const float* d_xyz, uint64_t n, const GridGeom& g, const LsdBuffers& b, PayOp0 pop0, cudaStream_t s) {
+    return radix_sort_records(n, grid_key_bits(g), KeysFromParticles{d_xyz, g}, pop0,
+                              SinkParticles{b.kfinal, reinterpret_cast<uint4*>(b.pts)}, b.kx, b.px, b.ky, b.py,
+                              b.hist, s);
 }
-
-int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s) {
-    static_assert(sizeof(Gap) == 12, "gap records are 12 bytes");
-    // A 16-byte-aligned particle array is staged tile by tile in the first
-    // pass; any other alignment is read particle by particle.
-    const bool staged = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
-    int rc;
-    if (b.digit_bits == 9)
-        rc = staged ? sort_particles<9>(d_xyz, n, g, b, PayFromXyzStaged{d_xyz}, s)
-                    : sort_particles<9>(d_xyz, n, g, b, PayFromParticles{d_xyz}, s);
-    else
-        rc = staged ? sort_particles<8>(d_xyz, n, g, b, PayFromXyzStaged{d_xyz}, s)
-                    : sort_particles<8>(d_xyz, n, g, b, PayFromParticles{d_xyz}, s);
-    if (rc) return rc;
-    return fill_cell_table(b.kfinal, n, g.ncells, b.cell_start, b.gaps, b.ngaps, s);
-}
+}  // namespace
 
 int fill_cell_table(const uint32_t* sorted_cells, uint64_t n, uint64_t ncells, uint32_t* cell_start, void* gaps,
                     uint32_t* ngaps, cudaStream_t s) {
@@ -685,26 +712,27 @@ int build_grid_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, const GridGe
     if (grid_key_bits(g) <= PB_MAX_KEY_BITS)
         return build_grid_partitioned(d_xyz, n, g, reinterpret_cast<float4*>(idx->pts), idx->cell_start, s);
 
-    GridBuildBuffers b{};
+    LsdBuffers b{};
     b.pts = idx->pts;
-    b.cell_start = idx->cell_start;
     const uint64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
-    b.digit_bits = grid_digit_bits(g);
-    const int passes = (grid_key_bits(g) + b.digit_bits - 1) / b.digit_bits;
     StreamScratch scr(s);  // freed (stream-ordered) on every return path
+    void* gaps = nullptr;
+    uint32_t* ngaps = nullptr;
     SJCS_CUDA_TRY(scr.alloc(&b.kfinal, nalloc * sizeof(uint32_t)));
-    if (passes > 1) {
-        SJCS_CUDA_TRY(scr.alloc(&b.kx, nalloc * sizeof(uint32_t)));
-        SJCS_CUDA_TRY(scr.alloc(&b.px, nalloc * sizeof(uint4)));
-    }
-    if (passes > 2) {
-        SJCS_CUDA_TRY(scr.alloc(&b.ky, nalloc * sizeof(uint32_t)));
-        SJCS_CUDA_TRY(scr.alloc(&b.py, nalloc * sizeof(uint4)));
-    }
-    SJCS_CUDA_TRY(scr.alloc(&b.hist, ((uint64_t)(1u << b.digit_bits) * (ntiles ? ntiles : 1)) * sizeof(uint32_t)));
-    SJCS_CUDA_TRY(scr.alloc(&b.gaps, kGridGaps * sizeof(Gap)));
-    SJCS_CUDA_TRY(scr.alloc(&b.ngaps, sizeof(uint32_t)));
-    return build_grid_into(d_xyz, n, g, b, s);
+    SJCS_CUDA_TRY(scr.alloc(&b.kx, nalloc * sizeof(uint32_t)));  // keys of 31 bits: four passes
+    SJCS_CUDA_TRY(scr.alloc(&b.px, nalloc * sizeof(uint4)));
+    SJCS_CUDA_TRY(scr.alloc(&b.ky, nalloc * sizeof(uint32_t)));
+    SJCS_CUDA_TRY(scr.alloc(&b.py, nalloc * sizeof(uint4)));
+    SJCS_CUDA_TRY(scr.alloc(&b.hist, ((uint64_t)RS_BINS * (ntiles ? ntiles : 1)) * sizeof(uint32_t)));
+    SJCS_CUDA_TRY(scr.alloc(&gaps, kGridGaps * sizeof(Gap)));
+    SJCS_CUDA_TRY(scr.alloc(&ngaps, sizeof(uint32_t)));
+    // A 16-byte-aligned particle array is staged tile by tile in the first
+    // pass; any other alignment is read particle by particle.
+    const bool staged = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
+    const int rc = staged ? sort_particles(d_xyz, n, g, b, PayFromXyzStaged{d_xyz}, s)
+                          : sort_particles(d_xyz, n, g, b, PayFromParticles{d_xyz}, s);
+    if (rc) return rc;
+    return fill_cell_table(b.kfinal, n, g.ncells, idx->cell_start, gaps, ngaps, s);
 }
 
 }  // namespace sjcs

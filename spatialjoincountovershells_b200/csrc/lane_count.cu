@@ -119,9 +119,9 @@ __device__ __noinline__ void serial_count(const CountParams& p, float4 c, uint32
             for (uint32_t j = p.mcs[f][rc + im.x0]; j < e; ++j) {
                 const float4 v = p.mpts[f][j];
                 if (flags & kItemZone)
-                    test_candidate<BIN_LUT, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
+                    test_candidate<BIN_BSEARCH, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
                 else
-                    test_candidate<BIN_LUT, true>(p, im, v, true, row, p.r2, p.lut);
+                    test_candidate<BIN_BSEARCH, true>(p, im, v, true, row, p.r2, p.lut);
             }
         }
 }
@@ -404,9 +404,9 @@ __device__ __forceinline__ void count_item(const CountParams& p, const LaneParam
         row_issue(pf, im, rb, lane, gy, gz, &a, &e);
         if (exactly) {
             if (it.y & kItemZone)
-                run_rows_part<BIN_LUT, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
+                run_rows_part<BIN_BSEARCH, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
             else
-                run_rows_part<BIN_LUT, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
+                run_rows_part<BIN_BSEARCH, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
             continue;
         }
         // this warp's share of the rows' candidates, [tb, te) of the flattened sequence
@@ -438,7 +438,7 @@ __device__ __forceinline__ void count_item(const CountParams& p, const LaneParam
         };
         // distances from safe2 on, which the slots leave out
         auto zone_test = [&](const float4& v) {
-            if (v.x != INFINITY) test_candidate<BIN_LUT, true, true>(pf, im, v, true, row, p.r2, p.lut, q.safe2);
+            if (v.x != INFINITY) test_candidate<BIN_BSEARCH, true, true>(pf, im, v, true, row, p.r2, p.lut, q.safe2);
         };
         const uint32_t excl = incl - len;
         const uint32_t lo = max(excl, tb), hi = min(incl, te);
@@ -561,13 +561,16 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
 }  // namespace
 
 bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
-    if (!q->lane.nslots || q->nlut == 0 || !p.prune || p.nhalos >= (1ull << 29)) return false;
+    if (!q->lane.nslots || !p.prune || p.nhalos >= (1ull << 29)) return false;
     for (int i = 0; i < p.nidx; ++i)
         if (p.mn[i] >= kEndSlot) return false;
     return true;
 }
 
-int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s) {
+uint64_t lane_list_items(uint64_t nhalos, int nidx) { return (uint64_t)nidx * (nhalos + nhalos / 2 + 1024); }
+
+int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s,
+                      const LaneScratch* given) {
     const auto& L = qq->lane;
     LaneParams q{};
     q.slots = L.slots;
@@ -583,13 +586,19 @@ int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p,
     std::memcpy(&km, &p.r2max, 4);
     q.zone = km - q.zone0;
     q.cmax = L.cmax;
-    q.cap = (uint32_t)std::min<uint64_t>((uint64_t)p.nidx * (p.nhalos + p.nhalos / 2 + 1024), 0xffffffffull);
     StreamScratch scr(s);
-    uint32_t* ctl = nullptr;
-    SJCS_CUDA_TRY(scr.alloc(&ctl, 32 + (uint64_t)q.cap * sizeof(uint2)));
-    SJCS_CUDA_TRY(cudaMemsetAsync(ctl, 0, 32, s));
-    q.ctl = ctl;
-    q.list = reinterpret_cast<uint2*>(ctl + 8);
+    if (given) {
+        q.ctl = given->ctl;
+        q.list = given->list;
+        q.cap = given->cap;
+    } else {
+        q.cap = (uint32_t)std::min<uint64_t>(lane_list_items(p.nhalos, p.nidx), 0xffffffffull);
+        uint32_t* ctl = nullptr;
+        SJCS_CUDA_TRY(scr.alloc(&ctl, kLaneCtlWords * sizeof(uint32_t) + (uint64_t)q.cap * sizeof(uint2)));
+        SJCS_CUDA_TRY(cudaMemsetAsync(ctl, 0, kLaneCtlWords * sizeof(uint32_t), s));
+        q.ctl = ctl;
+        q.list = reinterpret_cast<uint2*>(ctl + kLaneCtlWords);
+    }
     // one block per SM (neighbouring batches share its L1); blocks of fewer
     // warps when there are not enough batches for every SM
     const uint64_t nbatch = (p.nhalos + 31) / 32;

@@ -19,13 +19,15 @@
 // with the library.  Make that first call before any stream capture too.
 // All calls share the array and it keeps the last call's contents, so calls
 // that overlap on the GPU (two streams, two host threads) race and must be
-// serialised by the caller; the only state that must start at zero (the
-// cell-table gap counter) is cleared by each call.
+// serialised by the caller; what must start at zero (digit counts, list
+// control words) is cleared by each call.
+#include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <mutex>
+#include <vector>
 
-#include "radix_sort.cuh"
+#include "count_common.cuh"
+#include "lane_count.cuh"
 #include "sjcs_internal.cuh"
 
 namespace sjcs {
@@ -35,27 +37,30 @@ constexpr uint64_t kNP = SJCS_NOALLOC_MAX_PARTICLES;
 constexpr uint64_t kNH = SJCS_NOALLOC_MAX_HALOS;
 constexpr uint64_t kNC = SJCS_NOALLOC_MAX_CELLS;
 constexpr int kNR = SJCS_NOALLOC_MAX_SHELLS;
+constexpr int kMaxTable = 640;  // lane slots that travel with the launch (parameters stay under 4 KB)
 
 constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
-constexpr uint64_t kTiles = (kNP + RS_TILE - 1) / RS_TILE;
 // byte offsets of the sub-buffers (each 256-byte aligned)
+constexpr uint32_t kListItems = (uint32_t)(kNH + kNH / 2 + 1024);  // lane_list_items(kNH, 1)
 constexpr uint64_t kOffPts = 0;
 constexpr uint64_t kOffCells = align256(kOffPts + kNP * 16);
-constexpr uint64_t kOffKFinal = align256(kOffCells + (kNC + 1) * 4);
-constexpr uint64_t kOffKX = align256(kOffKFinal + kNP * 4);
-constexpr uint64_t kOffKY = align256(kOffKX + kNP * 4);
-constexpr uint64_t kOffPX = align256(kOffKY + kNP * 4);
-constexpr uint64_t kOffPY = align256(kOffPX + kNP * 16);
-constexpr uint64_t kOffHist = align256(kOffPY + kNP * 16);
-constexpr uint64_t kOffPartials = align256(kOffHist + (uint64_t)RS_BINS * kTiles * 4);
-constexpr uint64_t kOffGaps = align256(kOffPartials + 256 * 4);
-constexpr uint64_t kOffNGaps = align256(kOffGaps + (uint64_t)kGridGaps * 12);
-constexpr uint64_t kOffHalos = align256(kOffNGaps + 4);
+constexpr uint64_t kOffTmp = align256(kOffCells + (kNC + 1) * 4);
+constexpr uint64_t kOffTop = align256(kOffTmp + kNP * 16);
+constexpr uint64_t kOffCursors = align256(kOffTop + 513 * 4);
+constexpr uint64_t kOffHalos = align256(kOffCursors + 513 * 4);
 constexpr uint64_t kOffR2 = align256(kOffHalos + kNH * 16);
-constexpr uint64_t kScratchBytes = align256(kOffR2 + (uint64_t)kNR * 4);
-static_assert(kScratchBytes == SJCS_NOALLOC_SCRATCH_BYTES, "keep the header's scratch size in step");
+constexpr uint64_t kOffSlots = align256(kOffR2 + (uint64_t)kNR * 4);
+constexpr uint64_t kOffCtl = align256(kOffSlots + (uint64_t)kMaxTable * 4);
+constexpr uint64_t kOffList = align256(kOffCtl + (uint64_t)kLaneCtlWords * 4);
+constexpr uint64_t kScratchBytes = align256(kOffList + (uint64_t)kListItems * 8);
+static_assert(kScratchBytes <= SJCS_NOALLOC_SCRATCH_BYTES, "the scratch array holds every buffer");
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[SJCS_NOALLOC_SCRATCH_BYTES];
+
+// Pairs up to which every particle is tested against every halo: at 2^24 that
+// took 35-39 us a call and the index 45-47, at 2^25 65 and about 47 (2^23: 21
+// and 59; a call of 2003 x 97 24, of which the caller spends 20, was 73).
+constexpr uint64_t kDirectPairs = 1ull << 24;
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
@@ -79,20 +84,112 @@ int scratch_address(unsigned char** out) {
     return SJCS_OK;
 }
 
-// The padded radius table travels as a kernel argument (copied at launch),
-// so no host buffer has to outlive the call.
+// The padded radius table and the lane slots travel as kernel arguments
+// (copied at launch), so no host buffer has to outlive the call.
 struct R2Table {
     float v[kNR];
 };
-__global__ void k_put_r2(R2Table t, int pad, float* __restrict__ out) {
-    for (int i = threadIdx.x; i < pad; i += blockDim.x) out[i] = t.v[i];
+struct Tables {
+    R2Table r2;
+    uint32_t slots[kMaxTable];
+};
+
+// Everything the build and the count start from: the tables, the cleared
+// digit counts and list control words, and the halos in the caller's order.
+__global__ void __launch_bounds__(256) k_noalloc_prep(const __grid_constant__ Tables t, int pad, int nslots,
+                                                      const char* __restrict__ base, size_t stride, uint64_t nh,
+                                                      float* __restrict__ r2, uint32_t* __restrict__ slots,
+                                                      uint32_t* __restrict__ top, uint32_t* __restrict__ ctl,
+                                                      float4* __restrict__ halos) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0) {
+        for (int k = threadIdx.x; k < pad; k += blockDim.x) r2[k] = t.r2.v[k];
+        for (int k = threadIdx.x; k < nslots; k += blockDim.x) slots[k] = t.slots[k];
+        for (int k = threadIdx.x; k < 513; k += blockDim.x) top[k] = 0u;
+        if (threadIdx.x < kLaneCtlWords) ctl[threadIdx.x] = 0u;
+    }
+    if (i < nh) {
+        const float* p = reinterpret_cast<const float*>(base + i * stride);
+        halos[i] = make_float4(p[0], p[1], p[2], __uint_as_float((uint32_t)i));
+    }
 }
 
-__global__ void k_pack_halos(const char* __restrict__ base, size_t stride, uint64_t nh, float4* __restrict__ out) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nh) return;
-    const float* p = reinterpret_cast<const float*>(base + i * stride);
-    out[i] = make_float4(p[0], p[1], p[2], __uint_as_float((uint32_t)i));
+// Few enough pairs: every particle against every halo, no index.  A warp takes
+// four halos and every nslice-th run of 32 particles, so a particle is loaded
+// once for four tests.  Nearly all pairs fail the compare of the distance with
+// r2max; one that does not, and every shifted image, takes the reference's
+// predicate literally (test_candidate) into the warp's shared counters.
+constexpr int kDirectWarps = 8, kDirectHalos = 4;
+template <int BIN>
+__global__ void __launch_bounds__(kDirectWarps * 32)
+k_count_direct(const __grid_constant__ count::CountParams p, const __grid_constant__ R2Table t,
+               const float* __restrict__ xyz, uint32_t n, const char* __restrict__ base, size_t stride, uint32_t nslice) {
+    __shared__ float tab[kNR];
+    extern __shared__ uint32_t cnt_all[];  // [warp][halo][shell]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t* cnt = cnt_all + warp * kDirectHalos * p.nrads;
+    for (int i = threadIdx.x; i < p.pad; i += blockDim.x) tab[i] = t.v[i];
+    for (int i = lane; i < kDirectHalos * p.nrads; i += 32) cnt[i] = 0u;
+    __syncthreads();
+    const uint32_t item = blockIdx.x * kDirectWarps + (uint32_t)warp;
+    const uint32_t h0 = item / nslice * kDirectHalos, slice = item % nslice;
+    if (h0 >= p.nhalos) return;
+    float cx[kDirectHalos], cy[kDirectHalos], cz[kDirectHalos];
+    uint32_t F[kDirectHalos], anyF = 0u;
+#pragma unroll
+    for (int k = 0; k < kDirectHalos; ++k) {
+        cx[k] = cy[k] = cz[k] = NAN;  // no halo: no distance passes
+        F[k] = 0u;
+        if (h0 + k >= p.nhalos) continue;
+        const float* hp = reinterpret_cast<const float*>(base + (uint64_t)(h0 + k) * stride);
+        cx[k] = hp[0];
+        cy[k] = hp[1];
+        cz[k] = hp[2];
+        if (p.periodic)
+            F[k] = ((__fsub_rn(cx[k], p.half) < kBoxLow) | (__fadd_rn(cx[k], p.half) > kBoxUpp) ? 1u : 0u) |
+                   ((__fsub_rn(cy[k], p.half) < kBoxLow) | (__fadd_rn(cy[k], p.half) > kBoxUpp) ? 2u : 0u) |
+                   ((__fsub_rn(cz[k], p.half) < kBoxLow) | (__fadd_rn(cz[k], p.half) > kBoxUpp) ? 4u : 0u);
+        anyF |= F[k];
+    }
+    auto literal = [&](float x, float y, float z, const float4& v, bool live, int k) {
+        count::Image im;
+        im.cx = x;
+        im.cy = y;
+        im.cz = z;
+        im.lox = __fsub_rn(x, p.half);
+        im.hix = __fadd_rn(x, p.half);
+        im.loy = __fsub_rn(y, p.half);
+        im.hiy = __fadd_rn(y, p.half);
+        im.loz = __fsub_rn(z, p.half);
+        im.hiz = __fadd_rn(z, p.half);
+        count::test_candidate<BIN, false>(p, im, v, live, cnt + k * p.nrads, tab, nullptr);
+    };
+    auto image = [&](float c) {  // min_oob takes precedence over max_oob on an axis (MultiRangeCount.c:38-43)
+        return __fsub_rn(c, p.half) < kBoxLow ? __fadd_rn(c, kBoxUpp) : __fsub_rn(c, kBoxUpp);
+    };
+#pragma unroll 2
+    for (uint32_t j0 = slice * 32u; j0 < n; j0 += nslice * 32u) {
+        const uint32_t j = j0 + (uint32_t)lane;
+        const bool live = j < n;
+        float4 v = make_float4(NAN, 0.f, 0.f, 0.f);
+        if (live) v = make_float4(xyz[3 * (uint64_t)j], xyz[3 * (uint64_t)j + 1], xyz[3 * (uint64_t)j + 2], 0.f);
+#pragma unroll
+        for (int k = 0; k < kDirectHalos; ++k) {
+            const float dx = __fsub_rn(v.x, cx[k]), dy = __fsub_rn(v.y, cy[k]), dz = __fsub_rn(v.z, cz[k]);
+            const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+            if (BIN == count::BIN_FIRST_MATCH || dist < p.r2max) literal(cx[k], cy[k], cz[k], v, live, k);
+        }
+        if (anyF) {
+#pragma unroll
+            for (int k = 0; k < kDirectHalos; ++k)
+                for (uint32_t S = F[k]; S; S = (S - 1u) & F[k])
+                    literal((S & 1u) ? image(cx[k]) : cx[k], (S & 2u) ? image(cy[k]) : cy[k],
+                            (S & 4u) ? image(cz[k]) : cz[k], v, live, k);
+        }
+    }
+    __syncwarp();
+    for (int i = lane; i < kDirectHalos * p.nrads; i += 32)
+        if (cnt[i]) atomicAdd(p.counts + (uint64_t)h0 * (uint64_t)p.nrads + (uint64_t)i, cnt[i]);
 }
 
 }  // namespace
@@ -123,23 +220,72 @@ extern "C" int sjcs_count_noalloc(const float* d_xyz, uint64_t n, const float* d
     int rc = scratch_address(&base);
     if (rc) return rc;
 
-    // radius table, as sjcs_query_create builds it (binary-search binning),
-    // written by a kernel that receives it by value
-    R2Table tab;
+    // radius table, as sjcs_query_create builds it (binary-search binning)
+    Tables tab;
     int pad = 1;
     while (pad < nrads) pad <<= 1;
     bool mono = true;
-    for (int i = 0; i < pad; ++i) tab.v[i] = i < nrads ? r2[i] : INFINITY;
+    for (int i = 0; i < pad; ++i) tab.r2.v[i] = i < nrads ? r2[i] : INFINITY;
     for (int i = 0; i < nrads; ++i) {
         if (std::isnan(r2[i])) mono = false;
         if (i + 1 < nrads && !(r2[i] <= r2[i + 1])) mono = false;
     }
-    float* d_r2 = reinterpret_cast<float*>(base + kOffR2);
-    k_put_r2<<<1, kNR, 0, s>>>(tab, pad, d_r2);
-    SJCS_LAUNCH_CHECK();
+    const float R = (float)std::sqrt((double)r2[nrads - 1]);
+    const float half = (flags & SJCS_QUERY_PERIODIC) ? R : r2[nrads - 1];
+    if (n == 0 || nhalos == 0) return SJCS_OK;
+
+    sjcs_ctx c;
+    c.magic = kCtxMagic;
+    SJCS_CUDA_TRY(cudaGetDevice(&c.device));
+    SJCS_CUDA_TRY(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
+
+    if (n * nhalos <= kDirectPairs) {
+        count::CountParams p{};
+        p.nhalos = nhalos;
+        p.nrads = nrads;
+        p.pad = pad;
+        p.half = half;
+        p.r2max = r2[nrads - 1];
+        p.periodic = (flags & SJCS_QUERY_PERIODIC) ? 1 : 0;
+        p.counts = d_counts;
+        // slices: enough warps for every SM, at least 4 runs of 32 particles each
+        const uint64_t runs = (n + 31) / 32, warps = (uint64_t)c.num_sms * 32;
+        const uint64_t groups = (nhalos + kDirectHalos - 1) / kDirectHalos;
+        const uint32_t nslice = (uint32_t)std::max<uint64_t>(1, std::min((runs + 3) / 4, (warps + groups - 1) / groups));
+        const unsigned blocks = (unsigned)((groups * nslice + kDirectWarps - 1) / kDirectWarps);
+        auto kern = mono ? k_count_direct<count::BIN_BSEARCH> : k_count_direct<count::BIN_FIRST_MATCH>;
+        kern<<<blocks, kDirectWarps * 32, (size_t)kDirectWarps * kDirectHalos * nrads * sizeof(uint32_t), s>>>(
+            p, tab.r2, d_xyz, (uint32_t)n, reinterpret_cast<const char*>(d_halo_xyz), stride_bytes, nslice);
+        SJCS_LAUNCH_CHECK();
+        return SJCS_OK;
+    }
+
+    // objects that only point at the scratch
+    sjcs_query q{};
+    q.nhalos = nhalos;
+    q.nrads = nrads;
+    q.flags = flags;
+    q.pad = pad;
+    q.monotone = mono;
+    q.r2max = r2[nrads - 1];
+    q.R = R;
+    q.half = half;
+    q.halos = reinterpret_cast<float4*>(base + kOffHalos);
+    q.counts = d_counts;
+    q.d_r2 = reinterpret_cast<float*>(base + kOffR2);
+    q.d_lut = nullptr;
+    q.nlut = 0;
+    std::vector<uint32_t> slots;
+    if (mono) build_lane_table(r2, nrads, half, &slots, &q.lane);
+    if (slots.size() > (size_t)kMaxTable) q.lane = {};
+    std::copy(slots.begin(), slots.begin() + q.lane.nslots, tab.slots);
+    q.lane.slots = reinterpret_cast<uint32_t*>(base + kOffSlots);
+    LaneScratch list{};
+    list.ctl = reinterpret_cast<uint32_t*>(base + kOffCtl);
+    list.list = reinterpret_cast<uint2*>(base + kOffList);
+    list.cap = kListItems;
 
     // the grid index, in the scratch array
-    const float R = (float)std::sqrt((double)r2[nrads - 1]);
     GridGeom g = auto_grid(n, std::isfinite(R) ? R : 0.0f, nullptr);
     while (g.ncells > kNC) {
         int G[3] = {std::max(1, g.G[0] * 7 / 8), std::max(1, g.G[1] * 7 / 8), std::max(1, g.G[2] * 7 / 8)};
@@ -152,49 +298,20 @@ extern "C" int sjcs_count_noalloc(const float* d_xyz, uint64_t n, const float* d
     GridBuildBuffers b{};
     b.pts = reinterpret_cast<float4*>(base + kOffPts);
     b.cell_start = reinterpret_cast<uint32_t*>(base + kOffCells);
-    b.kfinal = reinterpret_cast<uint32_t*>(base + kOffKFinal);
-    b.kx = reinterpret_cast<uint32_t*>(base + kOffKX);
-    b.ky = reinterpret_cast<uint32_t*>(base + kOffKY);
-    b.px = reinterpret_cast<uint4*>(base + kOffPX);
-    b.py = reinterpret_cast<uint4*>(base + kOffPY);
-    b.hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-    b.partials = reinterpret_cast<uint32_t*>(base + kOffPartials);
-    b.gaps = base + kOffGaps;
-    b.ngaps = reinterpret_cast<uint32_t*>(base + kOffNGaps);
+    b.tmp = reinterpret_cast<float4*>(base + kOffTmp);
+    b.top = reinterpret_cast<uint32_t*>(base + kOffTop);
+    b.cursors = reinterpret_cast<uint32_t*>(base + kOffCursors);
+    k_noalloc_prep<<<(unsigned)((nhalos + 255) / 256), 256, 0, s>>>(
+        tab, pad, q.lane.nslots, reinterpret_cast<const char*>(d_halo_xyz), stride_bytes, nhalos, q.d_r2, q.lane.slots,
+        b.top, list.ctl, q.halos);
+    SJCS_LAUNCH_CHECK();
     rc = build_grid_into(d_xyz, n, g, b, s);
     if (rc) return rc;
 
-    // halos in the caller's order (no sort: inputs are small)
-    float4* halos = reinterpret_cast<float4*>(base + kOffHalos);
-    if (nhalos) {
-        k_pack_halos<<<(unsigned)((nhalos + 255) / 256), 256, 0, s>>>(reinterpret_cast<const char*>(d_halo_xyz),
-                                                                       stride_bytes, nhalos, halos);
-        SJCS_LAUNCH_CHECK();
-    }
-
-    // count through the regular kernel, on objects that only point at the scratch
-    sjcs_ctx c;
-    c.magic = kCtxMagic;
-    SJCS_CUDA_TRY(cudaGetDevice(&c.device));
-    SJCS_CUDA_TRY(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
     sjcs_index idx{};
     idx.n = n;
     idx.geom = g;
     idx.pts = b.pts;
     idx.cell_start = b.cell_start;
-    sjcs_query q{};
-    q.nhalos = nhalos;
-    q.nrads = nrads;
-    q.flags = flags;
-    q.pad = pad;
-    q.monotone = mono;
-    q.r2max = r2[nrads - 1];
-    q.R = R;
-    q.half = (flags & SJCS_QUERY_PERIODIC) ? R : r2[nrads - 1];
-    q.halos = halos;
-    q.counts = d_counts;
-    q.d_r2 = d_r2;
-    q.d_lut = nullptr;
-    q.nlut = 0;
-    return launch_shell_count(&c, &q, &idx, s);
+    return launch_shell_count_noalloc(&c, &q, &idx, list, s);
 }

@@ -628,6 +628,14 @@ int launch_shell_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx
     return launch_static(ctx, p, bin, big, smem, s, false);
 }
 
+int launch_shell_count_noalloc(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx, const LaneScratch& scratch,
+                               cudaStream_t s) {
+    if (q->nhalos == 0 || idx->n == 0) return SJCS_OK;
+    const CountParams p = count_params(q, idx);
+    if (lane_count_applies(q, p)) return launch_lane_count(ctx, q, p, s, &scratch);
+    return launch_static(ctx, p, bin_mode(q), big_tables(q), count_smem(q), s, false);
+}
+
 int launch_shell_count_multi(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* const* idx, int k,
                              cudaStream_t s) {
     if (k < 1 || k > kMaxFused) return fail(SJCS_ERR_INVALID, "between 1 and %d indexes per fused count", kMaxFused);

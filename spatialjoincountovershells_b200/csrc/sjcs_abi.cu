@@ -197,6 +197,8 @@ void build_shell_lut(const float* r2, int nrads, std::vector<uint32_t>* lut, uin
     *shift_out = shift;
 }
 
+}  // namespace
+
 // Slots of the lane-per-halo count over the bit patterns of squared distances
 // (see lane_count.cu).  Shells are counted by the lanes for distances below
 // safe2: with d = p - c rounded per axis and the box bounds rounded from c -+
@@ -249,8 +251,6 @@ void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32
     t->shift = shift;
     t->ncol = (int)th.size();
 }
-
-}  // namespace
 
 constexpr uint32_t kParamSlots = 8;
 constexpr size_t kParamSlotBytes = 64 << 10;

@@ -252,6 +252,9 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
 // zeroed accumulators, Morton-sorted halos) and schedule resolution
 int query_prepare(sjcs_ctx* ctx, const float* d_halo_xyz, size_t stride, uint64_t nhalos, const float* r2,
                   int nrads, int flags, sjcs_query* q, cudaStream_t s);
+// Slots of the lane-per-halo count for a non-decreasing table (sjcs_abi.cu);
+// leaves t->nslots 0 when the table does not fit the form.
+void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32_t>* slots, sjcs_query::LaneTable* t);
 struct Schedule;
 Schedule schedule_for(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx);
 Schedule resolve(const sjcs_schedule& in);
@@ -300,26 +303,19 @@ int exclusive_scan_u32(uint32_t* d_data, uint64_t m, cudaStream_t s, uint32_t* p
                        uint32_t* copy = nullptr);
 uint64_t scan_partials_needed(uint64_t m);
 
-// index_build.cu: the stable LSD grid build on caller-provided buffers (no
-// allocation; the fixed-buffer entry point and cell keys of more than 30 bits).
+// index_build.cu: the grid build on caller-provided buffers (no allocation)
+// for cell keys of at most 21 bits, which take one partition pass.
 struct GridBuildBuffers {
-    float4* pts;          // n sorted particles (output)
-    uint32_t* cell_start; // ncells + 1 (output)
-    uint32_t* kfinal;     // n
-    uint32_t* kx;         // n (needed for two or more passes)
-    uint4* px;            // n
-    uint32_t* ky;         // n (needed for three or more passes)
-    uint4* py;            // n
-    uint32_t* hist;       // 2^digit_bits * ceil(n / 4096)
-    uint32_t* partials;   // scan_partials_needed(2^digit_bits * ceil(n / 4096)), or null
-    void* gaps;           // kGridGaps gap records (12 bytes each)
-    uint32_t* ngaps;      // 1
-    int digit_bits;       // radix digit: 9, or 8 (also for 0)
+    float4* pts;           // n particles grouped by cell (output)
+    uint32_t* cell_start;  // ncells + 1 (output)
+    float4* tmp;           // n records
+    uint32_t* top;         // 513, zeroed
+    uint32_t* cursors;     // 513
 };
+constexpr int kGridMaxDirectBits = 21;
+int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s);
 constexpr uint32_t kGridGaps = 1u << 16;
 int grid_key_bits(const GridGeom& g);
-int grid_digit_bits(const GridGeom& g);  // LSD build: 9 for 25-27-bit cell keys, else 8
-int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s);
 // cell_start[c] = first slot of cell c, from the cell ids of the sorted particles.
 int fill_cell_table(const uint32_t* sorted_cells, uint64_t n, uint64_t ncells, uint32_t* cell_start, void* gaps,
                     uint32_t* ngaps, cudaStream_t s);
