@@ -10,9 +10,13 @@
 //                walked the same way.
 // k_listed_count what does not suit a lane: images of more than 25 rows, and
 //                lanes with so many candidates that the rest of the warp
-//                would wait.  k_lane_count lists them; here a warp takes an
-//                item (or a part of a large one), reads its rows in windows
-//                of 32 slots and counts in 32-bit columns, one per lane.
+//                would wait.  k_lane_count lists them; here a warp takes two
+//                neighbouring items (or a part of them), reads the rows that
+//                reach either sphere in windows of 32 slots, tests a loaded
+//                candidate against both centres and counts in 16-bit columns,
+//                one per lane and halo.  Two halos of one clump share nearly
+//                all candidates, so the loads and the row bookkeeping are
+//                paid once for both.
 //
 // A candidate costs one float4 load, the eight fp32 operations of the
 // reference's distance, one lookup and one counter update; the box test and
@@ -33,11 +37,14 @@
 // slots, measured), so staging the candidates would not pay.  What bounds it:
 // the L1/shared data pipe (81 % of its peak, 47 % issue active).
 //
-// Measured (B200, count kernels of one call, before -> after): 1e7 uniform
-// halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.32 ms; 1e6 on 1e7 0.42 ->
-// 0.21; 1e6 clustered halos on 3e7 clustered particles 9.2 (static schedule)
-// and 7.1 (queue) -> 4.3; 1e6 on 5e7, R = 20, 64 shells 55 and 40.8 -> 24.6;
-// 1e5 on 2e7, R = 10 2.14 and 1.45 -> 0.94.
+// k_listed_count runs at 68 % of both the data pipe and issue.
+//
+// Measured (B200, count kernels of one call, warp-per-halo kernel -> this one):
+// 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.31 ms; 1e6 on
+// 1e7 0.42 -> 0.22; 1e6 clustered halos on 3e7 clustered particles 9.2 (static
+// schedule) and 7.1 (queue) -> 3.68, one item at a time 4.28; 1e6 on 5e7, R =
+// 20, 64 shells 55 and 40.8 -> 17.9, one item at a time 24.3; 1e5 on 2e7, R =
+// 10 2.14 and 1.45 -> 0.78, one at a time 0.90.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -57,15 +64,18 @@ constexpr int LN_WARPS = 16;
 constexpr int LN_ROWS = 25;       // rows of cells a lane walks
 constexpr uint32_t LN_PEND = 96;  // shifted images waiting per warp
 constexpr int LN_DEPTH = 4;       // candidates in flight per lane (2: 4.42 ms, 3: 4.35, 6: 4.34)
-constexpr int HV_WARPS = 4, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 6;
+// Listed items: five blocks of four warps per SM (96 registers; six with 80
+// spill and take 7 % longer, four 10 %).
+constexpr int HV_WARPS = 4, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 5;
+constexpr uint32_t kSpan = 1u << 20;  // candidates between two looks at what the 16-bit counters hold
 // Items above this many candidates (in the box's rows) are split into at
-// least 8 parts: one warp would need longer than the rest of the pass.
-// 16384 and 32768 were slower (clustered R = 20: 32.3 and 30.7 against 29.9 ms).
+// least 8 parts: one warp would need longer than the rest of the pass (16384
+// and 32768 took 8 and 3 % longer on clustered data, R = 20).
 constexpr uint32_t kHuge = 65536;
 constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles on this path
 // Mean row length from which listed rows are read one by one; shorter rows
 // are flattened first (14: 3 % slower, 24 and 64: within 1 %).
-constexpr uint32_t kLongRow = 40;
+constexpr uint32_t kLongRow = 40, kLongBoxRow = 60;  // of rows clipped to the sphere; of the whole box
 // Work of a lane's step for the whole warp, of 32 listed candidates and of a
 // listed item, in cycles of the data pipe: decides which lanes are listed.
 constexpr uint32_t kStepCost = 26, kWindowCost = 9, kItemCost = 100;
@@ -75,17 +85,17 @@ struct LaneParams {
     int nslots, kbase, shift, ncol;
     float safe2, cmax;
     int khi;               // last key of the slots less kbase
-    uint32_t mask;         // (1 << shift) - 1
     uint32_t zone0, zone;  // bit pattern of safe2; that of r2max less it
     // Items: the huge ones from the front of the list, the others from its end.
     uint2* __restrict__ list;  // (halo, flags)
     uint32_t cap;
-    uint32_t* __restrict__ ctl;  // [0] items asked for, [1] huge, [2] others, [3] claims
+    uint32_t* __restrict__ ctl;  // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase
 };
 
 // An item's flags: bits 0-2 the shifted axes, bits 3-4 the index to count.
 constexpr uint32_t kItemZone = 1u << 7;  // only distances from safe2 on
 constexpr uint32_t kItemFar = 1u << 8;   // centre beyond cmax: literal test throughout
+constexpr uint32_t kItemShort = 1u << 9; // short rows: flattened before they are read
 
 // Shared memory of one warp beside its counters.
 struct LaneRows {
@@ -243,7 +253,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     T = kHuge + 1u;
                 }
                 __syncwarp();
-                push_items(p, q, listed, T > kHuge, h, file | S | (far ? kItemFar : 0u), c, lane);
+                push_items(p, q, listed, T > kHuge, h, file | S | (far ? kItemFar : 0u) | (T < kLongBoxRow * im.nrows ? kItemShort : 0u), c, lane);
                 T = 0;
             }
             const int ny = mine ? im.ny : 0, nz = mine ? im.nz : 0;
@@ -317,7 +327,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                 }
                 coop |= T > tau;
             }
-            if (__any_sync(0xffffffffu, coop)) push_items(p, q, coop, T > kHuge, h, file | S, c, lane);
+            if (__any_sync(0xffffffffu, coop)) push_items(p, q, coop, T > kHuge, h, file | S | (T < kLongRow * m ? kItemShort : 0u), c, lane);
             if (steps) {
                 // the list ends in a row of slots past the particles, which load nothing
                 const uint32_t mm = coop ? 0u : m;
@@ -342,23 +352,26 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                         nl = *rl;
                     }
                 };
-                auto test = [&](const float4& v) {
+                auto find = [&](const float4& v) {
                     const float dx = __fsub_rn(v.x, c.x), dy = __fsub_rn(v.y, c.y), dz = __fsub_rn(v.z, c.z);
                     const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
                     const uint32_t key = __float_as_uint(dist);
                     z = __viaddmin_u32(key, 0u - q.zone0, z);
                     const uint32_t t = (uint32_t)__viaddmin_s32_relu((int)key, -q.kbase, q.khi);
-                    const uint32_t w = slots[t >> q.shift] + (t & q.mask);
-                    uint16_t* cnt = reinterpret_cast<uint16_t*>(mycol + (w >> q.shift) * 64u);
-                    *cnt = (uint16_t)(*cnt + 1);
+                    return ((slots[t >> q.shift] + t) >> q.shift) * 64u;
                 };
 #pragma unroll
                 for (int u = 0; u < LN_DEPTH; ++u) next(buf[u]);
                 for (uint32_t it = 0; it < steps; it += LN_DEPTH) {
+                    uint32_t at[LN_DEPTH];
+#pragma unroll
+                    for (int u = 0; u < LN_DEPTH; ++u) at[u] = find(buf[u]);
+#pragma unroll
+                    for (int u = 0; u < LN_DEPTH; ++u) next(buf[u]);
 #pragma unroll
                     for (int u = 0; u < LN_DEPTH; ++u) {
-                        test(buf[u]);
-                        next(buf[u]);
+                        uint16_t* cnt = reinterpret_cast<uint16_t*>(mycol + at[u]);
+                        *cnt = (uint16_t)(*cnt + 1);
                     }
                 }
                 if (__any_sync(0xffffffffu, z < q.zone)) push_items(p, q, z < q.zone, false, h, file | S | kItemZone, c, lane);
@@ -379,35 +392,140 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
     }
 }
 
-// Part `part` of `nparts` of a listed item (an even share of every 32 rows'
-// candidates).
-__device__ __forceinline__ void count_item(const CountParams& p, const LaneParams& q, const uint2 it, uint32_t part,
-                                           uint32_t nparts, uint32_t* __restrict__ cols, const uint32_t* __restrict__ slots,
-                                           int lane) {
-    const uint32_t S = it.y & 7u;
+// The centre an item counts.
+__device__ __forceinline__ float4 item_centre(const CountParams& p, const uint2 it) {
     float4 c = p.halos[it.x];
-    if (S & 1u) c.x = shifted(c.x, p.half);
-    if (S & 2u) c.y = shifted(c.y, p.half);
-    if (S & 4u) c.z = shifted(c.z, p.half);
+    if (it.y & 1u) c.x = shifted(c.x, p.half);
+    if (it.y & 2u) c.y = shifted(c.y, p.half);
+    if (it.y & 4u) c.z = shifted(c.z, p.half);
+    return c;
+}
+
+// The rare parts of a listed count stay out of line: inlined at every use they
+// made the kernel larger than the instruction cache (11 of 17 stall cycles
+// per issue were instruction fetches).
+
+// Each lane's candidate (slot j, or none: ~0) against one centre, counted
+// literally if its distance lies in the zone.
+__device__ __noinline__ void zone_count(const CountParams& p, const float4* __restrict__ pts, uint32_t j, float4 c,
+                                        float safe2) {
+    if (j == 0xffffffffu) return;
+    Image im;
+    im.cx = c.x;
+    im.cy = c.y;
+    im.cz = c.z;
+    im.lox = __fsub_rn(c.x, p.half);
+    im.hix = __fadd_rn(c.x, p.half);
+    im.loy = __fsub_rn(c.y, p.half);
+    im.hiy = __fadd_rn(c.y, p.half);
+    im.loz = __fsub_rn(c.z, p.half);
+    im.hiz = __fadd_rn(c.z, p.half);
+    test_candidate<BIN_BSEARCH, true, true>(p, im, __ldg(pts + j), true,
+                                            p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads, p.r2, p.lut,
+                                            safe2);
+}
+
+// A warp's counters of one halo ([shell][lane], 16 bits each) to the halo's row.
+__device__ __noinline__ void flush_columns(uint32_t* __restrict__ cols, int ncol, uint32_t* __restrict__ row, int lane) {
+    __syncwarp();
+    for (int s = lane; s < ncol; s += 32) {
+        uint32_t sum = 0;
+        const uint32_t* r = cols + s * 16;
+#pragma unroll 4
+        for (int j = 0; j < 16; ++j) {
+            const uint32_t w = r[(j + lane) & 15];
+            sum += (w & 0xffffu) + (w >> 16);
+        }
+        if (sum) atomicAdd(row + s, sum);
+    }
+    __syncwarp();
+    for (int i = lane; i < (ncol + 1) * 16; i += 32) cols[i] = 0u;
+    __syncwarp();
+}
+
+// Zone and far items: the literal test, straight into the count row.
+__device__ __noinline__ void count_literal(const CountParams& p, const LaneParams& q, const uint2 it, uint32_t part,
+                                              uint32_t nparts, int lane) {
+    const float4 c = item_centre(p, it);
     uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
     const Image im = make_image(p, c.x, c.y, c.z);
     float gy, gz;
     gap_tables(p, im, lane, &gy, &gz);
-    const bool exactly = (it.y & (kItemZone | kItemFar)) != 0u;
-    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols) + 4 * lane;
-    bool any = false;
     CountParams pf = p;
     pf.pts = p.mpts[(it.y >> 3) & 3u];
     pf.cs = p.mcs[(it.y >> 3) & 3u];
     for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
         uint32_t a, e;
         row_issue(pf, im, rb, lane, gy, gz, &a, &e);
-        if (exactly) {
-            if (it.y & kItemZone)
-                run_rows_part<BIN_BSEARCH, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
-            else
-                run_rows_part<BIN_BSEARCH, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
-            continue;
+        if (it.y & kItemZone)
+            run_rows_part<BIN_BSEARCH, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
+        else
+            run_rows_part<BIN_BSEARCH, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
+    }
+}
+
+// Part `part` of `nparts` of H listed items of one index, counted together:
+// the rows are those that reach any of the H spheres, and a candidate once
+// loaded is tested against every centre.
+template <int H, bool SHORT>
+__device__ __forceinline__ void count_items(const CountParams& p, const LaneParams& q, const uint2* it, uint32_t part,
+                                            uint32_t nparts, uint32_t* __restrict__ cols,
+                                            const uint32_t* __restrict__ slots, int lane) {
+    float4 c[H];
+    Image im;
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        c[k] = item_centre(p, it[k]);
+        const Image ik = make_image(p, c[k].x, c[k].y, c[k].z);
+        if (k == 0) {
+            im = ik;
+        } else {
+            im.x0 = min(im.x0, ik.x0);
+            im.x1 = max(im.x1, ik.x1);
+            im.y0 = min(im.y0, ik.y0);
+            im.y1 = max(im.y1, ik.y1);
+            im.z0 = min(im.z0, ik.z0);
+            im.z1 = max(im.z1, ik.z1);
+        }
+    }
+    im.ny = im.y1 - im.y0 + 1;
+    im.nz = im.z1 - im.z0 + 1;
+    const uint64_t nr = (uint64_t)im.ny * (uint64_t)im.nz;
+    im.nrows = nr > 0x80000000ull ? 0x80000000u : (uint32_t)nr;
+    const uint32_t f = (it[0].y >> 3) & 3u;
+    const float4* __restrict__ pts = p.mpts[f];
+    const uint32_t* __restrict__ cs = p.mcs[f];
+    const uint32_t colwords = (uint32_t)(q.ncol + 1) * 16u;
+    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols) + 4 * (lane >> 1);
+    const uint32_t one = (lane & 1) ? 65536u : 1u;
+    uint32_t held = 0;  // bound of any 16-bit counter
+    for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
+        // lane r: slot range of row rb + r, clipped in x to the spheres
+        uint32_t a = 0, e = 0;
+        const uint32_t r = rb + (uint32_t)lane;
+        if (r < im.nrows) {
+            int yy, zz, xa = im.x1 + 1, xb = im.x0 - 1;
+            row_yz(im, r, &yy, &zz);
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                const float gy = cell_gap(c[k].y, yy, p.h[1], p.g.G[1]), gz = cell_gap(c[k].z, zz, p.h[2], p.g.G[2]);
+                const float rem =
+                    __fadd_rn(__fsub_rn(__fsub_rn(p.r2p, __fmul_rn(gy, gy)), __fmul_rn(gz, gz)), p.r2slack);
+                if (rem >= 0.0f) {
+                    // approximate square root: its error (< 1e-6 relative) is far inside the margin
+                    float xr = rem > 0.0f ? __fmul_rn(rem, rsqrtf(rem)) : 0.0f;
+                    xr = __fadd_rn(xr, 1e-3f + 1e-6f * (fabsf(c[k].x) + xr));
+                    xa = min(xa, cell_of(__fsub_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
+                    xb = max(xb, cell_of(__fadd_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
+                }
+            }
+            xa = max(xa, im.x0);
+            xb = min(xb, im.x1);
+            if (xa <= xb) {
+                const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
+                a = __ldg(cs + rc + xa);
+                e = __ldg(cs + rc + xb + 1);
+            }
         }
         // this warp's share of the rows' candidates, [tb, te) of the flattened sequence
         const uint32_t len = e - a;
@@ -423,111 +541,140 @@ __device__ __forceinline__ void count_item(const CountParams& p, const LaneParam
             tb = (uint32_t)(((uint64_t)total * part) / nparts);
             te = (uint32_t)(((uint64_t)total * (part + 1u)) / nparts);
         }
-        if (tb == te) continue;
-        any = true;
         uint32_t z = 0xffffffffu;
-        auto test = [&](const float4& v) {
-            const float dx = __fsub_rn(v.x, c.x), dy = __fsub_rn(v.y, c.y), dz = __fsub_rn(v.z, c.z);
-            const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-            const uint32_t key = __float_as_uint(dist);
-            z = __viaddmin_u32(key, 0u - q.zone0, z);
-            const uint32_t t = (uint32_t)__viaddmin_s32_relu((int)key, -q.kbase, q.khi);
-            const uint32_t w = slots[t >> q.shift] + (t & q.mask);
-            uint32_t* cnt = reinterpret_cast<uint32_t*>(mycol + (w >> q.shift) * 128u);
-            *cnt += 1u;
+        // a candidate's counter offset per centre; the lookups of several
+        // candidates are in flight before their counters are touched
+        auto find = [&](const float4& v, uint32_t* at) {
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                const float dx = __fsub_rn(v.x, c[k].x), dy = __fsub_rn(v.y, c[k].y), dz = __fsub_rn(v.z, c[k].z);
+                const float dist = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                const uint32_t key = __float_as_uint(dist);
+                z = __viaddmin_u32(key, 0u - q.zone0, z);
+                const uint32_t t = (uint32_t)__viaddmin_s32_relu((int)key, -q.kbase, q.khi);
+                at[k] = ((slots[t >> q.shift] + t) >> q.shift) * 64u;
+            }
+        };
+        auto add = [&](const uint32_t* at) {
+#pragma unroll
+            for (int k = 0; k < H; ++k)
+                atomicAdd(reinterpret_cast<uint32_t*>(mycol + at[k]) + k * colwords, one);
         };
         // distances from safe2 on, which the slots leave out
-        auto zone_test = [&](const float4& v) {
-            if (v.x != INFINITY) test_candidate<BIN_BSEARCH, true, true>(pf, im, v, true, row, p.r2, p.lut, q.safe2);
+        auto zone_at = [&](uint32_t j) {
+#pragma unroll
+            for (int k = 0; k < H; ++k) zone_count(p, pts, j, c[k], q.safe2);
         };
         const uint32_t excl = incl - len;
-        const uint32_t lo = max(excl, tb), hi = min(incl, te);
-        uint32_t bal = __ballot_sync(0xffffffffu, lo < hi);
-        if (te - tb >= kLongRow * (uint32_t)__popc(bal)) {
-            // long rows: each in windows of 32 slots
-            const uint32_t rs = a + (lo - excl), re = a + (hi - excl);
-            while (bal) {
-                const int r = __ffs(bal) - 1;
-                bal &= bal - 1;
-                const uint32_t s0 = __shfl_sync(0xffffffffu, rs, r), s1 = __shfl_sync(0xffffffffu, re, r);
-                const float4* src = pf.pts + s0 + lane;
-                uint32_t left = s1 - s0;
-                for (; left >= 128u; left -= 128u, src += 128) {
-                    const float4 v0 = __ldg(src), v1 = __ldg(src + 32), v2 = __ldg(src + 64), v3 = __ldg(src + 96);
-                    test(v0);
-                    test(v1);
-                    test(v2);
-                    test(v3);
+        // at most 2^20 candidates at a time: 2^15 windows and 64 partial ones
+        for (uint32_t t0 = tb, t1; t0 < te; t0 = t1) {
+            t1 = te - t0 > kSpan ? t0 + kSpan : te;
+            const uint32_t lo = max(excl, t0), hi = min(incl, t1);
+            if constexpr (!SHORT) {
+                // each row in windows of 32 slots
+                uint32_t bal = __ballot_sync(0xffffffffu, lo < hi);
+                const uint32_t rs = a + (lo - excl), re = a + (hi - excl);
+                while (bal) {
+                    const int j = __ffs(bal) - 1;
+                    bal &= bal - 1;
+                    const uint32_t s0 = __shfl_sync(0xffffffffu, rs, j), s1 = __shfl_sync(0xffffffffu, re, j);
+                    uint32_t w = s0 + (uint32_t)lane;  // the lane's slot
+                    const float4* src = pts + w;
+                    uint32_t left = s1 - s0;
+                    for (; left >= 128u; left -= 128u, src += 128, w += 128u) {
+                        const float4 v0 = __ldg(src), v1 = __ldg(src + 32), v2 = __ldg(src + 64), v3 = __ldg(src + 96);
+                        uint32_t at[4][H];
+                        find(v0, at[0]);
+                        find(v1, at[1]);
+                        find(v2, at[2]);
+                        find(v3, at[3]);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) add(at[u]);
+                        if (__any_sync(0xffffffffu, z < q.zone)) {
+#pragma unroll 1
+                            for (uint32_t u = 0; u < 128u; u += 32u) zone_at(w + u);
+                            z = 0xffffffffu;
+                        }
+                    }
+                    if (left) {
+                        float4 v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            v[u].x = INFINITY;
+                            if ((uint32_t)lane + 32u * (uint32_t)u < left) v[u] = __ldg(src + 32 * u);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (32u * (uint32_t)u < left) {
+                                uint32_t at[H];
+                                find(v[u], at);
+                                add(at);
+                            }
+                        if (__any_sync(0xffffffffu, z < q.zone)) {
+#pragma unroll 1
+                            for (uint32_t u = 0; u < 128u; u += 32u) zone_at(w + u < s1 ? w + u : 0xffffffffu);
+                            z = 0xffffffffu;
+                        }
+                    }
+                }
+            } else {
+                // windows over the flattened sequence
+                const uint32_t off = a - excl;
+                for (uint32_t wb = t0; wb < t1; wb += 64) {
+                    const uint32_t u0 = wb + (uint32_t)lane, u1 = u0 + 32u;
+                    int r0 = 0, r1 = 0;
+#pragma unroll
+                    for (int k = 16; k >= 1; k >>= 1) {
+                        const uint32_t v0 = __shfl_sync(0xffffffffu, incl, r0 + k - 1);
+                        const uint32_t v1 = __shfl_sync(0xffffffffu, incl, r1 + k - 1);
+                        r0 += (v0 <= u0) ? k : 0;
+                        r1 += (v1 <= u1) ? k : 0;
+                    }
+                    const uint32_t o0 = __shfl_sync(0xffffffffu, off, r0);
+                    const uint32_t o1 = __shfl_sync(0xffffffffu, off, r1);
+                    float4 v0, v1;
+                    v0.x = v1.x = INFINITY;
+                    if (u0 < t1) v0 = __ldg(pts + (u0 + o0));
+                    if (u1 < t1) v1 = __ldg(pts + (u1 + o1));
+                    uint32_t at0[H], at1[H];
+                    find(v0, at0);
+                    find(v1, at1);
+                    add(at0);
+                    if (wb + 32u < t1) add(at1);
                     if (__any_sync(0xffffffffu, z < q.zone)) {
-                        zone_test(v0);
-                        zone_test(v1);
-                        zone_test(v2);
-                        zone_test(v3);
+                        zone_at(u0 < t1 ? u0 + o0 : 0xffffffffu);
+                        zone_at(u1 < t1 ? u1 + o1 : 0xffffffffu);
                         z = 0xffffffffu;
                     }
                 }
-                if (left) {
-                    float4 v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        v[u].x = INFINITY;
-                        if ((uint32_t)lane + 32u * (uint32_t)u < left) v[u] = __ldg(src + 32 * u);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (32u * (uint32_t)u < left) test(v[u]);
-                    if (__any_sync(0xffffffffu, z < q.zone)) {
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) zone_test(v[u]);
-                        z = 0xffffffffu;
-                    }
-                }
             }
-        } else {
-            // short rows: windows over the flattened sequence
-            const uint32_t off = a - excl;
-            for (uint32_t wb = tb; wb < te; wb += 64) {
-                const uint32_t t0 = wb + (uint32_t)lane, t1 = t0 + 32u;
-                int r0 = 0, r1 = 0;
+            held += ((t1 - t0) >> 5) + 64u;
+            if (held > 32000u) {
 #pragma unroll
-                for (int k = 16; k >= 1; k >>= 1) {
-                    const uint32_t v0 = __shfl_sync(0xffffffffu, incl, r0 + k - 1);
-                    const uint32_t v1 = __shfl_sync(0xffffffffu, incl, r1 + k - 1);
-                    r0 += (v0 <= t0) ? k : 0;
-                    r1 += (v1 <= t1) ? k : 0;
-                }
-                const uint32_t o0 = __shfl_sync(0xffffffffu, off, r0);
-                const uint32_t o1 = __shfl_sync(0xffffffffu, off, r1);
-                float4 v0, v1;
-                v0.x = v1.x = INFINITY;
-                if (t0 < te) v0 = __ldg(pf.pts + (t0 + o0));
-                if (t1 < te) v1 = __ldg(pf.pts + (t1 + o1));
-                test(v0);
-                if (wb + 32u < te) test(v1);
-                if (__any_sync(0xffffffffu, z < q.zone)) {
-                    zone_test(v0);
-                    zone_test(v1);
-                    z = 0xffffffffu;
-                }
+                for (int k = 0; k < H; ++k)
+                    flush_columns(cols + k * colwords, q.ncol,
+                                  p.counts + (uint64_t)__float_as_uint(c[k].w) * (uint64_t)p.nrads, lane);
+                held = 0;
             }
         }
     }
-    if (any) {
-        __syncwarp();
-        for (int s0 = 0; s0 < q.ncol; s0 += 32) {
-            const int s = s0 + lane;
-            if (s < q.ncol) {
-                uint32_t sum = 0;
-                const uint32_t* r = cols + s * 32;
-#pragma unroll 8
-                for (int k = 0; k < 32; ++k) sum += r[(k + lane) & 31];
-                if (sum) atomicAdd(row + s, sum);
-            }
-        }
-        __syncwarp();
-        for (int i = lane; i < q.ncol * 32; i += 32) cols[i] = 0u;
-        __syncwarp();
+    if (held) {
+#pragma unroll
+        for (int k = 0; k < H; ++k)
+            flush_columns(cols + k * colwords, q.ncol, p.counts + (uint64_t)__float_as_uint(c[k].w) * (uint64_t)p.nrads,
+                          lane);
     }
+}
+
+// Two neighbouring items of the list are counted together when they are two
+// centres of one index no further apart than a radius: most candidates then
+// serve both.
+__device__ __forceinline__ bool paired(const CountParams& p, const uint2* it, uint32_t n) {
+    constexpr uint32_t kAlone = kItemZone | kItemFar | kItemShort;
+    if (n < 2u || ((it[0].y | it[1].y) & kAlone) || (((it[0].y ^ it[1].y) >> 3) & 3u)) return false;
+    const float4 a = item_centre(p, it[0]), b = item_centre(p, it[1]);
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    return dx * dx + dy * dy + dz * dz <= p.r2max;
 }
 
 __global__ void __launch_bounds__(HV_THREADS, HV_BLOCKS)
@@ -536,25 +683,53 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
     const uint32_t nhuge = min(q.ctl[1], q.cap), nother = min(q.ctl[2], q.cap);
     if (nhuge + nother == 0u) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int colwords = (q.ncol + 1) * 32;
+    const int colwords = 2 * (q.ncol + 1) * 16;
     uint32_t* slots = smem + HV_WARPS * colwords;
     uint32_t* cols = smem + warp * colwords;
     for (int i = tid; i < q.nslots; i += HV_THREADS) slots[i] = q.slots[i];
     for (int i = lane; i < colwords; i += 32) cols[i] = 0u;
     __syncthreads();
-    // Warps claim (item, part) pairs.  Items of more than kHuge candidates
-    // are always split; all items are when there are too few of them.
+    // Warps claim (two items, part).  Items of more than kHuge candidates are
+    // always split; all items are when there are too few of them.
     const uint32_t warps = gridDim.x * HV_WARPS;
-    const uint32_t ph = nhuge >= (1u << 28) ? 1u : max(8u, min(64u, 4u * warps / max(nhuge, 1u)));
-    const uint32_t po = max(1u, min(32u, 4u * warps / max(nother, 1u)));
-    const uint32_t ch = nhuge * ph, co = nother * po;
-    for (;;) {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(q.ctl + 3, 1u);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= ch + co) break;
-        if (i < ch) count_item(p, q, q.list[i / ph], i % ph, ph, cols, slots, lane);
-        else count_item(p, q, q.list[q.cap - 1u - (i - ch) / po], (i - ch) % po, po, cols, slots, lane);
+    const uint32_t mh = (nhuge + 1u) / 2u, mo = (nother + 1u) / 2u;
+    const uint32_t ph = mh >= (1u << 28) ? 1u : max(8u, min(64u, 4u * warps / max(mh, 1u)));
+    const uint32_t po = max(1u, min(32u, 4u * warps / max(mo, 1u)));
+    const uint32_t ch = mh * ph, co = mo * po;
+    // Pairs first, then long rows alone, then the rest: warps of an SM run the
+    // same loop at a time (the three together exceed the instruction cache).
+#pragma unroll 1
+    for (int phase = 0; phase < 3; ++phase) {
+        for (;;) {
+            uint32_t i = 0;
+            if (lane == 0) i = atomicAdd(q.ctl + 3 + phase, 1u);
+            i = __shfl_sync(0xffffffffu, i, 0);
+            if (i >= ch + co) break;
+            const bool huge = i < ch;
+            const uint32_t k = huge ? i / ph : (i - ch) / po, part = huge ? i % ph : (i - ch) % po;
+            const uint32_t nparts = huge ? ph : po, n = min(2u, (huge ? nhuge : nother) - 2u * k);
+            uint2 it[2];
+#pragma unroll
+            for (uint32_t j = 0; j < 2u; ++j)
+                it[j] = j < n ? q.list[huge ? 2u * k + j : q.cap - 1u - (2u * k + j)] : make_uint2(0u, 0u);
+            if (paired(p, it, n)) {
+                if (phase == 0) count_items<2, false>(p, q, it, part, nparts, cols, slots, lane);
+            } else if (phase == 1) {
+#pragma unroll 1
+                for (uint32_t j = 0; j < n; ++j) {
+                    const uint2 one = j ? it[1] : it[0];
+                    if (!(one.y & (kItemZone | kItemFar | kItemShort)))
+                        count_items<1, false>(p, q, &one, part, nparts, cols, slots, lane);
+                }
+            } else if (phase == 2) {
+#pragma unroll 1
+                for (uint32_t j = 0; j < n; ++j) {
+                    const uint2 one = j ? it[1] : it[0];
+                    if (one.y & (kItemZone | kItemFar)) count_literal(p, q, one, part, nparts, lane);
+                    else if (one.y & kItemShort) count_items<1, true>(p, q, &one, part, nparts, cols, slots, lane);
+                }
+            }
+        }
     }
 }
 
@@ -578,7 +753,6 @@ int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p,
     q.kbase = L.kbase;
     q.shift = L.shift;
     q.khi = (L.nslots << L.shift) - 1;
-    q.mask = (1u << L.shift) - 1u;
     q.ncol = L.ncol;
     q.safe2 = L.safe2;
     uint32_t km;
@@ -607,7 +781,7 @@ int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p,
     const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxSmem - table) / warp_a);  // >= 15 for any table
     const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + (uint64_t)ctx->num_sms - 1) / (uint64_t)ctx->num_sms);
     const size_t smem_a = nw * warp_a + table;
-    const size_t smem_b = HV_WARPS * (size_t)(L.ncol + 1) * 128 + (size_t)L.nslots * 4;
+    const size_t smem_b = HV_WARPS * 2 * (size_t)(L.ncol + 1) * 64 + (size_t)L.nslots * 4;
     SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
     const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
     k_lane_count<<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);

@@ -207,8 +207,9 @@ void build_shell_lut(const float* r2, int nrads, std::vector<uint32_t>* lut, uin
 // here for |c| <= cmax.  Slot j covers the keys [kbase + (j << shift), ... +
 // (1 << shift)) and holds at most one of the thresholds (r2 below safe2, then
 // safe2); word j is (thresholds before the slot << shift) + (1 << shift) - low
-// bits of its threshold, so adding a key's low bits carries into the index
-// exactly when the key has reached the threshold.
+// bits of its threshold - (j << shift), so adding key - kbase leaves the slot's
+// index above the low bits, carried by one exactly when the key has reached
+// the threshold.
 void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32_t>* slots,
                       sjcs_query::LaneTable* t) {
     constexpr int kMaxSlots = 2048, kMaxCols = 128;
@@ -244,7 +245,7 @@ void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32
         while (before < th.size() && th[before] < k) ++before;
         uint32_t low = 1u << shift;  // no threshold in this slot
         if (before < th.size() && th[before] - k < (1 << shift)) low = (uint32_t)(th[before] - k);
-        (*slots)[j] = ((uint32_t)before << shift) + (1u << shift) - low;
+        (*slots)[j] = ((uint32_t)before << shift) + (1u << shift) - low - ((uint32_t)j << shift);
     }
     t->nslots = n;
     t->kbase = kbase;
