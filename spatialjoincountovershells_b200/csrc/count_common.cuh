@@ -4,6 +4,8 @@
 // The arithmetic contract is documented in shell_count.cu.
 #pragma once
 
+#include <cmath>
+
 #include "sjcs_internal.cuh"
 
 namespace sjcs {
@@ -27,6 +29,7 @@ struct CountParams {
     uint32_t lut_k0;                 // bit pattern of r2[0]
     int lut_shift;
     float half;
+    float reach;                     // a counted particle lies within this of the centre on each axis (see make_image)
     float r2max;
     float r2p;                       // r2max * (1 + 1e-5)
     float r2slack;                   // r2max * 1e-5
@@ -39,6 +42,12 @@ struct CountParams {
     const uint32_t* mcs[kMaxFused];
     uint32_t mn[kMaxFused];  // particles of each index
 };
+
+// CountParams::reach: with pruning, a bound above the square root of r2p plus
+// the rounding of the differences; else no bound.
+inline float reach_of(float r2max, bool prune) {
+    return prune ? (float)(std::sqrt((double)r2max * (1.0 + 1e-5)) * (1.0 + 1e-6) + 4e-3) : INFINITY;
+}
 
 __device__ __forceinline__ float edge_margin(float v) { return 1e-3f + 2e-6f * fabsf(v); }
 
@@ -85,15 +94,19 @@ __device__ __forceinline__ Image make_image(const CountParams& p, float cx, floa
     im.hiy = __fadd_rn(cy, p.half);
     im.loz = __fsub_rn(cz, p.half);
     im.hiz = __fadd_rn(cz, p.half);
-    // A NaN bound passes every particle on that side of the box test, so it
-    // must open the cell range to the grid edge (cell_of maps NaN to cell 0,
-    // which is right for a lower bound only).
-    im.x0 = cell_of(im.lox, p.g.inv_h[0], p.g.G[0]);
-    im.x1 = (im.hix != im.hix) ? p.g.G[0] - 1 : cell_of(im.hix, p.g.inv_h[0], p.g.G[0]);
-    im.y0 = cell_of(im.loy, p.g.inv_h[1], p.g.G[1]);
-    im.y1 = (im.hiy != im.hiy) ? p.g.G[1] - 1 : cell_of(im.hiy, p.g.inv_h[1], p.g.G[1]);
-    im.z0 = cell_of(im.loz, p.g.inv_h[2], p.g.G[2]);
-    im.z1 = (im.hiz != im.hiz) ? p.g.G[2] - 1 : cell_of(im.hiz, p.g.inv_h[2], p.g.G[2]);
+    // Cells: those of the box, but no further from the centre than a counted
+    // particle can be (non-periodic boxes are r2max wide, far wider than the
+    // sphere when R > 1).  A NaN bound passes every particle on that side of
+    // the box test, so it must open the cell range to the grid edge (cell_of
+    // maps NaN to cell 0, which is right for a lower bound only).
+    const float rx = p.reach + 1e-6f * fabsf(cx), ry = p.reach + 1e-6f * fabsf(cy), rz = p.reach + 1e-6f * fabsf(cz);
+    const float hx = fminf(im.hix, cx + rx), hy = fminf(im.hiy, cy + ry), hz = fminf(im.hiz, cz + rz);
+    im.x0 = cell_of(fmaxf(im.lox, cx - rx), p.g.inv_h[0], p.g.G[0]);
+    im.x1 = (hx != hx) ? p.g.G[0] - 1 : cell_of(hx, p.g.inv_h[0], p.g.G[0]);
+    im.y0 = cell_of(fmaxf(im.loy, cy - ry), p.g.inv_h[1], p.g.G[1]);
+    im.y1 = (hy != hy) ? p.g.G[1] - 1 : cell_of(hy, p.g.inv_h[1], p.g.G[1]);
+    im.z0 = cell_of(fmaxf(im.loz, cz - rz), p.g.inv_h[2], p.g.G[2]);
+    im.z1 = (hz != hz) ? p.g.G[2] - 1 : cell_of(hz, p.g.inv_h[2], p.g.G[2]);
     im.ny = im.y1 - im.y0 + 1;
     im.nz = im.z1 - im.z0 + 1;
     const uint64_t nr = (uint64_t)im.ny * (uint64_t)im.nz;

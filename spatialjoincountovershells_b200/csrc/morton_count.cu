@@ -84,9 +84,10 @@ __device__ __forceinline__ void count_image_m(const CountParams& p, const Morton
     im.hiy = __fadd_rn(cy, p.half);
     im.loz = __fsub_rn(cz, p.half);
     im.hiz = __fadd_rn(cz, p.half);
-    const int x0 = mcell_lo(m, im.lox), x1 = mcell_hi(m, im.hix);
-    const int y0 = mcell_lo(m, im.loy), y1 = mcell_hi(m, im.hiy);
-    const int z0 = mcell_lo(m, im.loz), z1 = mcell_hi(m, im.hiz);
+    const float rx = p.reach + 1e-6f * fabsf(cx), ry = p.reach + 1e-6f * fabsf(cy), rz = p.reach + 1e-6f * fabsf(cz);
+    const int x0 = mcell_lo(m, fmaxf(im.lox, cx - rx)), x1 = mcell_hi(m, fminf(im.hix, cx + rx));
+    const int y0 = mcell_lo(m, fmaxf(im.loy, cy - ry)), y1 = mcell_hi(m, fminf(im.hiy, cy + ry));
+    const int z0 = mcell_lo(m, fmaxf(im.loz, cz - rz)), z1 = mcell_hi(m, fminf(im.hiz, cz + rz));
     const uint32_t nx = (uint32_t)(x1 - x0 + 1), ny = (uint32_t)(y1 - y0 + 1), nz = (uint32_t)(z1 - z0 + 1);
     const uint32_t total = nx * ny * nz;  // <= 2^30 (L <= 10)
     const uint32_t lt = (1u << lane) - 1u;
@@ -277,11 +278,13 @@ __global__ void k_estimate_m(CountParams p, MortonParams m, uint32_t* __restrict
         const int sh2 = m.sh + up, G2 = m.G >> up;
         const float lo[3] = {__fsub_rn(c.x, p.half), __fsub_rn(c.y, p.half), __fsub_rn(c.z, p.half)};
         const float hi[3] = {__fadd_rn(c.x, p.half), __fadd_rn(c.y, p.half), __fadd_rn(c.z, p.half)};
+        const float cc[3] = {c.x, c.y, c.z};
         int a0[3], a1[3];
         uint64_t ncell = 1;
         for (int a = 0; a < 3; ++a) {
-            a0[a] = (int)(morton_q(lo[a]) >> sh2);
-            a1[a] = (hi[a] != hi[a]) ? G2 - 1 : (int)(morton_q(hi[a]) >> sh2);
+            const float rr = p.reach + 1e-6f * fabsf(cc[a]), l = fmaxf(lo[a], cc[a] - rr), u = fminf(hi[a], cc[a] + rr);
+            a0[a] = (int)(morton_q(l) >> sh2);
+            a1[a] = (u != u) ? G2 - 1 : (int)(morton_q(u) >> sh2);
             ncell *= (uint64_t)(a1[a] - a0[a] + 1);
         }
         uint64_t e = 0;
@@ -430,6 +433,7 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
     p.r2slack = q->r2max * 1e-5f;
     p.periodic = (q->flags & SJCS_QUERY_PERIODIC) ? 1 : 0;
     p.prune = q->monotone && std::isfinite(q->r2max) ? 1 : 0;
+    p.reach = reach_of(q->r2max, p.prune);
     p.counts = q->counts;
     MortonParams m{};
     m.table = idx->cell_start;

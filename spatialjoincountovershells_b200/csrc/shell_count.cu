@@ -557,6 +557,7 @@ CountParams count_params(const sjcs_query* q, const sjcs_index* idx) {
     p.r2slack = q->r2max * 1e-5f;
     p.periodic = (q->flags & SJCS_QUERY_PERIODIC) ? 1 : 0;
     p.prune = q->monotone && std::isfinite(q->r2max) ? 1 : 0;
+    p.reach = reach_of(q->r2max, p.prune);
     p.counts = q->counts;
     p.nidx = 1;
     p.mpts[0] = idx->pts;
