@@ -1,4 +1,6 @@
-// Periodic multi-shell count of grid indexes with one lane per halo.
+// Periodic multi-shell count with one lane per halo, over grid indexes (whose
+// candidate ranges are rows of cells) and Morton indexes (single cells, their
+// ranks from the offset table or the learned model).
 //
 // k_lane_count   32 halos of the Morton order per warp, one per lane.  A lane
 //                plans its box's rows of cells (at most 5 x 5), clips each in x
@@ -40,17 +42,19 @@
 // k_listed_count runs at 68 % of both the data pipe and issue.
 //
 // Measured (B200, count kernels of one call, warp-per-halo kernel -> this one):
-// 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.31 ms; 1e6 on
-// 1e7 0.42 -> 0.22; 1e6 clustered halos on 3e7 clustered particles 9.2 (static
-// schedule) and 7.1 (queue) -> 3.68, one item at a time 4.28; 1e6 on 5e7, R =
-// 20, 64 shells 55 and 40.8 -> 17.9, one item at a time 24.3; 1e5 on 2e7, R =
-// 10 2.14 and 1.45 -> 0.78, one at a time 0.90.
+// 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.27 ms; 1e6 on
+// 1e7 0.42 -> 0.20; 1e6 clustered halos on 3e7 clustered particles 9.2 (static
+// schedule) and 7.1 (queue) -> 3.43, one item at a time 4.28; 1e6 on 5e7, R =
+// 20, 64 shells 55 and 40.8 -> 18.5, one item at a time 24.3; 1e5 on 2e7, R =
+// 10 2.14 and 1.45 -> 0.75, one at a time 0.90.  Morton forms, 5e5 clustered
+// halos on 2e7 particles: offset table 4.87 -> 2.19, learned 4.65 (queue) -> 2.86.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 
 #include "grid_rows.cuh"
 #include "lane_count.cuh"
+#include "morton.cuh"
 
 namespace sjcs {
 namespace {
@@ -64,9 +68,12 @@ constexpr int LN_WARPS = 16;
 constexpr int LN_ROWS = 25;       // rows of cells a lane walks
 constexpr uint32_t LN_PEND = 96;  // shifted images waiting per warp
 constexpr int LN_DEPTH = 4;       // candidates in flight per lane (2: 4.42 ms, 3: 4.35, 6: 4.34)
-// Listed items: five blocks of four warps per SM (96 registers; six with 80
-// spill and take 7 % longer, four 10 %).
-constexpr int HV_WARPS = 4, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 5;
+// Listed items: 20 blocks of one warp per SM (96 registers; five blocks of four
+// warps take 2 % longer, 16 warps without spills 11 %).
+constexpr int HV_WARPS = 1, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 20;
+// The allocation-free count takes 16: no local memory, which the driver may
+// have to set aside at a launch.
+constexpr int HV_BLOCKS_NOALLOC = 16;
 constexpr uint32_t kSpan = 1u << 20;  // candidates between two looks at what the 16-bit counters hold
 // Items above this many candidates (in the box's rows) are split into 8 to 64
 // parts: one warp would need longer than the rest of the pass (16384 and 32768
@@ -96,7 +103,52 @@ struct LaneParams {
     uint2* __restrict__ list;  // (halo, flags)
     uint32_t cap;
     uint32_t* __restrict__ ctl;  // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase
+    // learned index: its model (leaves null: the other kinds)
+    const LearnedLeaf* __restrict__ leaves;
+    const LearnedRoot* __restrict__ root;
+    const uint32_t* __restrict__ wpref;  // &pts[0].w (stride 4 words)
+    int key_shift;                       // cell code -> first key of the cell
 };
+
+// What a candidate range is: a row of grid cells clipped in x, or one Morton
+// cell, its ranks from the offset table or from the learned model.
+enum Ranges { RANGE_ROWS = 0, RANGE_CELLS = 1, RANGE_MODEL = 2 };
+
+// Ranges of an image's box (2^31 when there are more).
+template <int R>
+__device__ __forceinline__ uint32_t box_ranges(const Image& im) {
+    if (R == RANGE_ROWS) return im.nrows;
+    const uint64_t n = (uint64_t)im.nrows * (uint64_t)(im.x1 - im.x0 + 1);
+    return n > 0x80000000ull ? 0x80000000u : (uint32_t)n;
+}
+
+__device__ __forceinline__ uint2 table_range(const uint32_t* __restrict__ cs, uint32_t code) {
+    return make_uint2(__ldg(cs + code), __ldg(cs + code + 1u));
+}
+
+// Ranks of both ends of two cells from the model (the table if the judge found
+// it wrong), the four searches advanced together.  Out of line: see below.
+__device__ __noinline__ uint4 model_ranges(const LaneParams& q, const uint32_t* __restrict__ cs, uint32_t c0, bool k0,
+                                           uint32_t c1, bool k1) {
+    const LearnedRoot rt = *q.root;
+    uint32_t s[4] = {0u, 0u, 0u, 0u};
+    if (rt.mismatches != 0ull) {
+        if (k0) {
+            s[0] = __ldg(cs + c0);
+            s[1] = __ldg(cs + c0 + 1u);
+        }
+        if (k1) {
+            s[2] = __ldg(cs + c1);
+            s[3] = __ldg(cs + c1 + 1u);
+        }
+    } else {
+        const uint64_t key[4] = {(uint64_t)c0 << q.key_shift, (uint64_t)(c0 + 1u) << q.key_shift,
+                                 (uint64_t)c1 << q.key_shift, (uint64_t)(c1 + 1u) << q.key_shift};
+        const bool act[4] = {k0, k0, k1, k1};
+        learned_rank_n<4>(rt, q.leaves, q.wpref, key, act, s);
+    }
+    return make_uint4(s[0], s[1], s[2], s[3]);
+}
 
 // An item's flags: bits 0-2 the shifted axes, bits 3-4 the index to count.
 constexpr uint32_t kItemZone = 1u << 7;  // only distances from safe2 on
@@ -131,25 +183,36 @@ __device__ __forceinline__ uint32_t oob_flags(const CountParams& p, const float4
 
 // One lane counts one image by itself, straight into the count row: the way
 // out when the item list is full.
+template <int R>
 __device__ __noinline__ void serial_count(const CountParams& p, float4 c, uint32_t flags, float safe2) {
     const Image im = make_image(p, c.x, c.y, c.z);
     uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
     const uint32_t f = (flags >> 3) & 3u;
+    auto test = [&](uint32_t j0, uint32_t e) {
+        for (uint32_t j = j0; j < e; ++j) {
+            const float4 v = p.mpts[f][j];
+            if (flags & kItemZone)
+                test_candidate<BIN_BSEARCH, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
+            else
+                test_candidate<BIN_BSEARCH, true>(p, im, v, true, row, p.r2, p.lut);
+        }
+    };
     for (int zz = im.z0; zz <= im.z1; ++zz)
         for (int yy = im.y0; yy <= im.y1; ++yy) {
-            const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
-            const uint32_t e = p.mcs[f][rc + im.x1 + 1];
-            for (uint32_t j = p.mcs[f][rc + im.x0]; j < e; ++j) {
-                const float4 v = p.mpts[f][j];
-                if (flags & kItemZone)
-                    test_candidate<BIN_BSEARCH, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
-                else
-                    test_candidate<BIN_BSEARCH, true>(p, im, v, true, row, p.r2, p.lut);
+            if (R == RANGE_ROWS) {
+                const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
+                test(p.mcs[f][rc + im.x0], p.mcs[f][rc + im.x1 + 1]);
+            } else {
+                for (int xx = im.x0; xx <= im.x1; ++xx) {
+                    const uint32_t code = morton_cell((uint32_t)xx, (uint32_t)yy, (uint32_t)zz);
+                    test(p.mcs[f][code], p.mcs[f][code + 1u]);
+                }
             }
         }
 }
 
 // Lanes with `push` add an item (h, flags) to the list; c is its centre.
+template <int R>
 __device__ __forceinline__ void push_items(const CountParams& p, const LaneParams& q, bool push, bool huge, uint32_t h,
                                            uint32_t flags, float4 c, int lane) {
     const uint32_t all = __ballot_sync(0xffffffffu, push);
@@ -170,9 +233,10 @@ __device__ __forceinline__ void push_items(const CountParams& p, const LaneParam
         const uint32_t i = huge ? ah + (uint32_t)__popc(hb & lt) : q.cap - 1u - (ao + (uint32_t)__popc(ob & lt));
         q.list[i] = make_uint2(h, flags);
     }
-    if (push && !fits) serial_count(p, c, flags, q.safe2);
+    if (push && !fits) serial_count<R>(p, c, flags, q.safe2);
 }
 
+template <int R>
 __global__ void __launch_bounds__(LN_WARPS * 32, 1)
 k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
@@ -190,6 +254,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t nbatch = (uint32_t)((p.nhalos + 31) / 32);
     const uint32_t W = gridDim.x * (uint32_t)nwarps;
+    [[maybe_unused]] const float hmx = 0.5f * p.h[0] + 3e-3f;
     const float hmy = 0.5f * p.h[1] + 3e-3f, hmz = 0.5f * p.h[2] + 3e-3f;
     const uint32_t plane_cells = (uint32_t)p.g.G[1] * (uint32_t)p.g.G[0];
     // One index after the other: a batch counted on all of them at once held
@@ -238,7 +303,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                             if (T & 1u) ci.x = shifted(c.x, p.half);
                             if (T & 2u) ci.y = shifted(c.y, p.half);
                             if (T & 4u) ci.z = shifted(c.z, p.half);
-                            push_items(p, q, T != 0u, false, h, T | file, ci, lane);
+                            push_items<R>(p, q, T != 0u, false, h, T | file, ci, lane);
                         }
                         T = T ? (T - 1u) & F : 0u;
                     }
@@ -251,16 +316,19 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
             const bool fin = (c.x - c.x == 0.0f) & (c.y - c.y == 0.0f) & (c.z - c.z == 0.0f);
             const bool far = !(fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)) <= q.cmax);
             const Image im = make_image(p, c.x, c.y, c.z);
-            const bool cand = valid & fin & !far & (im.ny <= LN_ROWS) & (im.nrows <= kMaxWalkRows);
+            const uint32_t nranges = box_ranges<R>(im);
+            const bool cand = valid & fin & !far & (R != RANGE_ROWS || im.ny <= LN_ROWS) & (nranges <= kMaxWalkRows);
             bool mine = cand;
-            const bool chunked = __any_sync(0xffffffffu, cand && (im.ny > 5 || im.nz > 5));
+            const bool chunked = __any_sync(
+                0xffffffffu, cand && (R == RANGE_ROWS ? im.ny > 5 || im.nz > 5 : nranges > (uint32_t)LN_ROWS));
             if (chunked || __any_sync(0xffffffffu, valid & fin & !cand)) {
-                // Boxes of more than 25 rows are walked a few planes at a time.
+                // Boxes of more than 25 ranges are walked a few planes (of Morton
+                // cells: 25) at a time.
                 // What is listed instead is decided on the candidates of the
                 // whole box: long rows, more than the 16-bit counters hold, and
                 // lanes that would keep the others waiting.
                 uint32_t box = 0;
-                if (cand) {
+                if (R == RANGE_ROWS && cand) {
                     // eight rows' loads in flight at a time
                     const uint32_t gx = (uint32_t)p.g.G[0], xl = (uint32_t)im.x0, xh = (uint32_t)im.x1 + 1u;
                     uint32_t rc = ((uint32_t)im.z0 * (uint32_t)p.g.G[1] + (uint32_t)im.y0) * gx;
@@ -283,16 +351,31 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
 #pragma unroll
                         for (int u = 0; u < 8; ++u) box += hi[u] - lo[u];
                     }
+                } else if (cand) {
+                    // from the table; the model would answer the same
+                    for (int zz = im.z0; zz <= im.z1; ++zz)
+                        for (int yy = im.y0; yy <= im.y1; ++yy) {
+                            const uint32_t zy = (spread3_10((uint32_t)yy) << 1) | (spread3_10((uint32_t)zz) << 2);
+                            for (int xx = im.x0; xx <= im.x1; xx += 4) {
+                                uint2 r4[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u)
+                                    r4[u] = xx + u <= im.x1 ? table_range(cs, zy | spread3_10((uint32_t)(xx + u)))
+                                                            : make_uint2(0u, 0u);
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) box += r4[u].y - r4[u].x;
+                            }
+                        }
                 } else if (valid & fin) {
                     box = q.huge + 1u;
                 }
                 __syncwarp();
                 // about what the sphere leaves of the box
-                const uint32_t est = box - (box >> 2) - (box >> 3), rows_est = im.nrows - (im.nrows >> 2);
+                const uint32_t est = box - (box >> 2) - (box >> 3), rows_est = nranges - (nranges >> 2);
                 if (chunked) {
                     mine = cand && est <= q.walk_max;
                     const uint32_t mxT = __reduce_max_sync(0xffffffffu, mine ? est : 0u);
-                    const uint32_t hc = listed_cost(est, rows_est, im.nrows);
+                    const uint32_t hc = listed_cost(est, rows_est, nranges);
                     uint32_t best = kStepCost * mxT, tau = mxT;
 #pragma unroll
                     for (int k = 1; k < 5; ++k) {
@@ -307,15 +390,21 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     }
                     mine &= est <= tau;
                 }
-                push_items(p, q, valid & fin & !mine, box > q.huge, h,
+                push_items<R>(p, q, valid & fin & !mine, box > q.huge, h,
                            file | S | (far ? kItemFar : 0u) | (short_rows(est, rows_est) ? kItemShort : 0u), c, lane);
             }
             const int ny = mine ? im.ny : 0, nz = mine ? im.nz : 0;
             const int nymax = __reduce_max_sync(0xffffffffu, ny), nzmax = __reduce_max_sync(0xffffffffu, nz);
-            const int planes = chunked ? LN_ROWS / max(nymax, 1) : 5;  // per walk
+            // steps over the box: planes of rows, or runs of cells
+            const int planes = R != RANGE_ROWS ? LN_ROWS : chunked ? LN_ROWS / max(nymax, 1) : 5;  // per walk
+            const int ncell = R != RANGE_ROWS && mine ? (int)nranges : 0;
+            const int zend = R != RANGE_ROWS ? __reduce_max_sync(0xffffffffu, ncell) : nzmax;
+            [[maybe_unused]] int cxi = 0, cyi = 0, czi = 0;  // the next cell
             // Row gaps as max(0, |cell middle - centre| - half a cell - margin), the
             // centre clamped into the box (edge cells also hold what lies outside
             // it).  The margin of 3e-3 is that of cell_gap at the far face.
+            [[maybe_unused]] const float xbase =
+                ((float)im.x0 + 0.5f) * p.h[0] - fminf(fmaxf(c.x, 0.0f), kBoxUpp);
             const float ccy = fminf(fmaxf(c.y, 0.0f), kBoxUpp), ccz = fminf(fmaxf(c.z, 0.0f), kBoxUpp);
             const float ybase = ((float)im.y0 + 0.5f) * p.h[1] - ccy, zbase = ((float)im.z0 + 0.5f) * p.h[2] - ccz;
             constexpr int kMagicI = 0x4b400000;  // bits of 1.5 * 2^23: adding it rounds to an integer in the low bits
@@ -327,38 +416,83 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
             const uint32_t rowc0 = ((uint32_t)im.z0 * (uint32_t)p.g.G[1] + (uint32_t)im.y0) * (uint32_t)p.g.G[0] - (uint32_t)kMagicI;
             uint32_t z = 0xffffffffu;  // least key - zone0 met
             bool walked = false;
-            for (int zb = 0; zb < nzmax; zb += planes) {
+            for (int zb = 0; zb < zend; zb += planes) {
                 uint32_t m = 0, T = 0;
-                for (int zi = zb; zi < min(zb + planes, nzmax); ++zi) {
-                    const float gz = fmaxf(fabsf(__fmaf_rn((float)zi, p.h[2], zbase)) - hmz, 0.0f);
-                    const float rz2 = r2q - gz * gz;
-                    const uint32_t rowz = rowc0 + (uint32_t)zi * plane_cells;
-                    for (int y5 = 0; y5 < nymax; y5 += 5) {
-                        uint32_t a[5], e[5];
+                auto keep = [&](uint32_t a, uint32_t e) {
+                    const uint32_t l = e - a;
+                    if (l) {
+                        rows->s0[m][lane] = a;
+                        rows->len[m][lane] = (uint16_t)l;
+                        ++m;
+                        T += l;
+                    }
+                };
+                if constexpr (R == RANGE_ROWS) {
+                    for (int zi = zb; zi < min(zb + planes, nzmax); ++zi) {
+                        const float gz = fmaxf(fabsf(__fmaf_rn((float)zi, p.h[2], zbase)) - hmz, 0.0f);
+                        const float rz2 = r2q - gz * gz;
+                        const uint32_t rowz = rowc0 + (uint32_t)zi * plane_cells;
+                        for (int y5 = 0; y5 < nymax; y5 += 5) {
+                            uint32_t a[5], e[5];
 #pragma unroll
-                        for (int u = 0; u < 5; ++u) {
-                            const float gy = fmaxf(fabsf(__fmaf_rn((float)(y5 + u), p.h[1], ybase)) - hmy, 0.0f);
-                            const float rem = rz2 - gy * gy;
-                            a[u] = e[u] = 0u;
-                            if (rem >= 0.0f && y5 + u < ny && zi < nz) {
-                                // approximate square root: its error (< 1e-6 relative) is far inside the margin
-                                const float sq = rem * rsqrtf(fmaxf(rem, 1e-35f));
-                                const float xr = __fmaf_rn(sq, 1.0f + 2e-6f, xpad);
-                                const int xa = min(max(__float_as_int(__fmaf_rn(cxh - xr, p.g.inv_h[0], kMagic)), ra), rz);
-                                const int xb = min(max(__float_as_int(__fmaf_rn(cxh + xr, p.g.inv_h[0], kMagic)), ra), rz);
-                                const uint32_t row = rowz + (uint32_t)(y5 + u) * (uint32_t)p.g.G[0];
-                                a[u] = __ldg(cs + (row + (uint32_t)xa));
-                                e[u] = __ldg(cs + (row + (uint32_t)xb + 1u));
+                            for (int u = 0; u < 5; ++u) {
+                                const float gy = fmaxf(fabsf(__fmaf_rn((float)(y5 + u), p.h[1], ybase)) - hmy, 0.0f);
+                                const float rem = rz2 - gy * gy;
+                                a[u] = e[u] = 0u;
+                                if (rem >= 0.0f && y5 + u < ny && zi < nz) {
+                                    // approximate square root: its error (< 1e-6 relative) is far inside the margin
+                                    const float sq = rem * rsqrtf(fmaxf(rem, 1e-35f));
+                                    const float xr = __fmaf_rn(sq, 1.0f + 2e-6f, xpad);
+                                    const int xa = min(max(__float_as_int(__fmaf_rn(cxh - xr, p.g.inv_h[0], kMagic)), ra), rz);
+                                    const int xb = min(max(__float_as_int(__fmaf_rn(cxh + xr, p.g.inv_h[0], kMagic)), ra), rz);
+                                    const uint32_t row = rowz + (uint32_t)(y5 + u) * (uint32_t)p.g.G[0];
+                                    a[u] = __ldg(cs + (row + (uint32_t)xa));
+                                    e[u] = __ldg(cs + (row + (uint32_t)xb + 1u));
+                                }
+                            }
+#pragma unroll
+                            for (int u = 0; u < 5; ++u) keep(a[u], e[u]);
+                        }
+                    }
+                } else {
+                    const int left = min(zend - zb, planes);
+                    for (int k4 = 0; k4 < left; k4 += 4) {
+                        uint32_t code[4];
+                        bool in[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            in[u] = k4 + u < left && zb + k4 + u < ncell;
+                            code[u] = 0u;
+                            if (in[u]) {
+                                const float gx = fmaxf(fabsf(__fmaf_rn((float)cxi, p.h[0], xbase)) - hmx, 0.0f);
+                                const float gy = fmaxf(fabsf(__fmaf_rn((float)cyi, p.h[1], ybase)) - hmy, 0.0f);
+                                const float gz = fmaxf(fabsf(__fmaf_rn((float)czi, p.h[2], zbase)) - hmz, 0.0f);
+                                // no particle of this cell can be within R otherwise
+                                in[u] = r2q - gz * gz - gy * gy - gx * gx >= 0.0f;
+                                code[u] = morton_cell((uint32_t)(im.x0 + cxi), (uint32_t)(im.y0 + cyi),
+                                                      (uint32_t)(im.z0 + czi));
+                                if (++cxi > im.x1 - im.x0) {
+                                    cxi = 0;
+                                    if (++cyi == im.ny) {
+                                        cyi = 0;
+                                        ++czi;
+                                    }
+                                }
                             }
                         }
+                        if constexpr (R == RANGE_CELLS) {
+                            uint2 r4[4];
 #pragma unroll
-                        for (int u = 0; u < 5; ++u) {
-                            const uint32_t l = e[u] - a[u];
-                            if (l) {
-                                rows->s0[m][lane] = a[u];
-                                rows->len[m][lane] = (uint16_t)l;
-                                ++m;
-                                T += l;
+                            for (int u = 0; u < 4; ++u)
+                                r4[u] = in[u] ? table_range(cs, code[u]) : make_uint2(0u, 0u);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) keep(r4[u].x, r4[u].y);
+                        } else {
+#pragma unroll
+                            for (int u = 0; u < 4; u += 2) {
+                                const uint4 r = model_ranges(q, cs, code[u], in[u], code[u + 1], in[u + 1]);
+                                keep(r.x, r.y);
+                                keep(r.z, r.w);
                             }
                         }
                     }
@@ -384,7 +518,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     }
                     coop |= T > tau;
                 }
-                if (__any_sync(0xffffffffu, coop)) push_items(p, q, coop, T > q.huge, h, file | S | (short_rows(T, m) ? kItemShort : 0u), c, lane);
+                if (__any_sync(0xffffffffu, coop)) push_items<R>(p, q, coop, T > q.huge, h, file | S | (short_rows(T, m) ? kItemShort : 0u), c, lane);
                 if (steps) {
                     // the list ends in a row of slots past the particles, which load nothing
                     const uint32_t mm = coop ? 0u : m;
@@ -433,7 +567,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     walked = true;
                 }
             }
-            if (__any_sync(0xffffffffu, z < q.zone)) push_items(p, q, z < q.zone, false, h, file | S | kItemZone, c, lane);
+            if (__any_sync(0xffffffffu, z < q.zone)) push_items<R>(p, q, z < q.zone, false, h, file | S | kItemZone, c, lane);
             // the lanes' counters to their halos' rows
             if (walked) {
                 uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
@@ -501,31 +635,93 @@ __device__ __noinline__ void flush_columns(uint32_t* __restrict__ cols, int ncol
     __syncwarp();
 }
 
+// Cell r of an image's box of Morton cells, x fastest.
+__device__ __forceinline__ void cell_xyz(const Image& im, uint32_t r, int* x, int* y, int* z) {
+    const uint32_t nx = (uint32_t)(im.x1 - im.x0 + 1), t = r / nx;
+    *x = im.x0 + (int)(r - t * nx);
+    *z = im.z0 + (int)(t / (uint32_t)im.ny);
+    *y = im.y0 + (int)(t % (uint32_t)im.ny);
+}
+
+// Lane r's range: row or cell rb + r of the box, if it can reach any of the H
+// spheres (a row clipped in x to them); empty otherwise.
+template <int R, int H>
+__device__ __forceinline__ uint2 lane_range(const CountParams& p, const LaneParams& q, const uint32_t* __restrict__ cs,
+                                            const Image& im, const float4 (&c)[H], uint32_t r, uint32_t n) {
+    uint2 s = make_uint2(0u, 0u);
+    if constexpr (R == RANGE_ROWS) {
+        if (r >= n) return s;
+        int yy, zz, xa = im.x1 + 1, xb = im.x0 - 1;
+        row_yz(im, r, &yy, &zz);
+#pragma unroll
+        for (int k = 0; k < H; ++k) {
+            const float gy = cell_gap(c[k].y, yy, p.h[1], p.g.G[1]), gz = cell_gap(c[k].z, zz, p.h[2], p.g.G[2]);
+            const float rem = __fadd_rn(__fsub_rn(__fsub_rn(p.r2p, __fmul_rn(gy, gy)), __fmul_rn(gz, gz)), p.r2slack);
+            if (rem >= 0.0f) {
+                // approximate square root: its error (< 1e-6 relative) is far inside the margin
+                float xr = rem > 0.0f ? __fmul_rn(rem, rsqrtf(rem)) : 0.0f;
+                xr = __fadd_rn(xr, 1e-3f + 1e-6f * (fabsf(c[k].x) + xr));
+                xa = min(xa, cell_of(__fsub_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
+                xb = max(xb, cell_of(__fadd_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
+            }
+        }
+        xa = max(xa, im.x0);
+        xb = min(xb, im.x1);
+        if (xa <= xb) {
+            const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
+            s = make_uint2(__ldg(cs + rc + xa), __ldg(cs + rc + xb + 1));
+        }
+    } else {
+        int xx = 0, yy = 0, zz = 0;
+        bool reach = false;
+        if (r < n) {
+            cell_xyz(im, r, &xx, &yy, &zz);
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                const float gx = cell_gap(c[k].x, xx, p.h[0], p.g.G[0]), gy = cell_gap(c[k].y, yy, p.h[1], p.g.G[1]),
+                            gz = cell_gap(c[k].z, zz, p.h[2], p.g.G[2]);
+                const float rem =
+                    __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(p.r2p, __fmul_rn(gx, gx)), __fmul_rn(gy, gy)),
+                                        __fmul_rn(gz, gz)),
+                              p.r2slack);
+                reach |= rem >= 0.0f;
+            }
+        }
+        const uint32_t code = morton_cell((uint32_t)xx, (uint32_t)yy, (uint32_t)zz);
+        if constexpr (R == RANGE_CELLS) {
+            if (reach) s = table_range(cs, code);
+        } else {
+            const uint4 m = model_ranges(q, cs, code, reach, 0u, false);
+            s = make_uint2(m.x, m.y);
+        }
+    }
+    return s;
+}
+
 // Zone and far items: the literal test, straight into the count row.
+template <int R>
 __device__ __noinline__ void count_literal(const CountParams& p, const LaneParams& q, const uint2 it, uint32_t part,
-                                              uint32_t nparts, int lane) {
-    const float4 c = item_centre(p, it);
-    uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
-    const Image im = make_image(p, c.x, c.y, c.z);
-    float gy, gz;
-    gap_tables(p, im, lane, &gy, &gz);
+                                           uint32_t nparts, int lane) {
+    const float4 c[1] = {item_centre(p, it)};
+    uint32_t* row = p.counts + (uint64_t)__float_as_uint(c[0].w) * (uint64_t)p.nrads;
+    const Image im = make_image(p, c[0].x, c[0].y, c[0].z);
+    const uint32_t n = box_ranges<R>(im);
     CountParams pf = p;
     pf.pts = p.mpts[(it.y >> 3) & 3u];
-    pf.cs = p.mcs[(it.y >> 3) & 3u];
-    for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
-        uint32_t a, e;
-        row_issue(pf, im, rb, lane, gy, gz, &a, &e);
+    const uint32_t* __restrict__ cs = p.mcs[(it.y >> 3) & 3u];
+    for (uint32_t rb = 0; rb < n; rb += 32u) {
+        const uint2 s = lane_range<R, 1>(p, q, cs, im, c, rb + (uint32_t)lane, n);
         if (it.y & kItemZone)
-            run_rows_part<BIN_BSEARCH, true, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts, q.safe2);
+            run_rows_part<BIN_BSEARCH, true, true>(pf, im, s.x, s.y, row, p.r2, p.lut, lane, part, nparts, q.safe2);
         else
-            run_rows_part<BIN_BSEARCH, true>(pf, im, a, e, row, p.r2, p.lut, lane, part, nparts);
+            run_rows_part<BIN_BSEARCH, true>(pf, im, s.x, s.y, row, p.r2, p.lut, lane, part, nparts);
     }
 }
 
 // Part `part` of `nparts` of H listed items of one index, counted together:
 // the rows are those that reach any of the H spheres, and a candidate once
 // loaded is tested against every centre.
-template <int H, bool SHORT>
+template <int R, int H, bool SHORT>
 __device__ __forceinline__ void count_items(const CountParams& p, const LaneParams& q, const uint2* it, uint32_t part,
                                             uint32_t nparts, uint32_t* __restrict__ cols,
                                             const uint32_t* __restrict__ slots, int lane) {
@@ -557,34 +753,10 @@ __device__ __forceinline__ void count_items(const CountParams& p, const LanePara
     unsigned char* mycol = reinterpret_cast<unsigned char*>(cols) + 4 * (lane >> 1);
     const uint32_t one = (lane & 1) ? 65536u : 1u;
     uint32_t held = 0;  // bound of any 16-bit counter
-    for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
-        // lane r: slot range of row rb + r, clipped in x to the spheres
-        uint32_t a = 0, e = 0;
-        const uint32_t r = rb + (uint32_t)lane;
-        if (r < im.nrows) {
-            int yy, zz, xa = im.x1 + 1, xb = im.x0 - 1;
-            row_yz(im, r, &yy, &zz);
-#pragma unroll
-            for (int k = 0; k < H; ++k) {
-                const float gy = cell_gap(c[k].y, yy, p.h[1], p.g.G[1]), gz = cell_gap(c[k].z, zz, p.h[2], p.g.G[2]);
-                const float rem =
-                    __fadd_rn(__fsub_rn(__fsub_rn(p.r2p, __fmul_rn(gy, gy)), __fmul_rn(gz, gz)), p.r2slack);
-                if (rem >= 0.0f) {
-                    // approximate square root: its error (< 1e-6 relative) is far inside the margin
-                    float xr = rem > 0.0f ? __fmul_rn(rem, rsqrtf(rem)) : 0.0f;
-                    xr = __fadd_rn(xr, 1e-3f + 1e-6f * (fabsf(c[k].x) + xr));
-                    xa = min(xa, cell_of(__fsub_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
-                    xb = max(xb, cell_of(__fadd_rn(c[k].x, xr), p.g.inv_h[0], p.g.G[0]));
-                }
-            }
-            xa = max(xa, im.x0);
-            xb = min(xb, im.x1);
-            if (xa <= xb) {
-                const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
-                a = __ldg(cs + rc + xa);
-                e = __ldg(cs + rc + xb + 1);
-            }
-        }
+    const uint32_t nranges = box_ranges<R>(im);
+    for (uint32_t rb = 0; rb < nranges; rb += 32u) {
+        const uint2 range = lane_range<R, H>(p, q, cs, im, c, rb + (uint32_t)lane, nranges);
+        const uint32_t a = range.x, e = range.y;
         // this warp's share of the rows' candidates, [tb, te) of the flattened sequence
         const uint32_t len = e - a;
         uint32_t incl = len;
@@ -735,7 +907,8 @@ __device__ __forceinline__ bool paired(const CountParams& p, const uint2* it, ui
     return dx * dx + dy * dy + dz * dz <= p.r2max;
 }
 
-__global__ void __launch_bounds__(HV_THREADS, HV_BLOCKS)
+template <int R, int BLOCKS>
+__global__ void __launch_bounds__(HV_THREADS, BLOCKS)
 k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
     const uint32_t nhuge = min(q.ctl[1], q.cap), nother = min(q.ctl[2], q.cap);
@@ -769,20 +942,20 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
             for (uint32_t j = 0; j < 2u; ++j)
                 it[j] = j < n ? q.list[huge ? 2u * k + j : q.cap - 1u - (2u * k + j)] : make_uint2(0u, 0u);
             if (paired(p, it, n)) {
-                if (phase == 0) count_items<2, false>(p, q, it, part, nparts, cols, slots, lane);
+                if (phase == 0) count_items<R, 2, false>(p, q, it, part, nparts, cols, slots, lane);
             } else if (phase == 1) {
 #pragma unroll 1
                 for (uint32_t j = 0; j < n; ++j) {
                     const uint2 one = j ? it[1] : it[0];
                     if (!(one.y & (kItemZone | kItemFar | kItemShort)))
-                        count_items<1, false>(p, q, &one, part, nparts, cols, slots, lane);
+                        count_items<R, 1, false>(p, q, &one, part, nparts, cols, slots, lane);
                 }
             } else if (phase == 2) {
 #pragma unroll 1
                 for (uint32_t j = 0; j < n; ++j) {
                     const uint2 one = j ? it[1] : it[0];
-                    if (one.y & (kItemZone | kItemFar)) count_literal(p, q, one, part, nparts, lane);
-                    else if (one.y & kItemShort) count_items<1, true>(p, q, &one, part, nparts, cols, slots, lane);
+                    if (one.y & (kItemZone | kItemFar)) count_literal<R>(p, q, one, part, nparts, lane);
+                    else if (one.y & kItemShort) count_items<R, 1, true>(p, q, &one, part, nparts, cols, slots, lane);
                 }
             }
         }
@@ -800,8 +973,10 @@ bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
 
 uint64_t lane_list_items(uint64_t nhalos, int nidx) { return (uint64_t)nidx * (nhalos + nhalos / 2 + 1024); }
 
-int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s,
-                      const LaneScratch* given) {
+namespace {
+template <int R>
+int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
+                  const LaneModel* model) {
     const auto& L = qq->lane;
     LaneParams q{};
     q.slots = L.slots;
@@ -816,6 +991,12 @@ int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p,
     std::memcpy(&km, &p.r2max, 4);
     q.zone = km - q.zone0;
     q.cmax = L.cmax;
+    if (model) {
+        q.leaves = model->leaves;
+        q.root = model->root;
+        q.wpref = reinterpret_cast<const uint32_t*>(p.mpts[0]) + 3;
+        q.key_shift = model->key_shift;
+    }
     StreamScratch scr(s);
     if (given) {
         q.ctl = given->ctl;
@@ -841,19 +1022,34 @@ int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p,
     // walks are left to the list (1e5 clustered halos on 2e7 particles at R =
     // 10, 1.3 waves: 1.06 ms without this, 0.78 with it).
     q.huge = p.nhalos < (uint64_t)ctx->num_sms * HV_WARPS * HV_BLOCKS * 4 ? kHugeFew : kHuge;
-    q.walk_max = (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(96, nbatch * 8 / (uint64_t)ctx->num_sms));
+    q.walk_max = (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(160, nbatch * 8 / (uint64_t)ctx->num_sms));
     const size_t smem_b = HV_WARPS * 2 * (size_t)(L.ncol + 1) * 64 + (size_t)L.nslots * 4;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
     const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
-    k_lane_count<<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
+    k_lane_count<R><<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
     int per_sm = 0;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_listed_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
-    SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_listed_count, HV_THREADS, smem_b));
+    auto listed = k_listed_count<R, HV_BLOCKS>;
+    if constexpr (R == RANGE_ROWS)
+        if (given) listed = k_listed_count<R, HV_BLOCKS_NOALLOC>;
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(listed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+    SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, listed, HV_THREADS, smem_b));
     if (per_sm < 1) per_sm = 1;
-    k_listed_count<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
+    listed<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
     return SJCS_OK;
+}
+}  // namespace
+
+int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
+                      const LaneScratch* given) {
+    return launch_ranges<RANGE_ROWS>(ctx, q, p, s, given, nullptr);
+}
+
+int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
+                            const LaneModel* model) {
+    return model ? launch_ranges<RANGE_MODEL>(ctx, q, p, s, nullptr, model)
+                 : launch_ranges<RANGE_CELLS>(ctx, q, p, s, nullptr, nullptr);
 }
 
 }  // namespace sjcs

@@ -20,6 +20,17 @@ uint64_t lane_list_items(uint64_t nhalos, int nidx);
 // Count q against the p.nidx indexes of p (mpts, mcs, mn) on stream s.
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, cudaStream_t s,
                       const LaneScratch* given = nullptr);
+// The same over a Morton index (p.nidx == 1, p.g its cells per axis, mcs[0] its
+// offset table); with a model, ranks come from it.
+struct LearnedLeaf;
+struct LearnedRoot;
+struct LaneModel {
+    const LearnedLeaf* leaves;
+    const LearnedRoot* root;
+    int key_shift;  // 63 - 3 * level
+};
+int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, cudaStream_t s,
+                            const LaneModel* model);
 // launch_shell_count under the static schedule without allocating.
 int launch_shell_count_noalloc(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx, const LaneScratch& scratch,
                                cudaStream_t s);

@@ -18,6 +18,7 @@
 #include <cmath>
 
 #include "count_common.cuh"
+#include "lane_count.cuh"
 #include "morton.cuh"
 #include "queue_common.cuh"
 #include "sjcs_internal.cuh"
@@ -360,8 +361,6 @@ template <int LOOK, int BIN, bool BIG>
 int launch_mq(sjcs_ctx* ctx, const CountParams& p, const MortonParams& m, const Schedule& sc, size_t smem,
               cudaStream_t s) {
     const uint64_t n = p.nhalos;
-    if (n * (uint64_t)sc.max_pieces >= (1ull << 32))
-        return fail(SJCS_ERR_INVALID, "queue schedule: nhalos * max_pieces must stay below 2^32");
     const uint32_t ntiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
     StreamScratch scr(s);  // freed (stream-ordered) after the kernels below
     uint32_t *key, *ord, *ctl, *hist, *rhist;
@@ -435,6 +434,18 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
     p.prune = q->monotone && std::isfinite(q->r2max) ? 1 : 0;
     p.reach = reach_of(q->r2max, p.prune);
     p.counts = q->counts;
+    if (sc && sc->mode == SJCS_SCHED_QUEUE && q->nhalos * (uint64_t)sc->max_pieces >= (1ull << 32))
+        return fail(SJCS_ERR_INVALID, "queue schedule: nhalos * max_pieces must stay below 2^32");
+    p.g = idx->geom;
+    for (int a = 0; a < 3; ++a) p.h[a] = 1000.0f / (float)idx->geom.G[a];
+    p.nidx = 1;
+    p.mpts[0] = idx->pts;
+    p.mcs[0] = idx->cell_start;
+    p.mn[0] = (uint32_t)idx->n;
+    if (lane_count_applies(q, p)) {
+        const LaneModel model{idx->leaves, idx->root, 63 - 3 * idx->level};
+        return launch_lane_count_cells(ctx, q, p, s, idx->kind == SJCS_INDEX_LEARNED ? &model : nullptr);
+    }
     MortonParams m{};
     m.table = idx->cell_start;
     m.leaves = idx->leaves;

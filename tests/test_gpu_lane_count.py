@@ -14,10 +14,10 @@ from spatialjoincountovershells_b200 import _native as nat
 pytestmark = pytest.mark.gpu
 
 
-def _count(ctx, files, h, r2, periodic=True, hint=0.0, grid=None, sched=nat.SCHED_AUTO):
+def _count(ctx, files, h, r2, periodic=True, hint=0.0, grid=None, sched=nat.SCHED_AUTO, kind=nat.INDEX_GRID, level=0):
     q = ctx.query(h, r2, periodic=periodic)
     q.set_schedule(sched)
-    idx = [ctx.build_index(f, radius_hint=hint, grid=grid) for f in files]
+    idx = [ctx.build_index(f, radius_hint=hint, grid=grid, kind=kind, level=level) for f in files]
     q.count_many(idx)
     out = q.read_counts()
     for i in idx:
@@ -121,3 +121,28 @@ def test_wide_radius_ratio_and_close_shells(ctx):
               np.array([1.0, np.nextafter(last, np.float32(0)), last], np.float32), np.array([0.0, 25.0, last], np.float32)]
     for r2 in tables:
         assert np.array_equal(_count(ctx, [p], h, r2, hint=20.0), _want([p], h, r2))
+
+
+@pytest.mark.parametrize("kind", [nat.INDEX_MORTON, nat.INDEX_LEARNED])
+@pytest.mark.parametrize("level", [1, 3, 5, 7])
+@pytest.mark.parametrize("periodic", [True, False])
+def test_morton_cells(ctx, kind, level, periodic):
+    """Boxes of one cell to more than 400, dense and light halos together."""
+    rng = np.random.default_rng(980)
+    clump = (np.array([500.0, 3.0, 997.0]) + rng.normal(0, 2.0, (60000, 3))) % 1000.0
+    p = np.concatenate([clump, rng.uniform(0, 1000, (20000, 3))]).astype(np.float32)
+    at = (np.array([500.0, 3.0, 997.0]) + rng.normal(0, 2.0, (40, 3))) % 1000.0
+    h = np.concatenate([at, rng.uniform(0, 1000, (600, 3))]).astype(np.float32)
+    r2 = nat.radius_table(0.05, 25.0, 40)
+    assert np.array_equal(_count(ctx, [p], h, r2, periodic, kind=kind, level=level), _want([p], h, r2, periodic))
+
+
+@pytest.mark.parametrize("kind", [nat.INDEX_MORTON, nat.INDEX_LEARNED])
+def test_morton_full_list_and_odd_values(ctx, kind):
+    rng = np.random.default_rng(990)
+    p = (rng.normal(0, 40, (4000, 3)) % 1000.0).astype(np.float32)
+    p[:4] = [[np.nan, 1, 1], [np.inf, 2, 2], [3, -np.inf, 3], [-50, 1200, 3]]
+    h = (rng.normal(0, 6, (3000, 3)) % 1000.0).astype(np.float32)
+    h[:5] = [[np.nan, 5, 5], [np.inf, 5, 5], [-40, 1190, 2], [5000, 5, 5], [1e30, 1, 1]]
+    r2 = nat.radius_table(0.5, 30.0, 20)
+    assert np.array_equal(_count(ctx, [p], h, r2, kind=kind, level=6), _want([p], h, r2))
