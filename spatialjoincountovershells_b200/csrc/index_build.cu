@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "morton.cuh"
 #include "radix_sort.cuh"
 #include "sjcs_internal.cuh"
 
@@ -183,14 +184,29 @@ __device__ __forceinline__ uint32_t pb_block_scan(uint32_t v, uint32_t* ws, uint
 
 __device__ __forceinline__ uint32_t pb_key(const float4& r) { return __float_as_uint(r.w); }
 
+// Cell key of a particle: the grid's cell number, or the level-L Morton code.
+struct GridKey {
+    GridGeom g;
+    __device__ __forceinline__ uint32_t operator()(float x, float y, float z) const { return cell_key(g, x, y, z); }
+};
+struct MortonKey {
+    float scale;  // 2^L / 1000: the same cells as the top L bits of morton_q
+    int G;
+    __device__ __forceinline__ uint32_t operator()(float x, float y, float z) const {
+        return morton_cell((uint32_t)cell_of(x, scale, G), (uint32_t)cell_of(y, scale, G),
+                           (uint32_t)cell_of(z, scale, G));
+    }
+};
+
 // top_hist[cell >> shift] += 1 for every particle (at most PB_THREADS bins,
 // counted in shared memory first).  Block b takes tiles `tiles`*b ..
 // (one reduction per bin for all of them); each tile's x,y,z are staged in
 // shared memory with coalesced 16-byte copies (cp.async when the array is
 // 16-byte aligned) and the keys taken from there.
 constexpr uint32_t PB_TOP_TILES = 4;
+template <class Key>
 __global__ void __launch_bounds__(PB_THREADS)
-k_pb_top_hist(const float* __restrict__ xyz, int aligned, uint64_t n, GridGeom g, int shift,
+k_pb_top_hist(const float* __restrict__ xyz, int aligned, uint64_t n, Key key, int shift,
               uint32_t* __restrict__ top_hist, uint32_t tiles) {
     __shared__ uint32_t sh[PB_THREADS];
     extern __shared__ float4 stage4[];
@@ -217,7 +233,7 @@ k_pb_top_hist(const float* __restrict__ xyz, int aligned, uint64_t n, GridGeom g
 #pragma unroll
         for (int i = 0; i < PB_ITEMS; ++i) {
             const uint32_t loc = (uint32_t)i * PB_THREADS + (uint32_t)tid;
-            if (loc < len) atomicAdd(&sh[cell_key(g, sx[3 * loc], sx[3 * loc + 1], sx[3 * loc + 2]) >> shift], 1u);
+            if (loc < len) atomicAdd(&sh[key(sx[3 * loc], sx[3 * loc + 1], sx[3 * loc + 2]) >> shift], 1u);
         }
     }
     __syncthreads();
@@ -319,10 +335,10 @@ __device__ __forceinline__ uint32_t pb_stage(const float* __restrict__ base, int
 // A record's digit is (key >> shift) & (2^bits - 1) and its room is reserved
 // from cursors[(bucket << cur_shift) + digit].  With `mid` given, the pass
 // also writes mid[slot] = (key >> sb) & mid_mask beside every record.
-template <bool kTiles>
+template <bool kTiles, class Key>
 __global__ void __launch_bounds__(PB_THREADS, 2)
 k_pb_partition(const float* __restrict__ xyz, int xyz_aligned, const float4* __restrict__ in,
-               const PbTile* __restrict__ tiles, const uint32_t* __restrict__ ntiles, uint64_t n, GridGeom g,
+               const PbTile* __restrict__ tiles, const uint32_t* __restrict__ ntiles, uint64_t n, Key key,
                int shift, int bits, int cur_shift, uint32_t* __restrict__ cursors, float4* __restrict__ out,
                uint16_t* __restrict__ mid, int sb, uint32_t mid_mask) {
     __shared__ uint32_t cnt[PB_THREADS];  // one bin per thread (digits of <= 9 bits)
@@ -358,7 +374,7 @@ k_pb_partition(const float* __restrict__ xyz, int xyz_aligned, const float4* __r
             const uint32_t loc = (uint32_t)i * PB_THREADS + (uint32_t)tid;
             if (loc < len) {
                 const float x = sx[off + 3 * loc], y = sx[off + 3 * loc + 1], z = sx[off + 3 * loc + 2];
-                v[i] = make_float4(x, y, z, __uint_as_float(cell_key(g, x, y, z)));
+                v[i] = make_float4(x, y, z, __uint_as_float(key(x, y, z)));
             }
         }
     } else {
@@ -509,34 +525,36 @@ int segment_bits(int kb) {
     return kb <= PB_GROUP_BITS + 9 ? std::max(PB_MIN_SEG_BITS, kb - 9) : std::max(PB_MIN_SEG_BITS, kb - 18);
 }
 
+template <class Key>
 int set_partition_smem() {
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_top_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_top_hist<Key>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)PB_STAGE_SMEM));
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<true, Key>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)PB_SMEM));
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_partition<false, Key>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)PB_SMEM));
     SJCS_CUDA_TRY(cudaFuncSetAttribute(k_pb_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
     return SJCS_OK;
 }
 
-// The partition build into pts (n records) and cs (ncells + 1 entries).
-int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, float4* pts, uint32_t* cs,
-                           cudaStream_t s) {
+// The partition build into pts (n records) and cs (ncells + 1 entries) by a
+// cell key of kb <= 30 bits.
+template <class Key>
+int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t ncells, float4* pts, uint32_t* cs,
+                      cudaStream_t s) {
     if (n == 0) {
-        SJCS_CUDA_TRY(cudaMemsetAsync(cs, 0, (g.ncells + 1) * sizeof(uint32_t), s));
+        SJCS_CUDA_TRY(cudaMemsetAsync(cs, 0, (ncells + 1) * sizeof(uint32_t), s));
         return SJCS_OK;
     }
-    const int kb = grid_key_bits(g);
     const int sb = segment_bits(kb);
     const int upper = kb > sb ? kb - sb : 0;  // bits above the segment
     const int bits_mid = upper > 9 ? upper - 9 : 0;
     const int bits_top = upper - bits_mid;
-    const uint64_t nseg = (g.ncells + (1ull << sb) - 1) >> sb;
+    const uint64_t nseg = (ncells + (1ull << sb) - 1) >> sb;
     const uint32_t ntop = (uint32_t)((nseg + (1ull << bits_mid) - 1) >> bits_mid);
     const uint64_t ntiles_in = (n + PB_TILE - 1) / PB_TILE;
     const uint64_t ntiles_mid = ntiles_in + ntop;  // bound on the middle pass's tiles
-    const uint64_t ngroups = g.ncells / PB_GROUP_CELLS + 1;  // the last one holds cell_start[ncells]
+    const uint64_t ngroups = ncells / PB_GROUP_CELLS + 1;  // the last one holds cell_start[ncells]
     const int aligned = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
 
     StreamScratch scr(s);
@@ -560,12 +578,12 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         seg = top;
     }
     const int top_shift = sb + bits_mid;
-    int rc = set_partition_smem();
+    int rc = set_partition_smem<Key>();
     if (rc) return rc;
     SJCS_CUDA_TRY(cudaMemsetAsync(top, 0, ((uint64_t)ntop + 1) * sizeof(uint32_t), s));
     // four tiles a block once every SM has blocks enough
     const uint32_t per = ntiles_in >= 148ull * 4 * PB_TOP_TILES ? PB_TOP_TILES : 1u;
-    k_pb_top_hist<<<(unsigned)((ntiles_in + per - 1) / per), PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, g,
+    k_pb_top_hist<Key><<<(unsigned)((ntiles_in + per - 1) / per), PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, key,
                                                                                           top_shift, top, per);
     SJCS_LAUNCH_CHECK();
     rc = exclusive_scan_u32(top, (uint64_t)ntop + 1, s, nullptr, cur_top);
@@ -574,8 +592,8 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
     // last pass), else tmp; with a middle pass it also writes the middle digits
     float4* a_out = bits_mid ? pts : tmp;
     const uint32_t mid_mask = (1u << bits_mid) - 1u;
-    k_pb_partition<false><<<(unsigned)ntiles_in, PB_THREADS, PB_SMEM, s>>>(
-        d_xyz, aligned, nullptr, nullptr, nullptr, n, g, top_shift, bits_top, 0, cur_top, a_out, mid, sb, mid_mask);
+    k_pb_partition<false, Key><<<(unsigned)ntiles_in, PB_THREADS, PB_SMEM, s>>>(
+        d_xyz, aligned, nullptr, nullptr, nullptr, n, key, top_shift, bits_top, 0, cur_top, a_out, mid, sb, mid_mask);
     SJCS_LAUNCH_CHECK();
     if (bits_mid) {
         const unsigned tile_blocks = (unsigned)((ntiles_mid + PB_THREADS - 1) / PB_THREADS);
@@ -586,11 +604,11 @@ int build_grid_partitioned(const float* d_xyz, uint64_t n, const GridGeom& g, fl
         SJCS_LAUNCH_CHECK();
         rc = exclusive_scan_u32(seg, nseg + 1, s, nullptr, cur_seg);
         if (rc) return rc;
-        k_pb_partition<true><<<(unsigned)ntiles_mid, PB_THREADS, PB_SMEM, s>>>(
-            nullptr, 0, pts, tiles, ntiles, n, g, sb, bits_mid, bits_mid, cur_seg, tmp, nullptr, sb, 0u);
+        k_pb_partition<true, Key><<<(unsigned)ntiles_mid, PB_THREADS, PB_SMEM, s>>>(
+            nullptr, 0, pts, tiles, ntiles, n, key, sb, bits_mid, bits_mid, cur_seg, tmp, nullptr, sb, 0u);
         SJCS_LAUNCH_CHECK();
     }
-    k_pb_cells<<<(unsigned)ngroups, PB_THREADS, PB_SMEM, s>>>(tmp, seg, nseg, sb, g.ncells, cs, pts);
+    k_pb_cells<<<(unsigned)ngroups, PB_THREADS, PB_SMEM, s>>>(tmp, seg, nseg, sb, ncells, cs, pts);
     SJCS_LAUNCH_CHECK();
     return SJCS_OK;
 }
@@ -608,13 +626,15 @@ int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const Gri
     const uint64_t nseg = (g.ncells + (1ull << sb) - 1) >> sb;  // <= 512
     const uint64_t ntiles = (n + PB_TILE - 1) / PB_TILE;
     const int aligned = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
-    int rc = set_partition_smem();
+    int rc = set_partition_smem<GridKey>();
     if (rc) return rc;
-    k_pb_top_hist<<<(unsigned)ntiles, PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, g, sb, b.top, 1u);
+    k_pb_top_hist<GridKey><<<(unsigned)ntiles, PB_THREADS, PB_STAGE_SMEM, s>>>(
+        d_xyz, aligned, n, GridKey{g}, sb, b.top, 1u);
     SJCS_LAUNCH_CHECK();
     rc = exclusive_scan_u32(b.top, nseg + 1, s, nullptr, b.cursors);
     if (rc) return rc;
-    k_pb_partition<false><<<(unsigned)ntiles, PB_THREADS, PB_SMEM, s>>>(d_xyz, aligned, nullptr, nullptr, nullptr, n, g,
+    k_pb_partition<false, GridKey><<<(unsigned)ntiles, PB_THREADS, PB_SMEM, s>>>(d_xyz, aligned, nullptr, nullptr, nullptr, n,
+                                                                        GridKey{g},
                                                                         sb, bits_top, 0, b.cursors, b.tmp, nullptr, sb,
                                                                         0u);
     SJCS_LAUNCH_CHECK();
@@ -702,6 +722,12 @@ int fill_cell_table(const uint32_t* sorted_cells, uint64_t n, uint64_t ncells, u
     return SJCS_OK;
 }
 
+int build_morton_table(const float* d_xyz, uint64_t n, int level, float4* pts, uint32_t* table, cudaStream_t s) {
+    const int G = 1 << level;
+    return build_partitioned(d_xyz, n, MortonKey{(float)G / 1000.0f, G}, std::max(1, 3 * level), 1ull << (3 * level),
+                             pts, table, s);
+}
+
 int build_grid_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, const GridGeom& g,
                      sjcs_index* idx, cudaStream_t s) {
     (void)ctx;
@@ -710,7 +736,7 @@ int build_grid_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, const GridGe
     SJCS_CUDA_TRY(cudaMallocAsync(&idx->pts, nalloc * sizeof(float4), s));
     SJCS_CUDA_TRY(cudaMallocAsync(&idx->cell_start, (g.ncells + 1) * sizeof(uint32_t), s));
     if (grid_key_bits(g) <= PB_MAX_KEY_BITS)
-        return build_grid_partitioned(d_xyz, n, g, reinterpret_cast<float4*>(idx->pts), idx->cell_start, s);
+        return build_partitioned(d_xyz, n, GridKey{g}, grid_key_bits(g), g.ncells, idx->pts, idx->cell_start, s);
 
     LsdBuffers b{};
     b.pts = idx->pts;

@@ -6,19 +6,19 @@
 // in each query box, so any layout that hands the count kernel a superset of
 // the in-box particles gives the reference's counts.
 //
-// Build of one particle file:
+// Build of one particle file (plain form: the partition build of
+// index_build.cu by level-L cell; learned form:)
 //   sort     stable LSD radix sort by the 63-bit Morton key, 8 passes of 8
 //            bits.  The key is carried as two u32 halves: passes 0-3 sort on
 //            the low half with the high half riding in the payload's 4th word,
 //            pass 4 swaps them, passes 4-7 sort on the high half.  The last
 //            pass writes the particles as float4 (4th word = the key's level-10
-//            prefix), the level-L cell of every particle and (learned kind)
-//            the full keys
+//            prefix), the level-L cell of every particle and the full keys
 //   table    table[c] = first slot of level-L cell c (the plain offset table)
-//   train    (learned kind) equal-population leaf rank ranges, a fitted
+//   train    equal-population leaf rank ranges, a fitted
 //            fp32 slope and bias per leaf and its exact max error, the
 //            root's directory over the leaves' anchors
-//   judge    (learned kind, on request) the corrected model rank of every
+//   judge    (on request) the corrected model rank of every
 //            level-L cell boundary is compared with the table; any mismatch
 //            switches the count kernel to the table for this index
 #include <algorithm>
@@ -61,12 +61,12 @@ struct PaySwapKey {  // payload's 4th word becomes the low half carried so far
 struct SinkMorton {
     uint4* __restrict__ pts;
     uint32_t* __restrict__ cells;                  // level-L cell of every slot
-    unsigned long long* __restrict__ keys;         // full keys (learned kind) or null
+    unsigned long long* __restrict__ keys;         // full keys
     int cell_shift;                                // 31 - 3L: high half -> level-L cell
     __device__ __forceinline__ void operator()(uint32_t g, uint32_t hi, const uint4& v) const {
         pts[g] = make_uint4(v.x, v.y, v.z, hi >> 1);  // level-10 prefix = key >> 33
         cells[g] = hi >> cell_shift;
-        if (keys) keys[g] = ((unsigned long long)hi << 32) | v.w;
+        keys[g] = ((unsigned long long)hi << 32) | v.w;
     }
 };
 
@@ -282,6 +282,15 @@ int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level,
         return SJCS_OK;
     }
 
+    // The plain table only needs the cells together: the partition build by the
+    // level-L code (three streaming passes or fewer) instead of eight sort
+    // passes (2e7 particles: 2.3 -> 0.4 ms).
+    if (!learned) {
+        const int rc = build_morton_table(d_xyz, n, level, idx->pts, idx->cell_start, s);
+        if (rc) return rc;
+        cudaEventRecord(idx->ev_train0, s);
+        return SJCS_OK;
+    }
     const uint32_t ntiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
     StreamScratch scr(s);
     uint32_t *kx, *ky, *hist, *partials, *cells, *ngaps, *first = nullptr;
@@ -297,10 +306,8 @@ int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level,
     SJCS_CUDA_TRY(scr.alloc(&partials, scan_partials_needed((uint64_t)RS_BINS * ntiles) * sizeof(uint32_t)));
     SJCS_CUDA_TRY(scr.alloc(&gaps, (size_t)kGridGaps * 12));
     SJCS_CUDA_TRY(scr.alloc(&ngaps, sizeof(uint32_t)));
-    if (learned) {
-        SJCS_CUDA_TRY(scr.alloc(&keys, n * sizeof(unsigned long long)));
-        SJCS_CUDA_TRY(scr.alloc(&first, (kLeaves + 1) * sizeof(uint32_t)));
-    }
+    SJCS_CUDA_TRY(scr.alloc(&keys, n * sizeof(unsigned long long)));
+    SJCS_CUDA_TRY(scr.alloc(&first, (kLeaves + 1) * sizeof(uint32_t)));
 
     // passes 0-3: low half (A = x buffers after even passes, B = y after odd)
     int rc = radix_pass(MortonLoKey{d_xyz}, MortonPay{d_xyz}, SinkRecords{kx, px}, n, 0, hist, ntiles, s, partials);
@@ -325,7 +332,6 @@ int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level,
     rc = fill_cell_table(cells, n, ncells, idx->cell_start, gaps, ngaps, s);
     if (rc) return rc;
     cudaEventRecord(idx->ev_train0, s);
-    if (!learned) return SJCS_OK;
 
     k_root<<<1, 1, 0, s>>>(keys, n, idx->root);
     SJCS_LAUNCH_CHECK();

@@ -11,6 +11,7 @@
 //
 // HBM layout of a Morton index over n particles:
 //   pts[n]              float4 (x, y, z, level-10 prefix bits), sorted by key
+//                       (plain form: grouped by level-L cell, 4th word the code)
 //   table[8^L + 1]      u32 plain offset table of the index's cell level L
 //   leaves[4096]        LearnedLeaf, then the root's directory (2^16 + 1 u16),
 //   root                one LearnedRoot                         (learned kind)
