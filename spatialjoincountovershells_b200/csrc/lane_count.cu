@@ -6,7 +6,7 @@
 //                plans its box's rows of cells (at most 5 x 5), clips each in x
 //                to the sphere, fetches the rows' slot ranges and then walks
 //                its own candidates one by one; its counts go to a private
-//                column of 16-bit counters in shared memory (no atomics) and
+//                column of 16-bit counters in shared memory and
 //                from there to the halo's row.  Shifted periodic images wait
 //                in a per-warp list until there are 32 of them and are then
 //                walked the same way.
@@ -33,16 +33,17 @@
 // Why lanes walk their own rows: mapping 32 lanes onto one halo's ~21 rows of
 // ~5 candidates cost a five-step shuffle search per window and shared-memory
 // atomics on the few shells that hold most of the volume, 484-559 warp
-// instructions per halo and file; this form takes about 235.  The price is a
+// instructions per halo and file; this form takes about 235 (at 7 % of halos
+// near a face).  The price is a
 // gather of 32 addresses per load, but an L1 gather of 32 x 16 bytes takes
 // 11.0 cycles per SM against 5.2 coalesced and 9.2 from shared memory (random
 // slots, measured), so staging the candidates would not pay.  What bounds it:
-// the L1/shared data pipe (81 % of its peak, 47 % issue active).
+// the L1/shared data pipe (75 % of its peak, 51 % issue active).
 //
 // k_listed_count runs at 68 % of both the data pipe and issue.
 //
 // Measured (B200, count kernels of one call, warp-per-halo kernel -> this one):
-// 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.27 ms; 1e6 on
+// 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.00 ms; 1e6 on
 // 1e7 0.42 -> 0.20; 1e6 clustered halos on 3e7 clustered particles 9.2 (static
 // schedule) and 7.1 (queue) -> 3.43, one item at a time 4.28; 1e6 on 5e7, R =
 // 20, 64 shells 55 and 40.8 -> 18.5, one item at a time 24.3; 1e5 on 2e7, R =
@@ -62,12 +63,12 @@ namespace {
 using namespace count;
 
 // One block of 16 warps per SM: its warps take neighbouring batches and share
-// their particle lines in L1 (4.32 ms at 1e8 x 1e7; two blocks of 8 warps 4.68,
-// four of 4 5.08; 14 warps 4.46, 20 warps 4.84: more counters, less L1).
+// their particle lines in L1 (4.00 ms at 1e8 x 1e7; 18 warps 4.31, 20 4.05, 24
+// with spills 4.80; in smaller blocks the same warps took 8 to 17 % longer).
 constexpr int LN_WARPS = 16;
 constexpr int LN_ROWS = 25;       // rows of cells a lane walks
 constexpr uint32_t LN_PEND = 96;  // shifted images waiting per warp
-constexpr int LN_DEPTH = 4;       // candidates in flight per lane (2: 4.42 ms, 3: 4.35, 6: 4.34)
+constexpr int LN_DEPTH = 4;       // candidates in flight per lane (3: 1 % longer, 2: 2 %, 6: 1 %)
 // Listed items: 20 blocks of one warp per SM (96 registers; five blocks of four
 // warps take 2 % longer, 16 warps without spills 11 %).
 constexpr int HV_WARPS = 1, HV_THREADS = HV_WARPS * 32, HV_BLOCKS = 20;
@@ -163,11 +164,20 @@ __device__ __forceinline__ uint32_t listed_cost(uint32_t T, uint32_t rows, uint3
 }
 
 // Shared memory of one warp beside its counters.
-struct LaneRows {
-    uint32_t s0[LN_ROWS + 2][32];   // first slot of a lane's row
+template <bool PACK>
+struct LaneRows;
+template <>
+struct LaneRows<false> {
+    uint32_t s0[LN_ROWS + 2][32];   // first slot of a lane's range
     uint16_t len[LN_ROWS + 2][32];  // its candidates
     uint32_t pend[LN_PEND];         // halo | shifted axes << 29
 };
+template <>
+struct LaneRows<true> {
+    uint32_t row[LN_ROWS + 2][32];  // first slot less the lane's first one << 8 | candidates (<= 255)
+    uint32_t pend[LN_PEND];
+};
+constexpr uint32_t kPackSpan = 1u << 24, kPackLen = 255;
 
 // A coordinate's periodic image: lo < 0 takes precedence (MultiRangeCount.c:38-43).
 __device__ __forceinline__ float shifted(float v, float half) {
@@ -236,18 +246,20 @@ __device__ __forceinline__ void push_items(const CountParams& p, const LaneParam
     if (push && !fits) serial_count<R>(p, c, flags, q.safe2);
 }
 
-template <int R>
+template <int R, bool PACK>
 __global__ void __launch_bounds__(LN_WARPS * 32, 1)
 k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    LaneRows* rows = reinterpret_cast<LaneRows*>(smem) + warp;
+    LaneRows<PACK>* rows = reinterpret_cast<LaneRows<PACK>*>(smem) + warp;
     const int nwarps = (int)(blockDim.x >> 5);
-    uint32_t* cols32 = reinterpret_cast<uint32_t*>(reinterpret_cast<LaneRows*>(smem) + nwarps);
+    uint32_t* cols32 = reinterpret_cast<uint32_t*>(reinterpret_cast<LaneRows<PACK>*>(smem) + nwarps);
     const int colwords = (q.ncol + 1) * 16;
     uint32_t* slots = cols32 + nwarps * colwords;
     cols32 += warp * colwords;
-    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols32) + 2 * lane;
+    // two lanes' 16-bit counters to a word
+    unsigned char* mycol = reinterpret_cast<unsigned char*>(cols32) + 4 * (lane >> 1);
+    const uint32_t one = (lane & 1) ? 65536u : 1u;
     for (int i = tid; i < q.nslots; i += (int)blockDim.x) slots[i] = q.slots[i];
     for (int i = lane; i < colwords; i += 32) cols32[i] = 0u;
     __syncthreads();
@@ -328,6 +340,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                 // whole box: long rows, more than the 16-bit counters hold, and
                 // lanes that would keep the others waiting.
                 uint32_t box = 0;
+                [[maybe_unused]] uint32_t first = 0, last = 0, longest = 0;
                 if (R == RANGE_ROWS && cand) {
                     // eight rows' loads in flight at a time
                     const uint32_t gx = (uint32_t)p.g.G[0], xl = (uint32_t)im.x0, xh = (uint32_t)im.x1 + 1u;
@@ -349,7 +362,14 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                             }
                         }
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) box += hi[u] - lo[u];
+                        for (int u = 0; u < 8; ++u) {
+                            box += hi[u] - lo[u];
+                            if (PACK) {
+                                longest = max(longest, hi[u] - lo[u]);
+                                last = max(last, hi[u]);
+                            }
+                        }
+                        if (PACK && r == 0u) first = lo[0];
                     }
                 } else if (cand) {
                     // from the table; the model would answer the same
@@ -373,7 +393,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                 // about what the sphere leaves of the box
                 const uint32_t est = box - (box >> 2) - (box >> 3), rows_est = nranges - (nranges >> 2);
                 if (chunked) {
-                    mine = cand && est <= q.walk_max;
+                    mine = cand && est <= q.walk_max && (!PACK || (longest <= kPackLen && last - first < kPackSpan));
                     const uint32_t mxT = __reduce_max_sync(0xffffffffu, mine ? est : 0u);
                     const uint32_t hc = listed_cost(est, rows_est, nranges);
                     uint32_t best = kStepCost * mxT, tau = mxT;
@@ -418,11 +438,19 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
             bool walked = false;
             for (int zb = 0; zb < zend; zb += planes) {
                 uint32_t m = 0, T = 0;
+                [[maybe_unused]] uint32_t base = 0;
+                [[maybe_unused]] bool wide = false;
                 auto keep = [&](uint32_t a, uint32_t e) {
                     const uint32_t l = e - a;
                     if (l) {
-                        rows->s0[m][lane] = a;
-                        rows->len[m][lane] = (uint16_t)l;
+                        if constexpr (PACK) {
+                            if (m == 0u) base = a;
+                            wide |= (l > kPackLen) | (a - base >= kPackSpan);
+                            rows->row[m][lane] = ((a - base) << 8) | l;
+                        } else {
+                            rows->s0[m][lane] = a;
+                            rows->len[m][lane] = (uint16_t)l;
+                        }
                         ++m;
                         T += l;
                     }
@@ -498,7 +526,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     }
                 }
                 // which lanes walk their own rows: the threshold with the least work
-                bool coop = !chunked && T > q.walk_max;
+                bool coop = !chunked && (T > q.walk_max || (PACK && wide));
                 uint32_t steps = __reduce_max_sync(0xffffffffu, coop ? 0u : T);
                 if (!chunked && steps > 160u) {
                     const uint32_t mxT = steps;
@@ -520,26 +548,57 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                 }
                 if (__any_sync(0xffffffffu, coop)) push_items<R>(p, q, coop, T > q.huge, h, file | S | (short_rows(T, m) ? kItemShort : 0u), c, lane);
                 if (steps) {
-                    // the list ends in a row of slots past the particles, which load nothing
-                    const uint32_t mm = coop ? 0u : m;
-                    rows->s0[mm][lane] = kEndSlot;
-                    rows->len[mm][lane] = 0xffffu;
-                    uint32_t j = rows->s0[0][lane], e = j + rows->len[0][lane];
-                    const uint32_t* rs = &rows->s0[1][lane];
-                    const uint16_t* rl = &rows->len[1][lane];
-                    uint32_t ns = *rs, nl = *rl;
+                    uint32_t j, e;
                     float4 buf[LN_DEPTH];
+                    // The lane's next candidate; past its last one nothing is loaded.
+                    // Packed ranges: one lookup per range, and 27 KB an SM less for
+                    // the lists, which L1 has instead (4.24 -> 4.00 ms at 1e8 x 1e7).
+                    [[maybe_unused]] uint32_t left = coop ? 0u : T, nw = 0;
+                    [[maybe_unused]] const uint32_t *rs = nullptr, *rw = nullptr;
+                    [[maybe_unused]] const uint16_t* rl = nullptr;
+                    [[maybe_unused]] uint32_t ns = 0, nl = 0;
+                    if constexpr (PACK) {
+                        const uint32_t w = left ? rows->row[0][lane] : 0u;
+                        j = base + (w >> 8);
+                        e = j + (w & 255u);
+                        rw = &rows->row[1][lane];
+                        nw = *rw;
+                    } else {
+                        // the list ends in a range of slots past the particles
+                        const uint32_t mm = coop ? 0u : m;
+                        rows->s0[mm][lane] = kEndSlot;
+                        rows->len[mm][lane] = 0xffffu;
+                        j = rows->s0[0][lane];
+                        e = j + rows->len[0][lane];
+                        rs = &rows->s0[1][lane];
+                        rl = &rows->len[1][lane];
+                        ns = *rs;
+                        nl = *rl;
+                    }
                     auto next = [&](float4& v) {
                         v.x = INFINITY;
-                        if (j < np) v = __ldg(pts + j);
-                        ++j;
-                        if (j == e) {
-                            j = ns;
-                            e = ns + nl;
-                            rs += 32;
-                            rl += 32;
-                            ns = *rs;
-                            nl = *rl;
+                        if constexpr (PACK) {
+                            const bool more = left != 0u;
+                            if (more) v = __ldg(pts + j);
+                            ++j;
+                            left -= more ? 1u : 0u;
+                            if (more && j == e) {
+                                j = base + (nw >> 8);
+                                e = j + (nw & 255u);
+                                rw += 32;
+                                nw = *rw;
+                            }
+                        } else {
+                            if (j < np) v = __ldg(pts + j);
+                            ++j;
+                            if (j == e) {
+                                j = ns;
+                                e = ns + nl;
+                                rs += 32;
+                                rl += 32;
+                                ns = *rs;
+                                nl = *rl;
+                            }
                         }
                     };
                     auto find = [&](const float4& v) {
@@ -560,8 +619,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                         for (int u = 0; u < LN_DEPTH; ++u) next(buf[u]);
 #pragma unroll
                         for (int u = 0; u < LN_DEPTH; ++u) {
-                            uint16_t* cnt = reinterpret_cast<uint16_t*>(mycol + at[u]);
-                            *cnt = (uint16_t)(*cnt + 1);
+                            atomicAdd(reinterpret_cast<uint32_t*>(mycol + at[u]), one);
                         }
                     }
                     walked = true;
@@ -573,7 +631,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                 uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
 #pragma unroll 4
                 for (int sh = 0; sh < q.ncol; ++sh) {
-                    const uint32_t v = *reinterpret_cast<uint16_t*>(mycol + sh * 64);
+                    const uint32_t v = *reinterpret_cast<uint16_t*>(mycol + 2 * (lane & 1) + sh * 64);
                     if (v) atomicAdd(row + sh, v);
                 }
                 __syncwarp();
@@ -974,7 +1032,7 @@ bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
 uint64_t lane_list_items(uint64_t nhalos, int nidx) { return (uint64_t)nidx * (nhalos + nhalos / 2 + 1024); }
 
 namespace {
-template <int R>
+template <int R, bool PACK>
 int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
                   const LaneModel* model) {
     const auto& L = qq->lane;
@@ -1013,7 +1071,7 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     // one block per SM (neighbouring batches share its L1); blocks of fewer
     // warps when there are not enough batches for every SM
     const uint64_t nbatch = (p.nhalos + 31) / 32;
-    const size_t warp_a = sizeof(LaneRows) + (size_t)(L.ncol + 1) * 64, table = (size_t)L.nslots * 4;
+    const size_t warp_a = sizeof(LaneRows<PACK>) + (size_t)(L.ncol + 1) * 64, table = (size_t)L.nslots * 4;
     constexpr size_t kMaxSmem = 227 * 1024;
     const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxSmem - table) / warp_a);  // >= 15 for any table
     const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + (uint64_t)ctx->num_sms - 1) / (uint64_t)ctx->num_sms);
@@ -1029,9 +1087,9 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     const uint64_t floor = nbatch <= (uint64_t)ctx->num_sms ? 0 : 160;
     q.walk_max = (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(floor, nbatch * 8 / (uint64_t)ctx->num_sms));
     const size_t smem_b = HV_WARPS * 2 * (size_t)(L.ncol + 1) * 64 + (size_t)L.nslots * 4;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count<R, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
     const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
-    k_lane_count<R><<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
+    k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
     int per_sm = 0;
     auto listed = k_listed_count<R, HV_BLOCKS>;
@@ -1048,13 +1106,18 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
 
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
                       const LaneScratch* given) {
-    return launch_ranges<RANGE_ROWS>(ctx, q, p, s, given, nullptr);
+    // Packed rows need the slots of a box's planes within 2^24 of each other;
+    // with more than 2^29 particles ordinary boxes would not be.
+    bool pack = true;
+    for (int i = 0; i < p.nidx; ++i) pack &= p.mn[i] <= (1u << 29);
+    return pack ? launch_ranges<RANGE_ROWS, true>(ctx, q, p, s, given, nullptr)
+                : launch_ranges<RANGE_ROWS, false>(ctx, q, p, s, given, nullptr);
 }
 
 int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
                             const LaneModel* model) {
-    return model ? launch_ranges<RANGE_MODEL>(ctx, q, p, s, nullptr, model)
-                 : launch_ranges<RANGE_CELLS>(ctx, q, p, s, nullptr, nullptr);
+    return model ? launch_ranges<RANGE_MODEL, false>(ctx, q, p, s, nullptr, model)
+                 : launch_ranges<RANGE_CELLS, false>(ctx, q, p, s, nullptr, nullptr);
 }
 
 }  // namespace sjcs
