@@ -971,6 +971,15 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
     extern __shared__ uint32_t smem[];
     const uint32_t nhuge = min(q.ctl[1], q.cap), nother = min(q.ctl[2], q.cap);
     if (nhuge + nother == 0u) return;
+    // Warps claim (two items, part); only huge items have several parts.  With
+    // fewer items than warps each is claimed alone, and blocks beyond the last
+    // claim leave at once.
+    const uint32_t warps = gridDim.x * HV_WARPS;
+    const uint32_t uh = nhuge < warps / 16u ? 1u : 2u, uo = nother < warps ? 1u : 2u;
+    const uint32_t mh = (nhuge + uh - 1u) / uh, mo = (nother + uo - 1u) / uo;
+    const uint32_t ph = mh >= (1u << 28) ? 1u : max(8u, min(64u, 4u * warps / max(mh, 1u)));
+    const uint32_t ch = mh * ph;
+    if (blockIdx.x * HV_WARPS >= ch + mo) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int colwords = 2 * (q.ncol + 1) * 16;
     uint32_t* slots = smem + HV_WARPS * colwords;
@@ -978,11 +987,6 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
     for (int i = tid; i < q.nslots; i += HV_THREADS) slots[i] = q.slots[i];
     for (int i = lane; i < colwords; i += 32) cols[i] = 0u;
     __syncthreads();
-    // Warps claim (two items, part); only huge items have several parts.
-    const uint32_t warps = gridDim.x * HV_WARPS;
-    const uint32_t mh = (nhuge + 1u) / 2u, mo = (nother + 1u) / 2u;
-    const uint32_t ph = mh >= (1u << 28) ? 1u : max(8u, min(64u, 4u * warps / max(mh, 1u)));
-    const uint32_t ch = mh * ph;
     // Pairs first, then long rows alone, then the rest: warps of an SM run the
     // same loop at a time (the three together exceed the instruction cache).
 #pragma unroll 1
@@ -994,11 +998,12 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
             if (i >= ch + mo) break;
             const bool huge = i < ch;
             const uint32_t k = huge ? i / ph : i - ch, part = huge ? i % ph : 0u;
-            const uint32_t nparts = huge ? ph : 1u, n = min(2u, (huge ? nhuge : nother) - 2u * k);
+            const uint32_t nparts = huge ? ph : 1u, per = huge ? uh : uo;
+            const uint32_t n = min(per, (huge ? nhuge : nother) - per * k);
             uint2 it[2];
 #pragma unroll
             for (uint32_t j = 0; j < 2u; ++j)
-                it[j] = j < n ? q.list[huge ? 2u * k + j : q.cap - 1u - (2u * k + j)] : make_uint2(0u, 0u);
+                it[j] = j < n ? q.list[huge ? per * k + j : q.cap - 1u - (per * k + j)] : make_uint2(0u, 0u);
             if (paired(p, it, n)) {
                 if (phase == 0) count_items<R, 2, false>(p, q, it, part, nparts, cols, slots, lane);
             } else if (phase == 1) {
