@@ -141,9 +141,33 @@ __device__ __forceinline__ uint32_t learned_rank(const LearnedRoot& rt, const Le
     return lo;
 }
 
-// N exact lower bounds at once (as learned_rank), the N bounded binary
-// searches advanced together so their probes are independent loads in flight
-// at the same time.  act[j] == false: out[j] = 0 and no memory is read.
+// N binary searches of [lo, hi) over the prefixes, advanced together so their
+// probes are independent loads in flight at the same time.
+template <int N>
+__device__ __forceinline__ void lower_bound_n(const uint32_t* __restrict__ wpref, const uint32_t (&qp)[N],
+                                              uint32_t (&lo)[N], uint32_t (&hi)[N]) {
+    for (;;) {
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < N; ++j) any |= lo[j] < hi[j];
+        if (!any) break;
+        uint32_t v[N], mid[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            mid[j] = lo[j] + ((hi[j] - lo[j]) >> 1);
+            v[j] = lo[j] < hi[j] ? __ldg(wpref + 4ull * mid[j]) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            if (lo[j] < hi[j]) {
+                if (v[j] < qp[j]) lo[j] = mid[j] + 1u;
+                else hi[j] = mid[j];
+            }
+        }
+    }
+}
+
+// N exact lower bounds at once (as learned_rank).  act[j] == false: out[j] = 0 and no memory is read.
 template <int N>
 __device__ __forceinline__ void learned_rank_n(const LearnedRoot& rt, const LearnedLeaf* __restrict__ leaves,
                                                const uint32_t* __restrict__ wpref, const uint64_t (&q)[N],
@@ -166,25 +190,7 @@ __device__ __forceinline__ void learned_rank_n(const LearnedRoot& rt, const Lear
         const uint64_t h64 = (uint64_t)P + lf.err + 1ull;
         hi[j] = h64 < (uint64_t)lf.r1 ? (uint32_t)h64 : lf.r1;
     }
-    for (;;) {
-        bool any = false;
-#pragma unroll
-        for (int j = 0; j < N; ++j) any |= lo[j] < hi[j];
-        if (!any) break;
-        uint32_t v[N], mid[N];
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            mid[j] = lo[j] + ((hi[j] - lo[j]) >> 1);
-            v[j] = lo[j] < hi[j] ? __ldg(wpref + 4ull * mid[j]) : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            if (lo[j] < hi[j]) {
-                if (v[j] < qp[j]) lo[j] = mid[j] + 1u;
-                else hi[j] = mid[j];
-            }
-        }
-    }
+    lower_bound_n<N>(wpref, qp, lo, hi);
 #pragma unroll
     for (int j = 0; j < N; ++j) out[j] = lo[j];
 }
