@@ -17,11 +17,11 @@ the build stream behind file k's count (its upload overlaps that count).
           Steps are independent jobs run as a pipeline: job k's count
           read-back (device to host) overlaps job k+1's uploads (host to
           device); every job's copies are inside the timed region.
-  roofline  the shell-count kernel (the fused k_shell_count_multi: one launch
-          counts the step's halos against all its files): algorithmic bytes
-          per halo-file (12 + 8*nrads + 12*density*(2R)^3 = 1532 B) x
-          halo-files per launch over its average launch time (CUDA events on
-          the count stream).
+  roofline  the shell count (k_lane_count, and k_listed_count for what it
+          leaves; one call counts the step's halos against all its files):
+          algorithmic bytes per halo-file (12 + 8*nrads +
+          12*density*(2R)^3 = 1532 B) x halo-files per call over the call's
+          average time (CUDA events on the count stream).
   cpu_baseline  the reference program (oracle/_ref/astr_rcount.exe) on a
           bounded sample of the same workload on this host's cores.
 
@@ -269,10 +269,11 @@ def parity_record(ref_counts, forms: dict, workload: str, radius) -> dict:
 def profile_traffic(halo_files: float, fused: bool = False):
     """DRAM bytes per count launch from the committed ncu summary of that
     kernel (bytes per halo-file), scaled to the launch's halo-files."""
-    p = ROOT / "profiles" / ("shell_count_multi_uniform.md" if fused else "shell_count_uniform.md")
+    p = ROOT / "profiles" / "lane_count_uniform.md"
     if not p.exists():
         return None
-    m = re.search(r"dram_bytes_per_halo_file:\s*([0-9.eE+]+)", p.read_text())
+    key = "dram_bytes_per_halo_file" if fused else "dram_bytes_per_halo_one_file"
+    m = re.search(key + r":\s*([0-9.eE+]+)", p.read_text())
     return float(m.group(1)) * halo_files if m else None
 
 
@@ -523,7 +524,7 @@ def run_ours(args, w, dist, rank, world, local):
         achieved = ALGO_BYTES_PER_HALO_FILE * hf / (count_ms / 1e3) / 1e9
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": profile_traffic(hf, files_per_call > 1),
-                "kernel": "k_shell_count_multi" if files_per_call > 1 else "k_shell_count",
+                "kernel": "k_lane_count",
                 "files_per_launch": round(files_per_call, 3), "launch_ms": round(count_ms, 3),
                 "algorithmic_bytes_per_launch": ALGO_BYTES_PER_HALO_FILE * hf,
                 "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind}
