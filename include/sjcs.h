@@ -63,7 +63,11 @@ extern "C" {
                                    every cell boundary with the offset table; on any mismatch the
                                    index answers from the table */
 
-/* count schedules: how the count kernel hands halos to warps */
+/* count schedules: how the count kernel hands halos to warps.  Tables of up to
+ * 128 increasing, positive, finite squared radii that are not too close to one
+ * another are counted with a lane per halo, whichever schedule is set: halos
+ * too heavy for a lane go to a list, the heaviest are split there.  Other
+ * tables are counted warp by warp, as the schedule says. */
 #define SJCS_SCHED_AUTO    0 /* the context's autotuned choice for this workload shape, else STATIC */
 #define SJCS_SCHED_STATIC  1 /* warps take halos strided over the Morton order, in batches of 32 */
 #define SJCS_SCHED_QUEUE   2 /* persistent warps pull work from a queue ordered by estimated candidate
@@ -284,11 +288,9 @@ int sjcs_query_create_device(sjcs_ctx *ctx, const float *d_halo_xyz, size_t stri
 int sjcs_query_count(sjcs_ctx *ctx, sjcs_query *q, const sjcs_index *idx);
 /* The counts of sjcs_query_count(ctx, q, idx[i]) for i = 0 .. k-1, added to
  * the query's accumulators.  Runs of up to 4 grid indexes with the same cell
- * grid (equal particle counts and radius hints give the same automatic grid),
- * under the static schedule, are counted in one pass: each halo's rows are
- * planned once and its counters flushed once for the whole run, and the
- * indexes' row loads overlap each other's tests.  Any other index is counted
- * on its own.  The reference's file loop (src/astr_rcount/main.c:676-826)
+ * grid (equal particle counts and radius hints give the same automatic grid)
+ * are counted in one call; tables counted warp by warp only under the static
+ * schedule.  Any other index is counted on its own.  The reference's file loop (src/astr_rcount/main.c:676-826)
  * counts one file at a time; this is the same sum over files with every
  * file's index resident at once. */
 int sjcs_query_count_many(sjcs_ctx *ctx, sjcs_query *q, const sjcs_index *const *idx, int k);

@@ -1,5 +1,5 @@
 // Periodic multi-shell count with one lane per halo, over grid indexes (whose
-// candidate ranges are rows of cells) and Morton indexes (single cells, their
+// candidate ranges are rows of cells) and Morton indexes (quads of cells, their
 // ranks from the offset table or the learned model).
 //
 // k_lane_count   32 halos of the Morton order per warp, one per lane.  A lane
@@ -47,8 +47,10 @@
 // 1e7 0.42 -> 0.20; 1e6 clustered halos on 3e7 clustered particles 9.2 (static
 // schedule) and 7.1 (queue) -> 3.43, one item at a time 4.28; 1e6 on 5e7, R =
 // 20, 64 shells 55 and 40.8 -> 18.5, one item at a time 24.3; 1e5 on 2e7, R =
-// 10 2.14 and 1.45 -> 0.75, one at a time 0.90.  Morton forms, 5e5 clustered
-// halos on 2e7 particles: offset table 4.87 -> 2.19, learned 4.65 (queue) -> 2.86.
+// 10 2.14 and 1.45 -> 0.75, one at a time 0.90.  Morton forms, 1e7 uniform
+// halos on 1e8 particles: offset table 14.2 -> 8.0, learned 25.3 -> 17.2; 5e5
+// clustered ones on 2e7: 4.87 -> 2.19 and 4.65 (queue) -> 2.86 by single cells,
+// quads a few per cent less.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -1,5 +1,6 @@
 // Warp-cooperative periodic multi-shell count over a Morton index (plain
-// Morton offset table or learned rank model).
+// Morton offset table or learned rank model), for the radius tables that the
+// lane-per-halo count (lane_count.cu) does not take.
 //
 // One warp owns one halo at a time.  For every periodic image the warp lists
 // the level-L Morton cells of the query box (lane k takes cell k of the box),

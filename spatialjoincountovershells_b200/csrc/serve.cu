@@ -126,8 +126,8 @@ int enqueue(sjcs_server* srv, Slot& sl) {
     if (rc) return rc;
     if (n) {
         std::lock_guard<std::mutex> lk(srv->ctx->mu);  // launch set-up and the tuned-schedule cache
-        // grid indexes of one cell grid under the static schedule: one fused
-        // pass (each halo planned once for all of them)
+        // grid indexes of one cell grid, counted by lanes or under the static
+        // schedule: one call for all of them
         const size_t k = srv->idx.size();
         bool fuse = k >= 2 && k <= (size_t)kMaxFusedIndexes;
         for (size_t i = 0; fuse && i < k; ++i) {

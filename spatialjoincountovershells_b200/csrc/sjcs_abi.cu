@@ -1208,8 +1208,8 @@ int sjcs_query_count_many(sjcs_ctx* ctx, sjcs_query* q, const sjcs_index* const*
     int rc = set_device(ctx);
     if (rc) return rc;
     // Fused: runs of up to kMaxFused grid indexes of one geometry under the
-    // static schedule (or counted by lanes, which ignores it) whose counts fit the accumulators together; anything
-    // else is counted index by index.
+    // static schedule, or counted by lanes, which ignore it, whose counts fit
+    // the accumulators together; anything else is counted index by index.
     for (int i = 0; i < k;) {
         int j = i + 1;
         const sjcs_index* a = idx[i];
