@@ -246,11 +246,19 @@ __global__ void k_judge(const LearnedLeaf* __restrict__ leaves, LearnedRoot* rt,
 
 }  // namespace
 
-int morton_auto_level(uint64_t n, float radius_hint) {
-    // about 4 or more particles per cell on average ...
+// Particles per cell, on average, from which the next level is taken.  A count
+// whose radius is known pays for the candidates of its cells: with the table
+// finer cells win down to one particle per cell (2e7 particles, R = 5, level 7
+// -> 8: clustered 1.91 -> 1.70 ms, uniform 0.84 -> 0.83; 6e7: 8.39 -> 6.88 and
+// 5.82 -> 2.05; 5e6, 6 -> 7: 0.65 -> 0.50 and 0.21 -> 0.09).  A learned lookup
+// costs more than a table read, so its cells are larger (6e7: 9.65 -> 8.88 and
+// 8.28 -> 4.35, but 3e7, 1.8 per cell: 2.56 -> 3.38 uniform).  Without a radius
+// to go by the cells hold four or more.
+int morton_auto_level(uint64_t n, float radius_hint, bool learned) {
+    const double per_cell = radius_hint > 0.0f ? (learned ? 2.4 : 1.0) : 4.0;
     int L = 1;
-    while (L < 9 && (1ull << (3 * (L + 1))) * 4ull <= n) ++L;
-    // ... and cells no smaller than 0.7 R, so a query box spans <= 4 cells per axis
+    while (L < 9 && (double)(1ull << (3 * (L + 1))) * per_cell <= (double)n) ++L;
+    // cells no smaller than 0.7 R, so a query box spans <= 4 cells per axis
     if (radius_hint > 0.0f)
         while (L > 1 && 1000.0 / (double)(1u << L) < 0.7 * (double)radius_hint) --L;
     return L;

@@ -469,7 +469,7 @@ int check_opts(const sjcs_index_opts* opts, sjcs_index_opts* o_out) {
 int enqueue_build(sjcs_ctx* ctx, sjcs_index* idx, const float* d_xyz, uint64_t n, const sjcs_index_opts& o,
                   cudaStream_t s) {
     if (o.kind != SJCS_INDEX_GRID) {
-        const int level = o.grid[0] ? (int)o.grid[0] : morton_auto_level(n, o.radius_hint);
+        const int level = o.grid[0] ? (int)o.grid[0] : morton_auto_level(n, o.radius_hint, o.kind == SJCS_INDEX_LEARNED);
         return build_morton_index(ctx, d_xyz, n, level, o.kind == SJCS_INDEX_LEARNED,
                                   (o.flags & SJCS_INDEX_VERIFY) != 0, idx, s);
     }

@@ -239,7 +239,7 @@ int build_grid_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, const GridGe
 GridGeom auto_grid(uint64_t n, float radius_hint, const uint32_t* grid_req);
 
 // learned_index.cu: Morton kinds (plain Morton offset table, learned rank model)
-int morton_auto_level(uint64_t n, float radius_hint);
+int morton_auto_level(uint64_t n, float radius_hint, bool learned);
 int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level, bool learned, bool verify,
                        sjcs_index* idx, cudaStream_t s);
 

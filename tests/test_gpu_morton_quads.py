@@ -47,3 +47,27 @@ def test_quads(ctx, kind, data, level, radius, halos, periodic):
     idx.destroy()
     q.destroy()
     assert np.array_equal(out, oracle.count(p, h, r2, periodic=periodic))
+
+
+@pytest.mark.parametrize("kind,per_cell", [(nat.INDEX_MORTON, 1.0), (nat.INDEX_LEARNED, 2.4)])
+@pytest.mark.parametrize("hint,below", [(5.0, 4), (40.0, 4), (60.0, 4), (0.0, 4)])
+def test_automatic_level(ctx, kind, per_cell, hint, below):
+    """The cells halve where the particles per cell allow it: one more or less
+    particle than that, radii that allow the finer cells (40) and that do not
+    (60: 0.7 R is more than 31.25), and no radius (four per cell)."""
+    want = per_cell if hint else 4.0
+    fine = below if hint == 60.0 else below + 1
+    edge = int(np.ceil(8 ** (below + 1) * want))
+    rng = np.random.default_rng(1300)
+    h = rng.uniform(0, 1000, (300, 3)).astype(np.float32)
+    r2 = nat.radius_table(0.5, hint or 25.0, 12)
+    for n, level in ((edge - 1, below), (edge, fine)):
+        p = rng.uniform(0, 1000, (n, 3)).astype(np.float32)
+        idx = ctx.build_index(p, radius_hint=hint, kind=kind)
+        q = ctx.query(h, r2)
+        q.count(idx)
+        out, got = q.read_counts(), idx.grid
+        idx.destroy()
+        q.destroy()
+        assert tuple(got) == (2**level,) * 3
+        assert np.array_equal(out, oracle.count(p, h, r2))
