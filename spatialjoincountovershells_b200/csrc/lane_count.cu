@@ -93,7 +93,10 @@ constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles 
 // rows of 40, where row by row and flattened meet.
 constexpr uint32_t kStepCost = 36, kItemCost = 370, kRowCost = 20, kRowCand = 9, kFlatCand = 22;
 constexpr uint32_t kMaxWalkRows = 400;  // rows of a box that lanes walk
-constexpr uint32_t kWalkMax = 30000;    // 16-bit counters (a chunked box's candidates are known up to a factor of two)
+// 16-bit counters and range lengths: a lane's candidates are at most this many,
+// or 8/5 of it in a chunked box, whose ranges are summed before the sphere
+// leaves out any of them.
+constexpr uint32_t kWalkMax = 30000;
 
 struct LaneParams {
     const uint32_t* __restrict__ slots;  // the fields of sjcs_query::LaneTable
@@ -449,21 +452,31 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                         if (PACK && r == 0u) first = lo[0];
                     }
                 } else if (cand) {
-                    // from the table; the model would answer the same
-                    for (int zz = im.z0; zz <= im.z1; ++zz)
-                        for (int yy = im.y0; yy <= im.y1; ++yy) {
-                            const uint32_t zy = (spread3_10((uint32_t)yy) << 1) | (spread3_10((uint32_t)zz) << 2);
-                            for (int xx = im.x0; xx <= im.x1; xx += 4) {
-                                uint2 r4[4];
+                    // What the quads' ranges hold, from the first cell of the box in a
+                    // quad to its last: cells between them that lie outside the box are
+                    // walked too.  From the table; the model would answer the same.
+                    int qx = 0, qy = 0, qz = 0;
+                    for (uint32_t r = 0; r < nranges; r += 4u) {
+                        uint2 r4[4];
 #pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    const uint32_t code = zy | spread3_10((uint32_t)(xx + u));
-                                    r4[u] = xx + u <= im.x1 ? table_range(cs, code, code + 1u) : make_uint2(0u, 0u);
+                        for (int u = 0; u < 4; ++u) {
+                            uint32_t a = 0u, e = 0u;
+                            if (r + u < nranges) {
+                                const int xx = 2 * ((im.x0 >> 1) + qx), yy = 2 * ((im.y0 >> 1) + qy);
+                                quad_cells(quad_mask(im, xx, yy), xx, yy, im.z0 + qz, &a, &e);
+                            }
+                            r4[u] = a != e ? table_range(cs, a, e) : make_uint2(0u, 0u);
+                            if (++qx > (im.x1 >> 1) - (im.x0 >> 1)) {
+                                qx = 0;
+                                if (++qy > (im.y1 >> 1) - (im.y0 >> 1)) {
+                                    qy = 0;
+                                    ++qz;
                                 }
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) box += r4[u].y - r4[u].x;
                             }
                         }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) box += r4[u].y - r4[u].x;
+                    }
                 } else if (valid & fin) {
                     box = q.huge + 1u;
                 }
