@@ -19,6 +19,11 @@
 //                one per lane and halo.  Two halos of one clump share nearly
 //                all candidates, so the loads and the row bookkeeping are
 //                paid once for both.
+// k_left_count   when the list had no room for all items: a warp takes the
+//                marked images of 64 halos one by one.  (Single lanes counting
+//                them in k_lane_count took 7.6 ms for 20000 uniform halos on
+//                1e6 particles at R = 100 and 66 ms for 10000 on 5e4 at R =
+//                600; 0.34 and 1.1 since.)
 //
 // A candidate costs one float4 load, the eight fp32 operations of the
 // reference's distance, one lookup and one counter update; the box test and
@@ -83,6 +88,7 @@ constexpr uint32_t kSpan = 1u << 20;  // candidates between two looks at what th
 // took 8 and 3 % longer on clustered data, R = 20).  When there are fewer
 // halos than a few per warp, items are split from kHugeFew on.
 constexpr uint32_t kHuge = 65536, kHugeFew = 2048;
+constexpr int kCtlLeft = 6;  // control word: something was marked in LaneParams::left; the next one, claims of it
 constexpr uint32_t kGallop = 15;  // first step of the search for a cell's end
 constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles on this path
 // Work in cycles of the data pipe, to decide which lanes are listed and how: a
@@ -109,7 +115,8 @@ struct LaneParams {
     // Items: the huge ones from the front of the list, the others from its end.
     uint2* __restrict__ list;  // (halo, flags)
     uint32_t cap;
-    uint32_t* __restrict__ ctl;  // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase
+    uint32_t* __restrict__ ctl;   // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase, kCtlLeft
+    uint32_t* __restrict__ left;  // marks of what did not fit the list (null: the list holds every item)
     // learned index: its model (leaves null: the other kinds)
     const LearnedLeaf* __restrict__ leaves;
     const LearnedRoot* __restrict__ root;
@@ -264,6 +271,11 @@ __device__ __forceinline__ float shifted(float v, float half) {
     return (__fsub_rn(v, half) < kBoxLow) ? __fadd_rn(v, kBoxUpp) : __fsub_rn(v, kBoxUpp);
 }
 
+// A centre for which safe2 is not proved.
+__device__ __forceinline__ bool beyond(const LaneParams& q, const float4 c) {
+    return !(fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)) <= q.cmax);
+}
+
 // Axes on which the halo's box crosses a face.
 __device__ __forceinline__ uint32_t oob_flags(const CountParams& p, const float4 c) {
     return ((__fsub_rn(c.x, p.half) < kBoxLow) | (__fadd_rn(c.x, p.half) > kBoxUpp) ? 1u : 0u) |
@@ -271,47 +283,22 @@ __device__ __forceinline__ uint32_t oob_flags(const CountParams& p, const float4
            ((__fsub_rn(c.z, p.half) < kBoxLow) | (__fadd_rn(c.z, p.half) > kBoxUpp) ? 4u : 0u);
 }
 
-// One lane counts one image by itself, straight into the count row: the way
-// out when the item list is full.
-template <int R>
-__device__ __noinline__ void serial_count(const CountParams& p, float4 c, uint32_t flags, float safe2) {
-    const Image im = make_image(p, c.x, c.y, c.z);
-    uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
-    const uint32_t f = (flags >> 3) & 3u;
-    auto test = [&](uint32_t j0, uint32_t e) {
-        for (uint32_t j = j0; j < e; ++j) {
-            const float4 v = p.mpts[f][j];
-            if (flags & kItemZone)
-                test_candidate<BIN_BSEARCH, true, true>(p, im, v, true, row, p.r2, p.lut, safe2);
-            else
-                test_candidate<BIN_BSEARCH, true>(p, im, v, true, row, p.r2, p.lut);
-        }
-    };
-    for (int zz = im.z0; zz <= im.z1; ++zz)
-        for (int yy = im.y0; yy <= im.y1; ++yy) {
-            if (R == RANGE_ROWS) {
-                const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
-                test(p.mcs[f][rc + im.x0], p.mcs[f][rc + im.x1 + 1]);
-            } else {
-                for (int xx = im.x0; xx <= im.x1; ++xx) {
-                    const uint32_t code = morton_cell((uint32_t)xx, (uint32_t)yy, (uint32_t)zz);
-                    test(p.mcs[f][code], p.mcs[f][code + 1u]);
-                }
-            }
-        }
-}
-
-// Lanes with `push` add an item (h, flags) to the list; c is its centre.
-template <int R>
-__device__ __forceinline__ void push_items(const CountParams& p, const LaneParams& q, bool push, bool huge, uint32_t h,
-                                           uint32_t flags, float4 c, int lane) {
+// Lanes with `push` add an item (h, flags) to the list.  What a full list does
+// not take is marked in `left` instead: 16 bits per index and halo, one per
+// image of the halo and one per image of which only the zone is wanted;
+// k_left_count takes those.  Out of line: inlined at its four uses it left the
+// walk 96 registers instead of 106 and the kernel slower (5.6 ms instead of 4.0
+// for 1e7 halos on 1e8 particles).
+__device__ __noinline__ void push_items(const CountParams& p, const LaneParams& q, bool push, bool huge, uint32_t h,
+                                           uint32_t flags, int lane) {
     const uint32_t all = __ballot_sync(0xffffffffu, push);
     if (!all) return;
     const uint32_t lt = (1u << lane) - 1u;
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(q.ctl, (uint32_t)__popc(all));
+    uint32_t base = q.cap;
+    // a full list is not counted on: no wrap, however many items come
+    if (lane == 0 && *const_cast<volatile uint32_t*>(q.ctl) < q.cap) base = atomicAdd(q.ctl, (uint32_t)__popc(all));
     base = __shfl_sync(0xffffffffu, base, 0);
-    const bool fits = push && base + (uint32_t)__popc(all & lt) < q.cap;
+    const bool fits = push && base < q.cap && (uint32_t)__popc(all & lt) < q.cap - base;
     const uint32_t hb = __ballot_sync(0xffffffffu, fits && huge), ob = __ballot_sync(0xffffffffu, fits && !huge);
     uint32_t at = 0;
     if (lane < 2) {
@@ -322,8 +309,12 @@ __device__ __forceinline__ void push_items(const CountParams& p, const LaneParam
     if (fits) {
         const uint32_t i = huge ? ah + (uint32_t)__popc(hb & lt) : q.cap - 1u - (ao + (uint32_t)__popc(ob & lt));
         q.list[i] = make_uint2(h, flags);
+    } else if (push && q.left) {
+        const uint64_t at16 = (uint64_t)((flags >> 3) & 3u) * p.nhalos + h;
+        const uint32_t bit = (flags & 7u) + ((flags & kItemZone) ? 8u : 0u);
+        atomicOr(q.left + (at16 >> 1), 1u << (bit + 16u * (uint32_t)(at16 & 1u)));
+        q.ctl[kCtlLeft] = 1u;
     }
-    if (push && !fits) serial_count<R>(p, c, flags, q.safe2);
 }
 
 template <int R, bool PACK>
@@ -391,11 +382,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                             if (T) rows->pend[npend + __popc(bal & lt)] = h | (T << 29);
                             npend += __popc(bal);
                         } else {
-                            float4 ci = c;
-                            if (T & 1u) ci.x = shifted(c.x, p.half);
-                            if (T & 2u) ci.y = shifted(c.y, p.half);
-                            if (T & 4u) ci.z = shifted(c.z, p.half);
-                            push_items<R>(p, q, T != 0u, false, h, T | file, ci, lane);
+                            push_items(p, q, T != 0u, false, h, T | file, lane);
                         }
                         T = T ? (T - 1u) & F : 0u;
                     }
@@ -406,7 +393,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
             }
             // a centre that is not finite has no finite distance: nothing to count
             const bool fin = (c.x - c.x == 0.0f) & (c.y - c.y == 0.0f) & (c.z - c.z == 0.0f);
-            const bool far = !(fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z)) <= q.cmax);
+            const bool far = beyond(q, c);
             const Image im = make_image(p, c.x, c.y, c.z);
             const uint32_t nranges = box_ranges<R>(im);
             const bool cand = valid & fin & !far & (R != RANGE_ROWS || im.ny <= LN_ROWS) & (nranges <= kMaxWalkRows);
@@ -501,8 +488,8 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     }
                     mine &= est <= tau;
                 }
-                push_items<R>(p, q, valid & fin & !mine, box > q.huge, h,
-                           file | S | (far ? kItemFar : 0u) | (short_rows(est, rows_est) ? kItemShort : 0u), c, lane);
+                push_items(p, q, valid & fin & !mine, box > q.huge, h,
+                           file | S | (far ? kItemFar : 0u) | (short_rows(est, rows_est) ? kItemShort : 0u), lane);
             }
             const int ny = mine ? im.ny : 0, nz = mine ? im.nz : 0;
             const int nymax = __reduce_max_sync(0xffffffffu, ny), nzmax = __reduce_max_sync(0xffffffffu, nz);
@@ -640,7 +627,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     }
                     coop |= T > tau;
                 }
-                if (__any_sync(0xffffffffu, coop)) push_items<R>(p, q, coop, T > q.huge, h, file | S | (short_rows(T, m) ? kItemShort : 0u), c, lane);
+                if (__any_sync(0xffffffffu, coop)) push_items(p, q, coop, T > q.huge, h, file | S | (short_rows(T, m) ? kItemShort : 0u), lane);
                 if (steps) {
                     uint32_t j, e;
                     float4 buf[LN_DEPTH];
@@ -719,7 +706,7 @@ k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ Lane
                     walked = true;
                 }
             }
-            if (__any_sync(0xffffffffu, z < q.zone)) push_items<R>(p, q, z < q.zone, false, h, file | S | kItemZone, c, lane);
+            if (__any_sync(0xffffffffu, z < q.zone)) push_items(p, q, z < q.zone, false, h, file | S | kItemZone, lane);
             // the lanes' counters to their halos' rows
             if (walked) {
                 uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
@@ -1124,6 +1111,43 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
     }
 }
 
+// What the full list left: a warp claims the marks of 64 halos and counts the
+// images one after the other.
+template <int R>
+__global__ void __launch_bounds__(HV_THREADS, HV_BLOCKS)
+k_left_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
+    extern __shared__ uint32_t smem[];
+    if (q.ctl[kCtlLeft] == 0u) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int colwords = (q.ncol + 1) * 16;
+    uint32_t* slots = smem + HV_WARPS * colwords;
+    uint32_t* cols = smem + warp * colwords;
+    for (int i = tid; i < q.nslots; i += HV_THREADS) slots[i] = q.slots[i];
+    for (int i = lane; i < colwords; i += 32) cols[i] = 0u;
+    __syncthreads();
+    const uint64_t words = (p.nhalos * (uint64_t)p.nidx + 1u) / 2u;
+    for (;;) {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(q.ctl + kCtlLeft + 1, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        const uint64_t w0 = (uint64_t)i * 32u;
+        if (w0 >= words) break;
+        const uint32_t mine = w0 + lane < words ? q.left[w0 + lane] : 0u;
+        uint32_t any = __ballot_sync(0xffffffffu, mine != 0u);
+        for (; any; any &= any - 1u) {
+            const int j = __ffs((int)any) - 1;
+            for (uint32_t m = __shfl_sync(0xffffffffu, mine, j); m; m &= m - 1u) {
+                const uint32_t b = (uint32_t)__ffs((int)m) - 1u;
+                const uint64_t at16 = 2u * (w0 + (uint32_t)j) + (b >> 4), f = at16 / p.nhalos;
+                const uint2 it = make_uint2((uint32_t)(at16 - f * p.nhalos),
+                                            (b & 7u) | ((uint32_t)f << 3) | ((b & 8u) ? kItemZone : 0u));
+                if ((b & 8u) || beyond(q, item_centre(p, it))) count_literal<R>(p, q, it, 0u, 1u, lane);
+                else count_items<R, 1, true>(p, q, &it, 0u, 1u, cols, slots, lane);
+            }
+        }
+    }
+}
+
 }  // namespace
 
 bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
@@ -1133,9 +1157,41 @@ bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
     return true;
 }
 
-uint64_t lane_list_items(uint64_t nhalos, int nidx) { return (uint64_t)nidx * (nhalos + nhalos / 2 + 1024); }
-
 namespace {
+// The list takes 1.5 items per halo and index.  An image is one item at most:
+// lists of up to kExactItems (16 MB), and those of counts without images, have
+// room for all of them and nothing is ever left (marks and an idle k_left_count
+// cost about 5 us).
+constexpr uint64_t kExactItems = 1u << 21;
+
+// List, control words and marks of a count on stream s.  A pool that cannot
+// give the whole list gives a shorter one, down to none.
+int alloc_list(StreamScratch& scr, const CountParams& p, LaneParams* q, cudaStream_t s) {
+    const uint64_t n = p.nhalos * (uint64_t)p.nidx;
+    uint64_t cap = n * (p.periodic ? 8u : 1u), marks = 0;
+    auto not_all = [&] {
+        cap = std::min<uint64_t>(n + n / 2 + 1024, 0xf0000000ull);
+        marks = (n + 1) / 2;
+    };
+    if (cap > std::max(kExactItems, n + n / 2 + 1024) || cap > 0xf0000000ull) not_all();
+    uint32_t* ctl = nullptr;
+    for (;;) {
+        const cudaError_t e =
+            scr.alloc(&ctl, (kLaneCtlWords + marks + (marks & 1u)) * sizeof(uint32_t) + cap * sizeof(uint2));
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation || cap == 0) SJCS_CUDA_TRY(e);
+        cudaGetLastError();
+        if (!marks) not_all();
+        cap = cap > 4096 ? cap / 4 : 0;
+    }
+    SJCS_CUDA_TRY(cudaMemsetAsync(ctl, 0, (kLaneCtlWords + marks) * sizeof(uint32_t), s));
+    q->ctl = ctl;
+    q->left = marks ? ctl + kLaneCtlWords : nullptr;
+    q->list = reinterpret_cast<uint2*>(ctl + kLaneCtlWords + marks + (marks & 1u));
+    q->cap = (uint32_t)cap;
+    return SJCS_OK;
+}
+
 template <int R, bool PACK>
 int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
                   const LaneModel* model) {
@@ -1165,12 +1221,8 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
         q.list = given->list;
         q.cap = given->cap;
     } else {
-        q.cap = (uint32_t)std::min<uint64_t>(lane_list_items(p.nhalos, p.nidx), 0xffffffffull);
-        uint32_t* ctl = nullptr;
-        SJCS_CUDA_TRY(scr.alloc(&ctl, kLaneCtlWords * sizeof(uint32_t) + (uint64_t)q.cap * sizeof(uint2)));
-        SJCS_CUDA_TRY(cudaMemsetAsync(ctl, 0, kLaneCtlWords * sizeof(uint32_t), s));
-        q.ctl = ctl;
-        q.list = reinterpret_cast<uint2*>(ctl + kLaneCtlWords);
+        const int rc = alloc_list(scr, p, &q, s);
+        if (rc) return rc;
     }
     // one block per SM (neighbouring batches share its L1); blocks of fewer
     // warps when there are not enough batches for every SM
@@ -1207,6 +1259,11 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     if (per_sm < 1) per_sm = 1;
     listed<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
+    if (q.left) {
+        SJCS_CUDA_TRY(cudaFuncSetAttribute(k_left_count<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+        k_left_count<R><<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
+        SJCS_LAUNCH_CHECK();
+    }
     return SJCS_OK;
 }
 }  // namespace

@@ -9,14 +9,13 @@ namespace sjcs {
 // this size (any schedule: the counts are the same).
 bool lane_count_applies(const sjcs_query* q, const count::CountParams& p);
 // Item list of a count, when the caller provides it: kLaneCtlWords zeroed
-// control words and room for cap items (lane_list_items).
+// control words and room for cap items, eight per halo (one per image) or more.
 constexpr int kLaneCtlWords = 8;
 struct LaneScratch {
     uint32_t* ctl;
     uint2* list;
     uint32_t cap;
 };
-uint64_t lane_list_items(uint64_t nhalos, int nidx);
 // Count q against the p.nidx indexes of p (mpts, mcs, mn) on stream s.
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, cudaStream_t s,
                       const LaneScratch* given = nullptr);

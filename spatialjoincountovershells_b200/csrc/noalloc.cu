@@ -41,7 +41,7 @@ constexpr int kMaxTable = 640;  // lane slots that travel with the launch (param
 
 constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 // byte offsets of the sub-buffers (each 256-byte aligned)
-constexpr uint32_t kListItems = (uint32_t)(kNH + kNH / 2 + 1024);  // lane_list_items(kNH, 1)
+constexpr uint32_t kListItems = (uint32_t)(8 * kNH);  // every image of every halo
 constexpr uint64_t kOffPts = 0;
 constexpr uint64_t kOffCells = align256(kOffPts + kNP * 16);
 constexpr uint64_t kOffTmp = align256(kOffCells + (kNC + 1) * 4);

@@ -104,7 +104,7 @@ bool valid_server(const sjcs_server* s) { return s && s->magic == kServerMagic; 
 uint64_t request_bytes(uint64_t nhalos, size_t stride, int nrads) {
     // per halo: raw halo + ordered halo + counts, and 53 bytes of scratch: its
     // rank and share of the bucket counters (6 B) and the count's item list
-    // (12 B per index of a fused pass, up to 4), or the queue schedule's keys
+    // (14 B per index of a fused pass, up to 4; small ones up to 16 MB), or the queue schedule's keys
     // and order (13 B); fixed: radius and lookup tables, scan partials
     return nhalos * (uint64_t)(stride + 16 + 40 + 4 * (uint64_t)nrads + 13) + 65536 + 8 * (uint64_t)nrads;
 }

@@ -146,3 +146,20 @@ def test_morton_full_list_and_odd_values(ctx, kind):
     h[:5] = [[np.nan, 5, 5], [np.inf, 5, 5], [-40, 1190, 2], [5000, 5, 5], [1e30, 1, 1]]
     r2 = nat.radius_table(0.5, 30.0, 20)
     assert np.array_equal(_count(ctx, [p], h, r2, kind=kind, level=6), _want([p], h, r2))
+
+
+@pytest.mark.parametrize("kind,grid", [(nat.INDEX_GRID, (50, 20, 20)), (nat.INDEX_GRID, (100, 100, 100)),
+                                       (nat.INDEX_MORTON, None), (nat.INDEX_LEARNED, None)])
+@pytest.mark.parametrize("files,odd", [(1, 0), (3, 1)])
+def test_more_items_than_the_list_holds(ctx, kind, grid, files, odd):
+    """270000 halos in a corner, eight images each: with 1.5 items of room per
+    halo most images are left to the count after the list.  Halos and particles
+    outside the box among them (their images take the literal test)."""
+    rng = np.random.default_rng(995)
+    ps = [(rng.normal(0, 30, (900 + 7 * f, 3)) % 1000.0).astype(np.float32) for f in range(files)]
+    h = (rng.normal(0, 6, (270000 + odd, 3)) % 1000.0).astype(np.float32)
+    h[:400] = rng.normal(2100, 20, (400, 3)).astype(np.float32)
+    ps[0][:100] = rng.normal(1100, 20, (100, 3)).astype(np.float32)
+    r2 = nat.radius_table(0.5, 30.0, 9)
+    level = 0 if grid else 7
+    assert np.array_equal(_count(ctx, ps, h, r2, grid=grid, kind=kind, level=level), _want(ps, h, r2))
