@@ -43,6 +43,16 @@ struct CountParams {
     uint32_t mn[kMaxFused];  // particles of each index
 };
 
+// Lets kern use all the shared memory a block can have.  The limit belongs to
+// the function on its device, not to a launch: every call sets the same value,
+// so that host threads with contexts of their own cannot lower it between
+// another's setting and launch.  Not for kernels with static shared memory.
+constexpr size_t kMaxBlockSmem = 227 * 1024;
+template <class Kernel>
+inline cudaError_t allow_block_smem(Kernel kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxBlockSmem);
+}
+
 // CountParams::reach: with pruning, a bound above the square root of r2p plus
 // the rounding of the differences; else no bound.
 inline float reach_of(float r2max, bool prune) {

@@ -1228,8 +1228,7 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     // warps when there are not enough batches for every SM
     const uint64_t nbatch = (p.nhalos + 31) / 32;
     const size_t warp_a = sizeof(LaneRows<PACK>) + (size_t)(L.ncol + 1) * 64, table = (size_t)L.nslots * 4;
-    constexpr size_t kMaxSmem = 227 * 1024;
-    const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxSmem - table) / warp_a);  // >= 15 for any table
+    const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxBlockSmem - table) / warp_a);  // >= 15 for any table
     const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + (uint64_t)ctx->num_sms - 1) / (uint64_t)ctx->num_sms);
     const size_t smem_a = nw * warp_a + table;
     // A batch lasts as long as its longest lane: with few batches per SM long
@@ -1246,7 +1245,7 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     const uint64_t per = R == RANGE_ROWS ? 8 : 10;
     q.walk_max = (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(floor, nbatch * per / (uint64_t)ctx->num_sms));
     const size_t smem_b = HV_WARPS * 2 * (size_t)(L.ncol + 1) * 64 + (size_t)L.nslots * 4;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(k_lane_count<R, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    SJCS_CUDA_TRY(allow_block_smem(k_lane_count<R, PACK>));
     const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
     k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
@@ -1254,13 +1253,13 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     auto listed = k_listed_count<R, HV_BLOCKS>;
     if constexpr (R == RANGE_ROWS)
         if (given) listed = k_listed_count<R, HV_BLOCKS_NOALLOC>;
-    SJCS_CUDA_TRY(cudaFuncSetAttribute(listed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+    SJCS_CUDA_TRY(allow_block_smem(listed));
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, listed, HV_THREADS, smem_b));
     if (per_sm < 1) per_sm = 1;
     listed<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
     if (q.left) {
-        SJCS_CUDA_TRY(cudaFuncSetAttribute(k_left_count<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+        SJCS_CUDA_TRY(allow_block_smem(k_left_count<R>));
         k_left_count<R><<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
         SJCS_LAUNCH_CHECK();
     }

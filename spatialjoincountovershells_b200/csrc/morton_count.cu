@@ -346,8 +346,7 @@ __global__ void __launch_bounds__(MC_THREADS, 8) k_morton_count_queue(CountParam
 template <int LOOK, int BIN, bool BIG>
 int launch_m(sjcs_ctx* ctx, const CountParams& p, const MortonParams& m, size_t smem, cudaStream_t s) {
     auto kern = k_morton_count<LOOK, BIN, BIG>;
-    if (smem > 48 * 1024)
-        SJCS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MC_THREADS, smem));
     if (per_sm < 1) per_sm = 1;
@@ -378,8 +377,7 @@ int launch_mq(sjcs_ctx* ctx, const CountParams& p, const MortonParams& m, const 
     int rc = order_and_plan(n, key, hist, sc, ord, plan, ctl, rhist, s);
     if (rc) return rc;
     auto kern = k_morton_count_queue<LOOK, BIN, BIG>;
-    if (smem > 48 * 1024)
-        SJCS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MC_THREADS, smem));
     if (per_sm < 1) per_sm = 1;

@@ -489,8 +489,7 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_queue(CountParams
 template <int BIN, bool BIG>
 int launch_variant(sjcs_ctx* ctx, const CountParams& p, size_t smem, cudaStream_t s, bool multi = false) {
     auto kern = multi ? k_shell_count_multi<BIN, BIG> : k_shell_count<BIN, BIG>;
-    if (smem > 48 * 1024)
-        SJCS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CT_THREADS, smem));
     if (per_sm < 1) per_sm = 1;
@@ -521,8 +520,7 @@ int launch_queue(sjcs_ctx* ctx, const CountParams& p, const Schedule& sc, size_t
     int rc = order_and_plan(n, key, hist, sc, ord, plan, ctl, rhist, s);
     if (rc) return rc;
     auto kern = k_shell_count_queue<BIN, BIG>;
-    if (smem > 48 * 1024)
-        SJCS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CT_THREADS, smem));
     if (per_sm < 1) per_sm = 1;
