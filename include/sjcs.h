@@ -65,8 +65,9 @@ extern "C" {
 
 /* count schedules: how the count kernel hands halos to warps.  Tables of up to
  * 128 increasing, positive, finite squared radii that are not too close to one
- * another are counted with a lane per halo, whichever schedule is set: halos
- * too heavy for a lane go to a list, the heaviest are split there.  Other
+ * another are counted with a lane per halo, or a warp per halo when there are
+ * few, whichever schedule is set: halos too heavy for that go to a list, the
+ * heaviest are split there.  Other
  * tables are counted warp by warp, as the schedule says. */
 #define SJCS_SCHED_AUTO    0 /* the context's autotuned choice for this workload shape, else STATIC */
 #define SJCS_SCHED_STATIC  1 /* warps take halos strided over the Morton order, in batches of 32 */

@@ -41,7 +41,55 @@ struct CountParams {
     const float4* mpts[kMaxFused];
     const uint32_t* mcs[kMaxFused];
     uint32_t mn[kMaxFused];  // particles of each index
+    // Images of more than `heavy` candidates go to a list instead (LIST
+    // variants of the kernels) for k_listed_count, which splits those of more
+    // than `huge` over several warps.
+    uint32_t heavy, huge;
+    uint32_t list_cap, list_huge;  // room, and the part of it for huge ones
+    uint32_t* list_ctl;            // [1] huge ones, from the front, [2] others, from the end
+    uint32_t* list_clear;  // control words to clear for the next count, or null
+    uint2* list;
 };
+
+// Item of a list of images: the halo's place, and bits 0-2 the shifted axes,
+// bits 3-4 the index, from kItemFrom on the first 32 ranges still to count.
+constexpr uint32_t kItemShort = 1u << 9;  // short rows: flattened before they are read
+constexpr int kItemFrom = 10;
+constexpr uint32_t kItemFromMax = 1u << 22;
+constexpr int kListWords = 8;  // control words of a list
+
+// The control words that the next count of the query will use (its counts take
+// turns with two sets, so none needs a launch to clear its own).
+__device__ __forceinline__ void clear_next_list(const CountParams& p) {
+    if (p.list_clear && blockIdx.x == 0 && threadIdx.x < kListWords) p.list_clear[threadIdx.x] = 0u;
+}
+
+// Cycles of the data pipe that reading a listed item costs for one of its rows
+// and for a candidate, in 1/32 cycles, when rows are read one by one and when
+// they are flattened first (see lane_count.cu).
+constexpr uint32_t kRowCost = 20, kRowCand = 9, kFlatCand = 22;
+__device__ __forceinline__ bool short_rows(uint32_t T, uint32_t rows) {
+    return ((kFlatCand - kRowCand) * T >> 5) < kRowCost * rows;
+}
+
+// Puts a warp's image of T candidates in `rows` ranges on the list; false: no
+// room.
+__device__ __forceinline__ bool list_image(const CountParams& p, uint2 it, uint32_t T, uint32_t rows, int lane) {
+    bool fits = false;
+    if (lane == 0) {
+        const bool huge = T > p.huge;
+        uint32_t* n = p.list_ctl + (huge ? 1 : 2);
+        const uint32_t room = huge ? p.list_huge : p.list_cap - p.list_huge;
+        // a full part is not counted on: no wrap, however many items come
+        if (*const_cast<volatile uint32_t*>(n) < room) {
+            const uint32_t i = atomicAdd(n, 1u);
+            fits = i < room;
+            if (short_rows(min(T, 1u << 24), rows)) it.y |= kItemShort;
+            if (fits) p.list[huge ? i : p.list_cap - 1u - i] = it;
+        }
+    }
+    return __shfl_sync(0xffffffffu, fits, 0);
+}
 
 // Lets kern use all the shared memory a block can have.  The limit belongs to
 // the function on its device, not to a launch: every call sets the same value,
@@ -147,10 +195,14 @@ __device__ __forceinline__ void test_candidate(const CountParams& p, const Image
 
 // Scan the lanes' row lengths and test every candidate of those rows,
 // two windows of 32 candidates per iteration so two loads are in flight.
-template <int BIN, bool BIG>
-__device__ __forceinline__ void run_rows(const CountParams& p, const Image& im, uint32_t start, uint32_t end,
-                                         uint32_t* __restrict__ sink, const float* __restrict__ tab,
-                                         const uint32_t* __restrict__ lut, int lane) {
+// LIST: rows of more than `most` candidates are left to the list as item it;
+// returns the candidates counted, or kListed.
+constexpr uint32_t kListed = 0xffffffffu;
+template <int BIN, bool BIG, bool LIST = false>
+__device__ __forceinline__ uint32_t run_rows(const CountParams& p, const Image& im, uint32_t start, uint32_t end,
+                                             uint32_t* __restrict__ sink, const float* __restrict__ tab,
+                                             const uint32_t* __restrict__ lut, int lane, uint32_t most = 0,
+                                             uint2 it = make_uint2(0u, 0u)) {
     const uint32_t len = end - start;
     uint32_t incl = len;
 #pragma unroll
@@ -159,6 +211,10 @@ __device__ __forceinline__ void run_rows(const CountParams& p, const Image& im, 
         if (lane >= o) incl += v;
     }
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if constexpr (LIST)
+        if (total > most &&
+            list_image(p, it, total, (uint32_t)__popc(__ballot_sync(0xffffffffu, len != 0u)), lane))
+            return kListed;
     const uint32_t off = start - (incl - len);  // slot = t + off for t inside this row (mod 2^32)
     for (uint32_t wb = 0; wb < total; wb += 64) {
         const uint32_t t0 = wb + (uint32_t)lane, t1 = t0 + 32u;
@@ -179,6 +235,7 @@ __device__ __forceinline__ void run_rows(const CountParams& p, const Image& im, 
         test_candidate<BIN, BIG>(p, im, p0, l0, sink, tab, lut);
         test_candidate<BIN, BIG>(p, im, p1, l1, sink, tab, lut);
     }
+    return total;
 }
 
 // Piece `part` of `nparts` of the candidates of the lanes' rows: the

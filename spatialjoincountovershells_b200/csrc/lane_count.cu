@@ -1,18 +1,21 @@
 // Periodic multi-shell count with one lane per halo, over grid indexes (whose
 // candidate ranges are rows of cells) and Morton indexes (quads of cells, their
-// ranks from the offset table or the learned model).
+// ranks from the offset table or the learned model); for more than five batches
+// of 32 halos per SM.  With fewer a warp takes a halo (shell_count.cu,
+// morton_count.cu) and only the list is counted here.
 //
 // k_lane_count   32 halos of the Morton order per warp, one per lane.  A lane
-//                plans its box's rows of cells (at most 5 x 5), clips each in x
-//                to the sphere, fetches the rows' slot ranges and then walks
-//                its own candidates one by one; its counts go to a private
+//                plans its box's rows of cells, up to 25 at a time, clips each
+//                in x to the sphere, fetches the rows' slot ranges and then
+//                walks its own candidates one by one; its counts go to a private
 //                column of 16-bit counters in shared memory and
 //                from there to the halo's row.  Shifted periodic images wait
 //                in a per-warp list until there are 32 of them and are then
 //                walked the same way.
-// k_listed_count what does not suit a lane: images of more than 25 rows, and
+// k_listed_count what does not suit a lane: images of more than 400 rows, and
 //                lanes with so many candidates that the rest of the warp
-//                would wait.  k_lane_count lists them; here a warp takes two
+//                would wait.  k_lane_count (or the kernels that give a warp to
+//                each halo) lists them; here a warp takes two
 //                neighbouring items (or a part of them), reads the rows that
 //                reach either sphere in windows of 32 slots, tests a loaded
 //                candidate against both centres and counts in 16-bit columns,
@@ -97,7 +100,7 @@ constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles 
 // one and when they are flattened first.  Fitted to 9e5 halos of about 550
 // candidates in rows of 8 (2.5 ms walked, 5 flattened, 8 row by row) and to
 // rows of 40, where row by row and flattened meet.
-constexpr uint32_t kStepCost = 36, kItemCost = 370, kRowCost = 20, kRowCand = 9, kFlatCand = 22;
+constexpr uint32_t kStepCost = 36, kItemCost = 370;  // and those of count_common.cuh
 constexpr uint32_t kMaxWalkRows = 400;  // rows of a box that lanes walk
 // 16-bit counters and range lengths: a lane's candidates are at most this many,
 // or 8/5 of it in a chunked box, whose ranges are summed before the sphere
@@ -114,7 +117,7 @@ struct LaneParams {
     uint32_t zone0, zone;  // bit pattern of safe2; that of r2max less it
     // Items: the huge ones from the front of the list, the others from its end.
     uint2* __restrict__ list;  // (halo, flags)
-    uint32_t cap;
+    uint32_t cap, cap_huge, cap_other;  // its room, and that of either kind
     uint32_t* __restrict__ ctl;   // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase, kCtlLeft
     uint32_t* __restrict__ left;  // marks of what did not fit the list (null: the list holds every item)
     // learned index: its model (leaves null: the other kinds)
@@ -123,6 +126,14 @@ struct LaneParams {
     const uint32_t* __restrict__ wpref;  // &pts[0].w (stride 4 words)
     int key_shift;                       // cell code -> first key of the cell
 };
+
+// Up to this many batches of 32 halos per SM a warp takes a halo at a time:
+// lanes would plan for a few warps only and leave most of it to the list.  Count
+// alone, lanes -> warps: 5000 uniform halos on 1e6 particles at R = 5 37 -> 30
+// us, 20000 on 1e7 at R = 10 92 -> 62, 10500 clustered ones on 5e6 at R = 7 140
+// -> 113; learned index, 1500 on 1e6 77 -> 30.  35000 halos on 5e6, R = 7:
+// uniform 62 -> 55, clustered 151 -> 152; on 1e7, R = 10 98 -> 77 and 283 -> 325.
+constexpr uint64_t kFewBatches = 5;
 
 // What a candidate range is: a row of grid cells clipped in x; or four Morton
 // cells that follow each other in the curve (x and y even and the next ones),
@@ -241,11 +252,7 @@ __device__ __forceinline__ void quad_cells(uint32_t mask, int x, int y, int z, u
 // An item's flags: bits 0-2 the shifted axes, bits 3-4 the index to count.
 constexpr uint32_t kItemZone = 1u << 7;  // only distances from safe2 on
 constexpr uint32_t kItemFar = 1u << 8;   // centre beyond cmax: literal test throughout
-constexpr uint32_t kItemShort = 1u << 9; // short rows: flattened before they are read
 
-__device__ __forceinline__ bool short_rows(uint32_t T, uint32_t rows) {
-    return ((kFlatCand - kRowCand) * T >> 5) < kRowCost * rows;
-}
 __device__ __forceinline__ uint32_t listed_cost(uint32_t T, uint32_t rows, uint32_t box_rows) {
     return min(kFlatCand * T >> 5, (kRowCand * T >> 5) + kRowCost * rows) + kItemCost * ((box_rows + 31u) >> 5);
 }
@@ -864,11 +871,11 @@ __device__ __noinline__ void count_literal(const CountParams& p, const LaneParam
 
 // Part `part` of `nparts` of H listed items of one index, counted together:
 // the rows are those that reach any of the H spheres, and a candidate once
-// loaded is tested against every centre.
+// loaded is tested against every centre.  Starts with the box's range rb.
 template <int R, int H, bool SHORT>
 __device__ __forceinline__ void count_items(const CountParams& p, const LaneParams& q, const uint2* it, uint32_t part,
                                             uint32_t nparts, uint32_t* __restrict__ cols,
-                                            const uint32_t* __restrict__ slots, int lane) {
+                                            const uint32_t* __restrict__ slots, int lane, uint32_t rb = 0) {
     float4 c[H];
     Image im;
 #pragma unroll
@@ -898,7 +905,7 @@ __device__ __forceinline__ void count_items(const CountParams& p, const LanePara
     const uint32_t one = (lane & 1) ? 65536u : 1u;
     uint32_t held = 0;  // bound of any 16-bit counter
     const uint32_t nranges = box_ranges<R>(im);
-    for (uint32_t rb = 0; rb < nranges; rb += 32u) {
+    for (; rb < nranges; rb += 32u) {
         const uint2 range = lane_range<R, H>(p, q, cs, im, c, rb + (uint32_t)lane, nranges);
         const uint32_t a = range.x, e = range.y;
         // this warp's share of the rows' candidates, [tb, te) of the flattened sequence
@@ -1044,7 +1051,7 @@ __device__ __forceinline__ void count_items(const CountParams& p, const LanePara
 // centres of one index no further apart than a radius: most candidates then
 // serve both.
 __device__ __forceinline__ bool paired(const CountParams& p, const uint2* it, uint32_t n) {
-    constexpr uint32_t kAlone = kItemZone | kItemFar | kItemShort;
+    constexpr uint32_t kAlone = kItemZone | kItemFar | kItemShort | ~((1u << kItemFrom) - 1u);
     if (n < 2u || ((it[0].y | it[1].y) & kAlone) || (((it[0].y ^ it[1].y) >> 3) & 3u)) return false;
     const float4 a = item_centre(p, it[0]), b = item_centre(p, it[1]);
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
@@ -1055,7 +1062,7 @@ template <int R, int BLOCKS>
 __global__ void __launch_bounds__(HV_THREADS, BLOCKS)
 k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
-    const uint32_t nhuge = min(q.ctl[1], q.cap), nother = min(q.ctl[2], q.cap);
+    const uint32_t nhuge = min(q.ctl[1], q.cap_huge), nother = min(q.ctl[2], q.cap_other);
     if (nhuge + nother == 0u) return;
     // Warps claim (two items, part); only huge items have several parts.  With
     // fewer items than warps each is claimed alone, and blocks beyond the last
@@ -1097,7 +1104,7 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
                 for (uint32_t j = 0; j < n; ++j) {
                     const uint2 one = j ? it[1] : it[0];
                     if (!(one.y & (kItemZone | kItemFar | kItemShort)))
-                        count_items<R, 1, false>(p, q, &one, part, nparts, cols, slots, lane);
+                        count_items<R, 1, false>(p, q, &one, part, nparts, cols, slots, lane, 32u * (one.y >> kItemFrom));
                 }
             } else if (phase == 2) {
 #pragma unroll 1
@@ -1188,13 +1195,11 @@ int alloc_list(StreamScratch& scr, const CountParams& p, LaneParams* q, cudaStre
     q->ctl = ctl;
     q->left = marks ? ctl + kLaneCtlWords : nullptr;
     q->list = reinterpret_cast<uint2*>(ctl + kLaneCtlWords + marks + (marks & 1u));
-    q->cap = (uint32_t)cap;
+    q->cap = q->cap_huge = q->cap_other = (uint32_t)cap;
     return SJCS_OK;
 }
 
-template <int R, bool PACK>
-int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
-                  const LaneModel* model) {
+LaneParams lane_params(const sjcs_query* qq, const CountParams& p, const LaneModel* model) {
     const auto& L = qq->lane;
     LaneParams q{};
     q.slots = L.slots;
@@ -1215,57 +1220,142 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
         q.wpref = reinterpret_cast<const uint32_t*>(p.mpts[0]) + 3;
         q.key_shift = model->key_shift;
     }
-    StreamScratch scr(s);
-    if (given) {
-        q.ctl = given->ctl;
-        q.list = given->list;
-        q.cap = given->cap;
-    } else {
-        const int rc = alloc_list(scr, p, &q, s);
-        if (rc) return rc;
-    }
-    // one block per SM (neighbouring batches share its L1); blocks of fewer
-    // warps when there are not enough batches for every SM
-    const uint64_t nbatch = (p.nhalos + 31) / 32;
-    const size_t warp_a = sizeof(LaneRows<PACK>) + (size_t)(L.ncol + 1) * 64, table = (size_t)L.nslots * 4;
-    const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxBlockSmem - table) / warp_a);  // >= 15 for any table
-    const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + (uint64_t)ctx->num_sms - 1) / (uint64_t)ctx->num_sms);
-    const size_t smem_a = nw * warp_a + table;
-    // A batch lasts as long as its longest lane: with few batches per SM long
-    // walks are left to the list (1e5 clustered halos on 2e7 particles at R =
-    // 10, 1.3 waves: 1.06 ms without this, 0.78 with it).
-    q.huge = p.nhalos < (uint64_t)ctx->num_sms * HV_WARPS * HV_BLOCKS * 4 ? kHugeFew : kHuge;
-    // With less than a batch per SM only the time of the longest walk counts,
-    // and a warp on one halo is done sooner: all are listed (100 clustered halos
-    // on one file 34 us instead of 51, 2886 uniform ones at R = 10 45 instead
-    // of 57).
-    const uint64_t floor = nbatch <= (uint64_t)ctx->num_sms ? 0 : 160;
-    // Quads of Morton cells hold a quarter more candidates than rows (1e6 x 2e5
-    // uniform at R = 20: 0.50 ms with 8, 0.35 with 10, 0.42 with 13).
-    const uint64_t per = R == RANGE_ROWS ? 8 : 10;
-    q.walk_max = (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(floor, nbatch * per / (uint64_t)ctx->num_sms));
-    const size_t smem_b = HV_WARPS * 2 * (size_t)(L.ncol + 1) * 64 + (size_t)L.nslots * 4;
-    SJCS_CUDA_TRY(allow_block_smem(k_lane_count<R, PACK>));
-    const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, (uint64_t)ctx->num_sms);
-    k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, smem_a, s>>>(p, q);
-    SJCS_LAUNCH_CHECK();
+    return q;
+}
+
+size_t listed_smem(const LaneParams& q) { return HV_WARPS * 2 * (size_t)(q.ncol + 1) * 64 + (size_t)q.nslots * 4; }
+
+// The items of q's list (front and end), and what was marked beside it.
+template <int R>
+int launch_listed(sjcs_ctx* ctx, const CountParams& p, const LaneParams& q, bool noalloc, cudaStream_t s) {
+    const size_t smem = listed_smem(q);
     int per_sm = 0;
     auto listed = k_listed_count<R, HV_BLOCKS>;
     if constexpr (R == RANGE_ROWS)
-        if (given) listed = k_listed_count<R, HV_BLOCKS_NOALLOC>;
+        if (noalloc) listed = k_listed_count<R, HV_BLOCKS_NOALLOC>;
     SJCS_CUDA_TRY(allow_block_smem(listed));
-    SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, listed, HV_THREADS, smem_b));
+    SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, listed, HV_THREADS, smem));
     if (per_sm < 1) per_sm = 1;
-    listed<<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
+    const unsigned blocks = (unsigned)(ctx->num_sms * per_sm);
+    listed<<<blocks, HV_THREADS, smem, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
     if (q.left) {
         SJCS_CUDA_TRY(allow_block_smem(k_left_count<R>));
-        k_left_count<R><<<(unsigned)(ctx->num_sms * per_sm), HV_THREADS, smem_b, s>>>(p, q);
+        k_left_count<R><<<blocks, HV_THREADS, smem, s>>>(p, q);
         SJCS_LAUNCH_CHECK();
     }
     return SJCS_OK;
 }
+
+// Most candidates of a lane's walk: a batch lasts as long as its longest lane,
+// so with few batches per SM long walks are left to the list (1e5 clustered
+// halos on 2e7 particles at R = 10, 1.3 waves: 1.06 ms without this, 0.78 with
+// it).  Quads of Morton cells hold a quarter more candidates than rows (1e6 x
+// 2e5 uniform at R = 20: 0.50 ms with 8, 0.35 with 10, 0.42 with 13).
+uint32_t walk_limit(sjcs_ctx* ctx, const CountParams& p, bool rows) {
+    const uint64_t nbatch = (p.nhalos + 31) / 32, per = rows ? 8 : 10;
+    return (uint32_t)std::min<uint64_t>(kWalkMax, std::max<uint64_t>(160, nbatch * per / (uint64_t)ctx->num_sms));
+}
+
+// Fewer halos than a few for every warp.
+bool few_halos(sjcs_ctx* ctx, const CountParams& p) {
+    return p.nhalos < (uint64_t)ctx->num_sms * HV_WARPS * HV_BLOCKS * 4;
+}
+
+template <int R, bool PACK>
+int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
+                  const LaneModel* model) {
+    LaneParams q = lane_params(qq, p, model);
+    StreamScratch scr(s);
+    if (given) {
+        q.ctl = given->ctl;
+        q.list = given->list;
+        q.cap = q.cap_huge = q.cap_other = given->cap;
+    } else {
+        const int rc = alloc_list(scr, p, &q, s);
+        if (rc) return rc;
+    }
+    q.huge = few_halos(ctx, p) ? kHugeFew : kHuge;
+    q.walk_max = walk_limit(ctx, p, R == RANGE_ROWS);
+    // one block per SM (neighbouring batches share its L1); blocks of fewer
+    // warps when there are not enough batches for every SM
+    const uint64_t nbatch = (p.nhalos + 31) / 32, sms = (uint64_t)ctx->num_sms;
+    const size_t warp_a = sizeof(LaneRows<PACK>) + (size_t)(q.ncol + 1) * 64, table = (size_t)q.nslots * 4;
+    const int fit = (int)std::min<size_t>(LN_WARPS, (kMaxBlockSmem - table) / warp_a);  // >= 15 for any table
+    const int nw = (int)std::min<uint64_t>((uint64_t)fit, (nbatch + sms - 1) / sms);
+    const uint64_t blocks = std::min<uint64_t>((nbatch + (uint64_t)nw - 1) / (uint64_t)nw, sms);
+    SJCS_CUDA_TRY(allow_block_smem(k_lane_count<R, PACK>));
+    k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, nw * warp_a + table, s>>>(p, q);
+    SJCS_LAUNCH_CHECK();
+    return launch_listed<R>(ctx, p, q, given != nullptr, s);
+}
 }  // namespace
+
+bool warps_count_sooner(sjcs_ctx* ctx, const CountParams& p) {
+    return (p.nhalos + 31) / 32 <= (uint64_t)ctx->num_sms * kFewBatches;
+}
+
+namespace {
+// About the candidates that the sphere leaves of a box far from the faces, were
+// the particles uniform.
+double uniform_candidates(const CountParams& p, bool rows) {
+    const double e = std::min(p.half, p.reach);
+    double c = 0.0;
+    for (int f = 0; f < p.nidx; ++f) c += (double)p.mn[f] / p.nidx;
+    for (int a = 0; a < 3; ++a)  // quads begin and end at even cells
+        c *= std::min(1.0, (2.0 * e + (!rows && a < 2 ? 2.0 : 1.0) * 1000.0 / p.g.G[a]) / 1000.0);
+    return 0.625 * c;
+}
+}  // namespace
+
+int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, CountParams* p, RangesOf ranges, StreamScratch& scr,
+                   cudaStream_t s, const LaneScratch* given) {
+    // What is ordinary at this density stays with its warp (listing from 1.1
+    // times that on took 106 us for 10500 uniform halos on 1e7 particles at R =
+    // 20, 1.3 to 2.5 times 97).  With less than a warp for every listed image
+    // each is split; the more halos, the more of them are left to balance the
+    // warps (clustered, 100 halos: 45 us from 512 on and 60 from 1024; 20000: 141
+    // and 129).
+    const bool split = (p->nhalos + 31) / 32 <= (uint64_t)ctx->num_sms;
+    p->heavy = (uint32_t)std::min(1e9, std::max(split ? 512.0 : 1024.0,
+                                                1.5 * uniform_candidates(*p, ranges == RangesOf::Rows)));
+    p->huge = split ? 0u : kHugeFew;
+    if (given) {
+        p->list_ctl = given->ctl;
+        p->list = given->list;
+        p->list_cap = given->cap;
+    } else {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        SJCS_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+        uint32_t* base = q->list_ctl;
+        if (capture != cudaStreamCaptureStatusNone) {
+            // a graph may run beside other counts of its query
+            SJCS_CUDA_TRY(scr.alloc(&base, kQueryListBytes));
+            SJCS_CUDA_TRY(cudaMemsetAsync(base, 0, kListWords * sizeof(uint32_t), s));
+            p->list_ctl = base;
+        } else {
+            p->list_ctl = base + (q->list_turn & 1u) * kListWords;
+            p->list_clear = base + (~q->list_turn & 1u) * kListWords;
+            ++q->list_turn;
+        }
+        p->list = reinterpret_cast<uint2*>(base + 2 * kListWords);
+        p->list_cap = kQueryListItems;
+    }
+    p->list_huge = split ? p->list_cap : p->list_cap / 2u;
+    return SJCS_OK;
+}
+
+int launch_listed_images(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, RangesOf ranges, cudaStream_t s,
+                         const LaneScratch* given, const LaneModel* model) {
+    LaneParams q = lane_params(qq, p, model);
+    q.ctl = p.list_ctl;
+    q.list = p.list;
+    q.cap = p.list_cap;
+    q.cap_huge = p.list_huge;
+    q.cap_other = p.list_cap - p.list_huge;
+    if (ranges == RangesOf::Rows) return launch_listed<RANGE_ROWS>(ctx, p, q, given != nullptr, s);
+    return model ? launch_listed<RANGE_MODEL>(ctx, p, q, false, s) : launch_listed<RANGE_CELLS>(ctx, p, q, false, s);
+}
 
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
                       const LaneScratch* given) {

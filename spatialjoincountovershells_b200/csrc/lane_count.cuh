@@ -10,7 +10,7 @@ namespace sjcs {
 bool lane_count_applies(const sjcs_query* q, const count::CountParams& p);
 // Item list of a count, when the caller provides it: kLaneCtlWords zeroed
 // control words and room for cap items, eight per halo (one per image) or more.
-constexpr int kLaneCtlWords = 8;
+constexpr int kLaneCtlWords = count::kListWords;
 struct LaneScratch {
     uint32_t* ctl;
     uint2* list;
@@ -30,6 +30,15 @@ struct LaneModel {
 };
 int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, cudaStream_t s,
                             const LaneModel* model);
+// Whether a warp to a halo is done sooner than a lane to a halo; the list that
+// its count leaves heavy images to (the query's own, or `given`; under capture
+// memory of the stream); and the count of what was listed.
+enum class RangesOf { Rows, Cells };
+bool warps_count_sooner(sjcs_ctx* ctx, const count::CountParams& p);
+int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, count::CountParams* p, RangesOf ranges, StreamScratch& scr,
+                   cudaStream_t s, const LaneScratch* given);
+int launch_listed_images(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, RangesOf ranges,
+                         cudaStream_t s, const LaneScratch* given, const LaneModel* model);
 // launch_shell_count under the static schedule without allocating.
 int launch_shell_count_noalloc(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx, const LaneScratch& scratch,
                                cudaStream_t s);

@@ -1,6 +1,6 @@
 // Warp-cooperative periodic multi-shell count over a Morton index (plain
-// Morton offset table or learned rank model), for the radius tables that the
-// lane-per-halo count (lane_count.cu) does not take.
+// Morton offset table or learned rank model), for few halos and for the radius
+// tables that the lane-per-halo count (lane_count.cu) does not take.
 //
 // One warp owns one halo at a time.  For every periodic image the warp lists
 // the level-L Morton cells of the query box (lane k takes cell k of the box),
@@ -70,12 +70,15 @@ __device__ __forceinline__ void run_ranges(const CountParams& p, const Image& im
     else run_rows<BIN, BIG>(p, im, s0, s1, sink, tab, lut, lane);
 }
 
-template <int LOOK, int BIN, bool BIG>
+// LIST: an image whose first 64 cells hold more than p.heavy candidates (its
+// whole box, when the cells are no smaller than 0.7 R) is left to the list as
+// item it.
+template <int LOOK, int BIN, bool BIG, bool LIST = false>
 __device__ __forceinline__ void count_image_m(const CountParams& p, const MortonParams& m, const RootRegs& rr,
                                               float cx, float cy, float cz, uint32_t* __restrict__ sink,
                                               const float* __restrict__ tab, const uint32_t* __restrict__ lut,
                                               uint2* __restrict__ pend, int lane, uint32_t part = 0,
-                                              uint32_t nparts = 1) {
+                                              uint32_t nparts = 1, uint2 it = make_uint2(0u, 0u)) {
     Image im;
     im.cx = cx;
     im.cy = cy;
@@ -130,6 +133,13 @@ __device__ __forceinline__ void count_image_m(const CountParams& p, const Morton
             const bool act[4] = {keep[0], keep[0], keep[1], keep[1]};
             learned_rank_n<4>(rt, m.leaves, m.wpref, qk, act, s);
         }
+        if constexpr (LIST) {
+            if (cb == 0u) {
+                const uint32_t T = __reduce_add_sync(0xffffffffu, (s[1] - s[0]) + (s[3] - s[2]));
+                // their quads: about two ranges of four cells each
+                if (T > p.heavy && list_image(p, it, T, (min(total, 64u) + 1u) / 2u, lane)) return;
+            }
+        }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const uint32_t s0 = s[2 * u], s1 = s[2 * u + 1];
@@ -158,14 +168,16 @@ __device__ __forceinline__ void count_image_m(const CountParams& p, const Morton
 
 // One halo: every periodic image (MultiRangeCount.c:31-71), then the warp's
 // counters flushed into the halo's row.
-template <int LOOK, int BIN, bool BIG>
+template <int LOOK, int BIN, bool BIG, bool LIST = false>
 __device__ __forceinline__ void count_halo_m(const CountParams& p, const MortonParams& m, const RootRegs& rr,
                                              const float4 c, uint32_t* __restrict__ wcnt,
                                              const float* __restrict__ tab, const uint32_t* __restrict__ lut,
-                                             uint2* __restrict__ pend, int lane, uint32_t part, uint32_t nparts) {
+                                             uint2* __restrict__ pend, int lane, uint32_t part, uint32_t nparts,
+                                             uint32_t place = 0) {
     uint32_t* row = p.counts + (uint64_t)__float_as_uint(c.w) * (uint64_t)p.nrads;
     uint32_t* sink = BIG ? row : wcnt;
-    count_image_m<LOOK, BIN, BIG>(p, m, rr, c.x, c.y, c.z, sink, tab, lut, pend, lane, part, nparts);
+    count_image_m<LOOK, BIN, BIG, LIST>(p, m, rr, c.x, c.y, c.z, sink, tab, lut, pend, lane, part, nparts,
+                                        make_uint2(place, 0u));
     if (p.periodic) {
         const float lox = __fsub_rn(c.x, p.half), hix = __fadd_rn(c.x, p.half);
         const float loy = __fsub_rn(c.y, p.half), hiy = __fadd_rn(c.y, p.half);
@@ -179,8 +191,9 @@ __device__ __forceinline__ void count_halo_m(const CountParams& p, const MortonP
             const float sy = (loy < kBoxLow) ? __fadd_rn(c.y, kBoxUpp) : __fsub_rn(c.y, kBoxUpp);
             const float sz = (loz < kBoxLow) ? __fadd_rn(c.z, kBoxUpp) : __fsub_rn(c.z, kBoxUpp);
             for (unsigned S = F; S != 0; S = (S - 1u) & F)
-                count_image_m<LOOK, BIN, BIG>(p, m, rr, (S & 1u) ? sx : c.x, (S & 2u) ? sy : c.y,
-                                              (S & 4u) ? sz : c.z, sink, tab, lut, pend, lane, part, nparts);
+                count_image_m<LOOK, BIN, BIG, LIST>(p, m, rr, (S & 1u) ? sx : c.x, (S & 2u) ? sy : c.y,
+                                                    (S & 4u) ? sz : c.z, sink, tab, lut, pend, lane, part, nparts,
+                                                    make_uint2(place, S));
         }
     }
     if (!BIG) {
@@ -233,15 +246,17 @@ __device__ __forceinline__ MView setup_m(const CountParams& p, const MortonParam
 
 // Static schedule: warp gw of W takes halos gw, gw + W, ... (the resident
 // warps work on one window of the Morton order and share particle lines).
-template <int LOOK, int BIN, bool BIG>
+template <int LOOK, int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(MC_THREADS, 8) k_morton_count(CountParams p, MortonParams m) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if constexpr (LIST) clear_next_list(p);
     const MView v = setup_m<LOOK, BIG>(p, m, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * MC_WARPS;
     for (uint64_t hk = (uint64_t)blockIdx.x * MC_WARPS + warp; hk < p.nhalos; hk += W)
-        count_halo_m<LOOK, BIN, BIG>(p, m, v.rr, p.halos[hk], v.wcnt, v.tab, v.lut, v.pend, lane, 0, 1);
+        count_halo_m<LOOK, BIN, BIG, LIST>(p, m, v.rr, p.halos[hk], v.wcnt, v.tab, v.lut, v.pend, lane, 0, 1,
+                                           (uint32_t)hk);
 }
 
 // Rank of a cell boundary at any level <= 10 (queue estimates): the table
@@ -343,9 +358,9 @@ __global__ void __launch_bounds__(MC_THREADS, 8) k_morton_count_queue(CountParam
     }
 }
 
-template <int LOOK, int BIN, bool BIG>
+template <int LOOK, int BIN, bool BIG, bool LIST = false>
 int launch_m(sjcs_ctx* ctx, const CountParams& p, const MortonParams& m, size_t smem, cudaStream_t s) {
-    auto kern = k_morton_count<LOOK, BIN, BIG>;
+    auto kern = k_morton_count<LOOK, BIN, BIG, LIST>;
     if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MC_THREADS, smem));
@@ -441,10 +456,10 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
     p.mpts[0] = idx->pts;
     p.mcs[0] = idx->cell_start;
     p.mn[0] = (uint32_t)idx->n;
-    if (lane_count_applies(q, p)) {
-        const LaneModel model{idx->leaves, idx->root, 63 - 3 * idx->level};
-        return launch_lane_count_cells(ctx, q, p, s, idx->kind == SJCS_INDEX_LEARNED ? &model : nullptr);
-    }
+    const bool lanes = lane_count_applies(q, p), learned = idx->kind == SJCS_INDEX_LEARNED;
+    const LaneModel model{idx->leaves, idx->root, 63 - 3 * idx->level};
+    if (lanes && !warps_count_sooner(ctx, p))
+        return launch_lane_count_cells(ctx, q, p, s, learned ? &model : nullptr);
     MortonParams m{};
     m.table = idx->cell_start;
     m.leaves = idx->leaves;
@@ -458,6 +473,19 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
     const bool big = q->pad > kMaxSmemTable || q->nrads > kMaxSmemRads;
     const size_t smem = MC_WARPS * kPend * sizeof(uint2) +
                         (big ? 0 : (size_t)(q->pad + q->nlut + MC_WARPS * q->nrads) * sizeof(uint32_t));
+    if (lanes) {
+        // a warp to a halo, the heavy images left to the listed count
+        StreamScratch scr(s);
+        int rc = list_for_warps(ctx, q, &p, RangesOf::Cells, scr, s, nullptr);
+        if (rc) return rc;
+        if (learned)
+            rc = bin == BIN_LUT ? launch_m<LOOK_MODEL, BIN_LUT, false, true>(ctx, p, m, smem, s)
+                                : launch_m<LOOK_MODEL, BIN_BSEARCH, false, true>(ctx, p, m, smem, s);
+        else
+            rc = bin == BIN_LUT ? launch_m<LOOK_TABLE, BIN_LUT, false, true>(ctx, p, m, smem, s)
+                                : launch_m<LOOK_TABLE, BIN_BSEARCH, false, true>(ctx, p, m, smem, s);
+        return rc ? rc : launch_listed_images(ctx, q, p, RangesOf::Cells, s, nullptr, learned ? &model : nullptr);
+    }
     // Learned kind: model lookups, unless the judge recorded a mismatch (the
     // kernel reads the record and then answers from the table).
     return idx->kind == SJCS_INDEX_LEARNED ? dispatch_bin<LOOK_MODEL>(ctx, bin, big, p, m, smem, s, sc)

@@ -1,7 +1,8 @@
-// Warp-cooperative periodic multi-shell count (plain grid index), for the
-// radius tables the lane-per-halo count (lane_count.cu) does not take: more
-// than 128 shells, repeated, unordered, infinite or NaN values, tables whose
-// closest values need more lookup slots than it keeps.
+// Warp-cooperative periodic multi-shell count (plain grid index), for few
+// halos, and for the radius tables the lane-per-halo count (lane_count.cu) does
+// not take: more than 128 shells, repeated, unordered, infinite or NaN values,
+// tables whose closest values need more lookup slots than it keeps.  With a
+// table that it takes, images of many candidates are left to its list.
 //
 // One warp owns one halo at a time.  For every periodic image of the halo the
 // warp turns the query box into rows of cells (one row = one contiguous slot
@@ -57,17 +58,27 @@ constexpr int CT_THREADS = CT_WARPS * 32;
 constexpr int kMaxSmemTable = 8192;  // r2 entries held in shared memory
 constexpr int kMaxSmemRads = 1024;   // per-warp shared counters up to this many shells
 
-// Every row chunk of an image from chunk `first_chunk` on, synchronously.
-template <int BIN, bool BIG>
-__device__ __forceinline__ void count_image(const CountParams& p, const Image& im, uint32_t first_chunk,
-                                            uint32_t* __restrict__ sink, const float* __restrict__ tab,
-                                            const uint32_t* __restrict__ lut, int lane) {
+// Every row chunk of an image, synchronously.  LIST: from the chunk on with
+// which it has more than p.heavy candidates it is left to the list.
+template <int BIN, bool BIG, bool LIST = false>
+__device__ __forceinline__ void count_image(const CountParams& p, const Image& im, uint32_t* __restrict__ sink,
+                                            const float* __restrict__ tab, const uint32_t* __restrict__ lut, int lane,
+                                            uint2 it = make_uint2(0u, 0u)) {
     float gy, gz;
     gap_tables(p, im, lane, &gy, &gz);
-    for (uint32_t rb = first_chunk * 32u; rb < im.nrows; rb += 32u) {
+    uint32_t most = p.heavy;
+    for (uint32_t rb = 0; rb < im.nrows; rb += 32u) {
         uint32_t s0, s1;
         row_issue(p, im, rb, lane, gy, gz, &s0, &s1);
-        run_rows<BIN, BIG>(p, im, s0, s1, sink, tab, lut, lane);
+        if constexpr (LIST) {
+            const bool may = (rb >> 5) < kItemFromMax;
+            const uint32_t n = run_rows<BIN, BIG, true>(p, im, s0, s1, sink, tab, lut, lane, may ? most : 0xffffffffu,
+                                                        make_uint2(it.x, it.y | ((rb >> 5) << kItemFrom)));
+            if (n == kListed) return;
+            most -= min(n, most);
+        } else {
+            run_rows<BIN, BIG>(p, im, s0, s1, sink, tab, lut, lane);
+        }
     }
 }
 
@@ -90,11 +101,12 @@ __device__ __forceinline__ void count_image_part(const CountParams& p, const Ima
 // Periodic images other than the un-shifted one: every non-empty subset S of
 // the flagged axes (MultiRangeCount.c:31-71).  nparts > 1: this warp's piece
 // of each image only.
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool LIST = false>
 __device__ __forceinline__ void count_shifted_images(const CountParams& p, const float4 c,
                                                      uint32_t* __restrict__ sink, const float* __restrict__ tab,
                                                      const uint32_t* __restrict__ lut, int lane,
-                                                     uint32_t part = 0, uint32_t nparts = 1) {
+                                                     uint32_t part = 0, uint32_t nparts = 1,
+                                                     uint2 it = make_uint2(0u, 0u)) {
     const float lox = __fsub_rn(c.x, p.half), hix = __fadd_rn(c.x, p.half);
     const float loy = __fsub_rn(c.y, p.half), hiy = __fadd_rn(c.y, p.half);
     const float loz = __fsub_rn(c.z, p.half), hiz = __fadd_rn(c.z, p.half);
@@ -109,7 +121,7 @@ __device__ __forceinline__ void count_shifted_images(const CountParams& p, const
     for (unsigned S = F; S != 0; S = (S - 1u) & F) {
         const Image im = make_image(p, (S & 1u) ? sx : c.x, (S & 2u) ? sy : c.y, (S & 4u) ? sz : c.z);
         if (nparts > 1) count_image_part<BIN, BIG>(p, im, sink, tab, lut, lane, part, nparts);
-        else count_image<BIN, BIG>(p, im, 0, sink, tab, lut, lane);
+        else count_image<BIN, BIG, LIST>(p, im, sink, tab, lut, lane, make_uint2(it.x, it.y | S));
     }
 }
 
@@ -213,11 +225,13 @@ __device__ __forceinline__ void flush_counts(const CountParams& p, uint32_t* __r
 // lane per halo; execution runs the whole warp on one halo at a time over its
 // planned rows, while the cell-table loads of the next halo of the batch are
 // in flight.  Halos with more than 28 rows and the shifted periodic images
-// (about 3% of halos at the workload's sizes) are counted in place.
-template <int BIN, bool BIG>
+// (about 3% of halos at the workload's sizes) are counted in place.  Halo k is
+// the one at place h0 + k * step.
+template <int BIN, bool BIG, bool LIST = false>
 __device__ __forceinline__ void count_batch(const CountParams& p, WarpPlans* wp, uint32_t nb, float4 c_lane,
                                             uint32_t* __restrict__ wcnt, const float* __restrict__ tab,
-                                            const uint32_t* __restrict__ lut, int lane) {
+                                            const uint32_t* __restrict__ lut, int lane, uint32_t h0 = 0,
+                                            uint32_t step = 0) {
     {
         const bool valid = (uint32_t)lane < nb;
         plan_halo(p, c_lane, valid, &wp->plan[lane], wp->row_cell[lane], wp->row_len[lane]);
@@ -248,12 +262,15 @@ __device__ __forceinline__ void count_batch(const CountParams& p, WarpPlans* wp,
         im.hiy = __fadd_rn(pl.cy, p.half);
         im.loz = __fsub_rn(pl.cz, p.half);
         im.hiz = __fadd_rn(pl.cz, p.half);
+        const uint2 it = make_uint2(h0 + k * step, 0u);
         if (pl.nrows == kSlowPlan) {
-            count_image<BIN, BIG>(p, make_image(p, pl.cx, pl.cy, pl.cz), 0, sink, tab, lut, lane);
+            count_image<BIN, BIG, LIST>(p, make_image(p, pl.cx, pl.cy, pl.cz), sink, tab, lut, lane, it);
         } else {
-            run_rows<BIN, BIG>(p, im, s0, s1, sink, tab, lut, lane);
+            run_rows<BIN, BIG, LIST>(p, im, s0, s1, sink, tab, lut, lane, p.heavy, it);
         }
-        if (pl.flags) count_shifted_images<BIN, BIG>(p, make_float4(pl.cx, pl.cy, pl.cz, 0.f), sink, tab, lut, lane);
+        if (pl.flags)
+            count_shifted_images<BIN, BIG, LIST>(p, make_float4(pl.cx, pl.cy, pl.cz, 0.f), sink, tab, lut, lane, 0, 1,
+                                                 it);
         if (!BIG) flush_counts(p, wcnt, row, lane);
         s0 = t0;
         s1 = t1;
@@ -267,10 +284,11 @@ __device__ __forceinline__ void count_batch(const CountParams& p, WarpPlans* wp,
 // tests -- before its counters are flushed once.  Each index is counted
 // through a copy of the parameters that points at it, so the row and
 // candidate code is the single-index code.
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool LIST = false>
 __device__ __forceinline__ void count_batch_multi(const CountParams& p, WarpPlans* wp, uint32_t nb, float4 c_lane,
                                                   uint32_t* __restrict__ wcnt, const float* __restrict__ tab,
-                                                  const uint32_t* __restrict__ lut, int lane) {
+                                                  const uint32_t* __restrict__ lut, int lane, uint32_t h0 = 0,
+                                                  uint32_t step = 0) {
     {
         const bool valid = (uint32_t)lane < nb;
         plan_halo(p, c_lane, valid, &wp->plan[lane], wp->row_cell[lane], wp->row_len[lane]);
@@ -302,8 +320,9 @@ __device__ __forceinline__ void count_batch_multi(const CountParams& p, WarpPlan
             // across the index loop
             const HaloPlan pl = wp->plan[k];
             uint32_t* sink = BIG ? p.counts + (uint64_t)pl.row * (uint64_t)p.nrads : wcnt;
+            const uint2 it = make_uint2(h0 + k * step, (uint32_t)f << 3);
             if (pl.nrows == kSlowPlan) {
-                count_image<BIN, BIG>(pf, make_image(pf, pl.cx, pl.cy, pl.cz), 0, sink, tab, lut, lane);
+                count_image<BIN, BIG, LIST>(pf, make_image(pf, pl.cx, pl.cy, pl.cz), sink, tab, lut, lane, it);
             } else {
                 Image im;
                 im.cx = pl.cx;
@@ -315,9 +334,11 @@ __device__ __forceinline__ void count_batch_multi(const CountParams& p, WarpPlan
                 im.hiy = __fadd_rn(pl.cy, p.half);
                 im.loz = __fsub_rn(pl.cz, p.half);
                 im.hiz = __fadd_rn(pl.cz, p.half);
-                run_rows<BIN, BIG>(pf, im, s0, s1, sink, tab, lut, lane);
+                run_rows<BIN, BIG, LIST>(pf, im, s0, s1, sink, tab, lut, lane, p.heavy, it);
             }
-            if (pl.flags) count_shifted_images<BIN, BIG>(pf, make_float4(pl.cx, pl.cy, pl.cz, 0.f), sink, tab, lut, lane);
+            if (pl.flags)
+                count_shifted_images<BIN, BIG, LIST>(pf, make_float4(pl.cx, pl.cy, pl.cz, 0.f), sink, tab, lut, lane, 0,
+                                                     1, it);
             s0 = t0;
             s1 = t1;
         }
@@ -355,10 +376,11 @@ __device__ __forceinline__ SmemView setup_smem(const CountParams& p, uint32_t* s
 // Static schedule: warp gw of W takes halos gw, gw + W, gw + 2W, ... in
 // batches of 32, so at any moment the resident warps work on one contiguous
 // window of the Morton order and share particle lines in L1/L2.
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count(CountParams p) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if constexpr (LIST) clear_next_list(p);
     const SmemView v = setup_smem<BIG>(p, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * CT_WARPS;
@@ -367,15 +389,16 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count(CountParams p) {
     for (uint64_t b0 = 0; b0 < mine; b0 += kBatch) {
         const uint32_t nb = (uint32_t)min((uint64_t)kBatch, mine - b0);
         const float4 c = (uint32_t)lane < nb ? p.halos[(b0 + lane) * W + gw] : make_float4(0.f, 0.f, 0.f, 0.f);
-        count_batch<BIN, BIG>(p, v.wp, nb, c, v.wcnt, v.tab, v.lut, lane);
+        count_batch<BIN, BIG, LIST>(p, v.wp, nb, c, v.wcnt, v.tab, v.lut, lane, (uint32_t)(b0 * W + gw), (uint32_t)W);
     }
 }
 
 // Static schedule over p.nidx indexes of one grid (count_batch_multi).
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_multi(CountParams p) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if constexpr (LIST) clear_next_list(p);
     const SmemView v = setup_smem<BIG>(p, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * CT_WARPS;
@@ -384,7 +407,8 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_multi(CountParams
     for (uint64_t b0 = 0; b0 < mine; b0 += kBatch) {
         const uint32_t nb = (uint32_t)min((uint64_t)kBatch, mine - b0);
         const float4 c = (uint32_t)lane < nb ? p.halos[(b0 + lane) * W + gw] : make_float4(0.f, 0.f, 0.f, 0.f);
-        count_batch_multi<BIN, BIG>(p, v.wp, nb, c, v.wcnt, v.tab, v.lut, lane);
+        count_batch_multi<BIN, BIG, LIST>(p, v.wp, nb, c, v.wcnt, v.tab, v.lut, lane, (uint32_t)(b0 * W + gw),
+                                          (uint32_t)W);
     }
 }
 
@@ -473,7 +497,7 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_queue(CountParams
             uint32_t* sink = BIG ? row : v.wcnt;
             const Image im = make_image(p, c.x, c.y, c.z);
             if (bp.pieces > 1) count_image_part<BIN, BIG>(p, im, sink, v.tab, v.lut, lane, part, bp.pieces);
-            else count_image<BIN, BIG>(p, im, 0, sink, v.tab, v.lut, lane);
+            else count_image<BIN, BIG>(p, im, sink, v.tab, v.lut, lane);
             if (p.periodic) count_shifted_images<BIN, BIG>(p, c, sink, v.tab, v.lut, lane, part, bp.pieces);
             if (!BIG) flush_counts(p, v.wcnt, row, lane);
         } else {
@@ -486,9 +510,9 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_queue(CountParams
     }
 }
 
-template <int BIN, bool BIG>
+template <int BIN, bool BIG, bool LIST = false>
 int launch_variant(sjcs_ctx* ctx, const CountParams& p, size_t smem, cudaStream_t s, bool multi = false) {
-    auto kern = multi ? k_shell_count_multi<BIN, BIG> : k_shell_count<BIN, BIG>;
+    auto kern = multi ? k_shell_count_multi<BIN, BIG, LIST> : k_shell_count<BIN, BIG, LIST>;
     if (smem > 48 * 1024) SJCS_CUDA_TRY(allow_block_smem(kern));
     int per_sm = 0;
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CT_THREADS, smem));
@@ -587,6 +611,23 @@ int launch_static(sjcs_ctx* ctx, const CountParams& p, int bin, bool big, size_t
 
 }  // namespace
 
+// A query that lanes can count: by lanes, or where a warp to a halo is done
+// sooner by the static kernel, whose heavy images the listed count splits.
+namespace {
+int launch_lanes_or_warps(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
+                          const LaneScratch* given) {
+    if (!warps_count_sooner(ctx, p)) return launch_lane_count(ctx, q, p, s, given);
+    CountParams w = p;
+    StreamScratch scr(s);
+    int rc = list_for_warps(ctx, q, &w, RangesOf::Rows, scr, s, given);
+    if (rc) return rc;
+    const bool multi = p.nidx > 1;
+    rc = bin_mode(q) == BIN_LUT ? launch_variant<BIN_LUT, false, true>(ctx, w, count_smem(q), s, multi)
+                                : launch_variant<BIN_BSEARCH, false, true>(ctx, w, count_smem(q), s, multi);
+    return rc ? rc : launch_listed_images(ctx, q, w, RangesOf::Rows, s, given, nullptr);
+}
+}  // namespace
+
 namespace {
 // Sizes the queue schedule refuses, whichever kernel counts.
 bool queue_too_large(const sjcs_query* q, const Schedule& sc) {
@@ -606,8 +647,8 @@ int launch_shell_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* idx
     const CountParams p = count_params(q, idx);
     if (sc && sc->mode == SJCS_SCHED_QUEUE && queue_too_large(q, *sc))
         return fail(SJCS_ERR_INVALID, "queue schedule: nhalos * max_pieces must stay below 2^32");
-    // Either schedule: the lane count lists heavy halos itself and splits them.
-    if (lane_count_applies(q, p)) return launch_lane_count(ctx, q, p, s);
+    // Either schedule: these list heavy halos themselves and split them.
+    if (lane_count_applies(q, p)) return launch_lanes_or_warps(ctx, q, p, s, nullptr);
     const int bin = bin_mode(q);
     const bool big = big_tables(q);
     const size_t smem = count_smem(q);
@@ -631,7 +672,7 @@ int launch_shell_count_noalloc(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_in
                                cudaStream_t s) {
     if (q->nhalos == 0 || idx->n == 0) return SJCS_OK;
     const CountParams p = count_params(q, idx);
-    if (lane_count_applies(q, p)) return launch_lane_count(ctx, q, p, s, &scratch);
+    if (lane_count_applies(q, p)) return launch_lanes_or_warps(ctx, q, p, s, &scratch);
     return launch_static(ctx, p, bin_mode(q), big_tables(q), count_smem(q), s, false);
 }
 
@@ -648,7 +689,7 @@ int launch_shell_count_multi(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_inde
         ++p.nidx;
     }
     if (q->nhalos == 0 || p.nidx == 0) return SJCS_OK;
-    if (lane_count_applies(q, p)) return launch_lane_count(ctx, q, p, s);
+    if (lane_count_applies(q, p)) return launch_lanes_or_warps(ctx, q, p, s, nullptr);
     return launch_static(ctx, p, bin_mode(q), big_tables(q), count_smem(q), s, true);
 }
 

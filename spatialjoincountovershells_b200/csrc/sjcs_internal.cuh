@@ -166,6 +166,11 @@ struct sjcs_index {
     bool had_h2d;
 };
 
+namespace sjcs {
+constexpr uint32_t kQueryListItems = 16384;
+constexpr size_t kQueryListBytes = 2 * 8 * sizeof(uint32_t) + kQueryListItems * sizeof(uint2);
+}  // namespace sjcs
+
 struct sjcs_query {
     uint32_t magic;
     sjcs_ctx* ctx;
@@ -179,6 +184,11 @@ struct sjcs_query {
     float r2max;
     float4* halos;      // Morton-sorted halos, .w = original index bits
     uint32_t* counts;   // [nhalos][nrads], caller's halo order
+    // Behind them: two sets of control words and a list of images for counts
+    // that give a warp to each halo (shell_count.cu, morton_count.cu).  A count
+    // takes the sets in turn and clears the other one.
+    uint32_t* list_ctl;
+    mutable uint32_t list_turn;
     float* d_r2;        // [pad], entries past nrads = +inf
     // Shell lookup on the bit pattern of dist (non-negative floats order like
     // their bits): slot j covers keys [lut_k0 + j<<lut_shift, ...+1<<lut_shift)

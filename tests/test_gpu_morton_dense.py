@@ -28,8 +28,8 @@ def test_dense_cell_outside_the_box(ctx, kind, dense, many):
     block = corner + rng.uniform(0.05, 0.95, (many, 3)) * CELL
     p = np.concatenate([block, rng.uniform(0, 1000, (20000, 3))]).astype(np.float32)
     # around the dense cell, where most warps hold a lane with more than 25
-    # quads; more than a batch of 32 per SM, so that lanes walk
-    h = rng.uniform(corner - 80, corner + 110, (5200, 3)).astype(np.float32)
+    # quads; more than five batches of 32 per SM, so that lanes walk
+    h = rng.uniform(corner - 80, corner + 110, (25000, 3)).astype(np.float32)
     r2 = nat.radius_table(0.5, RADIUS, 12)
     idx = ctx.build_index(p, radius_hint=RADIUS, kind=kind, level=LEVEL)
     q = ctx.query(h, r2)
