@@ -1111,7 +1111,8 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
                 for (uint32_t j = 0; j < n; ++j) {
                     const uint2 one = j ? it[1] : it[0];
                     if (one.y & (kItemZone | kItemFar)) count_literal<R>(p, q, one, part, nparts, lane);
-                    else if (one.y & kItemShort) count_items<R, 1, true>(p, q, &one, part, nparts, cols, slots, lane);
+                    else if (one.y & kItemShort)
+                        count_items<R, 1, true>(p, q, &one, part, nparts, cols, slots, lane, 32u * (one.y >> kItemFrom));
                 }
             }
         }

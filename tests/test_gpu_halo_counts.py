@@ -94,3 +94,28 @@ def test_many_halos_on_cells_of_any_level(ctx, kind, level):
     grid = None if kind != nat.INDEX_GRID else (2**level,) * 3
     got = _count(ctx, [p], h, r2, kind=kind, grid=grid, level=0 if grid else level)
     assert np.array_equal(got, oracle.count(p, h, r2))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("data", ["uniform", "clumps", "few clumps"])
+@pytest.mark.parametrize("files", [1, 3])
+@pytest.mark.parametrize("m", [3000])
+def test_full_boxes(ctx, kind, data, files, m):
+    """Boxes of many rows of many candidates, clumps around most halos or around
+    3 % of them: images listed from a later part of their box on, in short rows
+    and long ones."""
+    rng = np.random.default_rng(1550)
+    n, radius = 40000, 120.0
+    ps = [rng.uniform(0, 1000, (n, 3)) for _ in range(files)]
+    h = rng.uniform(0, 1000, (m, 3))
+    if data != "uniform":
+        centre = rng.uniform(0, 1000, (20, 3))
+        for p in ps:
+            p[: n // 2] = (centre[rng.integers(0, 20, n // 2)] + rng.normal(0, 25, (n // 2, 3))) % 1000.0
+        k = m if data == "clumps" else m // 32
+        h[:k] = (centre[rng.integers(0, 20, k)] + rng.normal(0, 20, (k, 3))) % 1000.0
+        rng.shuffle(h)
+    ps, h = [p.astype(np.float32) for p in ps], h.astype(np.float32)
+    r2 = nat.radius_table(2.0, radius, 14)
+    got = _count(ctx, ps, h, r2, hint=radius, kind=kind)
+    assert np.array_equal(got[:6000], sum(oracle.count(p, h[:6000], r2) for p in ps))
