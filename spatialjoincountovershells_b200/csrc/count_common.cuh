@@ -48,6 +48,7 @@ struct CountParams {
     uint32_t list_cap, list_huge;  // room, and the part of it for huge ones
     uint32_t* list_ctl;            // [1] huge ones, from the front, [2] others, from the end
     uint32_t* list_clear;  // control words to clear for the next count, or null
+    const uint32_t* gate;  // LIST variants count only if this holds a 1 (null: always)
     uint2* list;
 };
 

@@ -92,6 +92,7 @@ constexpr uint32_t kSpan = 1u << 20;  // candidates between two looks at what th
 // halos than a few per warp, items are split from kHugeFew on.
 constexpr uint32_t kHuge = 65536, kHugeFew = 2048;
 constexpr int kCtlLeft = 6;  // control word: something was marked in LaneParams::left; the next one, claims of it
+constexpr int kCtlGate = 8;  // LaneParams::gate
 constexpr uint32_t kGallop = 15;  // first step of the search for a cell's end
 constexpr uint32_t kEndSlot = 0xfffeffffu;  // no index has this many particles on this path
 // Work in cycles of the data pipe, to decide which lanes are listed and how: a
@@ -117,7 +118,8 @@ struct LaneParams {
     uint32_t zone0, zone;  // bit pattern of safe2; that of r2max less it
     // Items: the huge ones from the front of the list, the others from its end.
     uint2* __restrict__ list;  // (halo, flags)
-    uint32_t cap, cap_huge, cap_other;  // its room, and that of either kind
+    uint32_t cap, cap_huge, cap_other;  // its room, and that of either kind when warps counted
+    uint32_t* __restrict__ gate;        // 1: warps count instead of lanes (null: lanes)
     uint32_t* __restrict__ ctl;   // [0] items asked for, [1] huge, [2] others, [3-5] claims by phase, kCtlLeft
     uint32_t* __restrict__ left;  // marks of what did not fit the list (null: the list holds every item)
     // learned index: its model (leaves null: the other kinds)
@@ -134,6 +136,14 @@ struct LaneParams {
 // -> 113; learned index, 1500 on 1e6 77 -> 30.  35000 halos on 5e6, R = 7:
 // uniform 62 -> 55, clustered 151 -> 152; on 1e7, R = 10 98 -> 77 and 283 -> 325.
 constexpr uint64_t kFewBatches = 5;
+// Candidates per row and per quad of a box up to which a warp to a halo is ahead
+// of the listed count (uniform halos, nothing walked; 2e5 on 1e7 particles: R =
+// 20 and 30, 8 and 22 to a row, 575 us against 1048 and 1319 against 1683, R =
+// 50, 102 to a row, 5121 against 2793; quads of 94 at R = 20 893 against 991, of
+// 705 at R = 30 3140 against 1664).
+constexpr double kLongRow = 37.0, kLongQuad = 200.0;
+// Halos sampled to see whether they lie in clumps, and how many of them may.
+constexpr int kSample = 256, kSampleDense = 32;
 
 // What a candidate range is: a row of grid cells clipped in x; or four Morton
 // cells that follow each other in the curve (x and y even and the next ones),
@@ -328,6 +338,7 @@ template <int R, bool PACK>
 __global__ void __launch_bounds__(LN_WARPS * 32, 1)
 k_lane_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
+    if (q.gate && *q.gate != 0u) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     LaneRows<PACK>* rows = reinterpret_cast<LaneRows<PACK>*>(smem) + warp;
     const int nwarps = (int)(blockDim.x >> 5);
@@ -1062,7 +1073,9 @@ template <int R, int BLOCKS>
 __global__ void __launch_bounds__(HV_THREADS, BLOCKS)
 k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
-    const uint32_t nhuge = min(q.ctl[1], q.cap_huge), nother = min(q.ctl[2], q.cap_other);
+    const bool whole = q.gate && *q.gate == 0u;  // lanes counted: all room was for either kind
+    const uint32_t nhuge = min(q.ctl[1], whole ? q.cap : q.cap_huge);
+    const uint32_t nother = min(q.ctl[2], whole ? q.cap : q.cap_other);
     if (nhuge + nother == 0u) return;
     // Warps claim (two items, part); only huge items have several parts.  With
     // fewer items than warps each is claimed alone, and blocks beyond the last
@@ -1200,6 +1213,37 @@ int alloc_list(StreamScratch& scr, const CountParams& p, LaneParams* q, cudaStre
     return SJCS_OK;
 }
 
+// 1 to *gate if few of the halos sampled lie in clumps: if the 3 x 3 rows around
+// a halo's, as far as its box in x (its own quad, in a Morton index), hold more
+// than 2.5 times the particles of a uniform set there.
+template <bool ROWS>
+__global__ void __launch_bounds__(kSample) k_sample_density(const __grid_constant__ CountParams p,
+                                                            uint32_t* __restrict__ gate) {
+    const uint64_t h = (uint64_t)threadIdx.x * p.nhalos / kSample;
+    const float4 c = p.halos[h];
+    const Image im = make_image(p, c.x, c.y, c.z);
+    const int y = cell_of(c.y, p.g.inv_h[1], p.g.G[1]), z = cell_of(c.z, p.g.inv_h[2], p.g.G[2]);
+    const uint32_t* __restrict__ cs = p.mcs[0];
+    uint32_t n = 0, cells = 0;
+    if constexpr (ROWS) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int yy = y + k % 3 - 1, zz = z + k / 3 - 1;
+            if (yy < 0 || yy >= p.g.G[1] || zz < 0 || zz >= p.g.G[2]) continue;
+            const uint64_t rc = ((uint64_t)zz * (uint64_t)p.g.G[1] + (uint64_t)yy) * (uint64_t)p.g.G[0];
+            n += __ldg(cs + rc + im.x1 + 1) - __ldg(cs + rc + im.x0);
+            cells += (uint32_t)(im.x1 - im.x0 + 1);
+        }
+    } else {
+        const uint32_t code = morton_cell((uint32_t)cell_of(c.x, p.g.inv_h[0], p.g.G[0]), (uint32_t)y, (uint32_t)z) & ~3u;
+        n = __ldg(cs + code + 4u) - __ldg(cs + code);
+        cells = 4u;
+    }
+    const bool dense = (float)n > 2.5f * (float)p.mn[0] * (float)cells / (float)p.g.ncells;
+    const int all = __syncthreads_count(dense);
+    if (threadIdx.x == 0) *gate = all <= kSampleDense ? 1u : 0u;
+}
+
 LaneParams lane_params(const sjcs_query* qq, const CountParams& p, const LaneModel* model) {
     const auto& L = qq->lane;
     LaneParams q{};
@@ -1263,9 +1307,27 @@ bool few_halos(sjcs_ctx* ctx, const CountParams& p) {
     return p.nhalos < (uint64_t)ctx->num_sms * HV_WARPS * HV_BLOCKS * 4;
 }
 
+// The box of a halo far from the faces, were the particles uniform: about the
+// candidates that the sphere leaves of it, and its ranges.
+struct UniformBox {
+    double candidates, ranges;
+};
+UniformBox uniform_box(const CountParams& p, bool rows) {
+    const double e = std::min(p.half, p.reach);
+    UniformBox b{0.0, 1.0};
+    for (int f = 0; f < p.nidx; ++f) b.candidates += 0.625 * p.mn[f] / p.nidx;
+    for (int a = 0; a < 3; ++a) {
+        const double h = 1000.0 / p.g.G[a], unit = !rows && a < 2 ? 2.0 * h : h;  // quads begin and end at even cells
+        const double w = std::min(1000.0, 2.0 * e + unit);
+        b.candidates *= w / 1000.0;
+        if (!rows || a > 0) b.ranges *= w / unit;
+    }
+    return b;
+}
+
 template <int R, bool PACK>
 int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cudaStream_t s, const LaneScratch* given,
-                  const LaneModel* model) {
+                  const LaneModel* model, const Warps& warps) {
     LaneParams q = lane_params(qq, p, model);
     StreamScratch scr(s);
     if (given) {
@@ -1278,6 +1340,21 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     }
     q.huge = few_halos(ctx, p) ? kHugeFew : kHuge;
     q.walk_max = walk_limit(ctx, p, R == RANGE_ROWS);
+    if (warps) {
+        CountParams w = p;
+        w.gate = q.gate = q.ctl + kCtlGate;
+        k_sample_density<R == RANGE_ROWS><<<1, kSample, 0, s>>>(p, q.gate);
+        SJCS_LAUNCH_CHECK();
+        w.heavy = (uint32_t)std::min(1e9, 1.5 * uniform_box(p, R == RANGE_ROWS).candidates);
+        w.huge = q.huge;
+        w.list_ctl = q.ctl;
+        w.list = q.list;
+        w.list_cap = q.cap;
+        w.list_huge = q.cap_huge = q.cap / 8u;
+        q.cap_other = q.cap - q.cap_huge;
+        const int rc = warps(w);
+        if (rc) return rc;
+    }
     // one block per SM (neighbouring batches share its L1); blocks of fewer
     // warps when there are not enough batches for every SM
     const uint64_t nbatch = (p.nhalos + 31) / 32, sms = (uint64_t)ctx->num_sms;
@@ -1292,22 +1369,34 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
 }
 }  // namespace
 
-bool warps_count_sooner(sjcs_ctx* ctx, const CountParams& p) {
-    return (p.nhalos + 31) / 32 <= (uint64_t)ctx->num_sms * kFewBatches;
-}
-
 namespace {
-// About the candidates that the sphere leaves of a box far from the faces, were
-// the particles uniform.
-double uniform_candidates(const CountParams& p, bool rows) {
-    const double e = std::min(p.half, p.reach);
-    double c = 0.0;
-    for (int f = 0; f < p.nidx; ++f) c += (double)p.mn[f] / p.nidx;
-    for (int a = 0; a < 3; ++a)  // quads begin and end at even cells
-        c *= std::min(1.0, (2.0 * e + (!rows && a < 2 ? 2.0 : 1.0) * 1000.0 / p.g.G[a]) / 1000.0);
-    return 0.625 * c;
+bool few_batches(const sjcs_ctx* ctx, uint64_t nhalos) {
+    return (nhalos + 31) / 32 <= (uint64_t)ctx->num_sms * kFewBatches;
 }
 }  // namespace
+
+// Most halos have an image or two that is listed, on one to three indexes.
+uint32_t count_by_warps_items(const sjcs_ctx* ctx, uint64_t nhalos) {
+    return few_batches(ctx, nhalos) ? (uint32_t)std::min<uint64_t>(8 * nhalos, 131072) : 0u;
+}
+
+// Boxes that lanes would walk: by the number of batches.  Fuller ones are all
+// listed by lanes: that is ahead in long rows, and behind in short ones unless
+// the halos lie in clumps (1e5 on 3e7 particles, R = 15: uniform 805 us listed
+// and 404 by warps, clustered 1388 and 1870), which a sample of 6 us tells; the
+// extra launches take 15 us of a small count.  Below a batch per SM nothing
+// pays for a sample, and rows are better off with warps (1000 on 2e7, R = 20:
+// clustered 151 and 153, uniform 73 and 54), quads of the table with lanes (124
+// and 212, 107 and 75), those of the model with warps (473 and 262, 350 and 91).
+Counter who_counts(sjcs_ctx* ctx, const CountParams& p, RangesOf of) {
+    const bool rows = of == RangesOf::Rows, few = few_batches(ctx, p.nhalos);
+    const UniformBox b = uniform_box(p, rows);
+    if (b.candidates <= (double)walk_limit(ctx, p, rows)) return few ? Counter::Warps : Counter::Lanes;
+    if (b.candidates >= (rows ? kLongRow : kLongQuad) * b.ranges) return Counter::Lanes;
+    if (few && of == RangesOf::Model) return Counter::Warps;
+    if ((p.nhalos + 31) / 32 <= (uint64_t)ctx->num_sms) return rows ? Counter::Warps : Counter::Lanes;
+    return Counter::Sampled;
+}
 
 int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, CountParams* p, RangesOf ranges, StreamScratch& scr,
                    cudaStream_t s, const LaneScratch* given) {
@@ -1318,8 +1407,8 @@ int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, CountParams* p, RangesOf 
     // warps (clustered, 100 halos: 45 us from 512 on and 60 from 1024; 20000: 141
     // and 129).
     const bool split = (p->nhalos + 31) / 32 <= (uint64_t)ctx->num_sms;
-    p->heavy = (uint32_t)std::min(1e9, std::max(split ? 512.0 : 1024.0,
-                                                1.5 * uniform_candidates(*p, ranges == RangesOf::Rows)));
+    p->heavy = (uint32_t)std::min(
+        1e9, std::max(split ? 512.0 : 1024.0, (split ? 1.2 : 1.5) * uniform_box(*p, ranges == RangesOf::Rows).candidates));
     p->huge = split ? 0u : kHugeFew;
     if (given) {
         p->list_ctl = given->ctl;
@@ -1331,7 +1420,7 @@ int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, CountParams* p, RangesOf 
         uint32_t* base = q->list_ctl;
         if (capture != cudaStreamCaptureStatusNone) {
             // a graph may run beside other counts of its query
-            SJCS_CUDA_TRY(scr.alloc(&base, kQueryListBytes));
+            SJCS_CUDA_TRY(scr.alloc(&base, count_by_warps_bytes(q->list_items)));
             SJCS_CUDA_TRY(cudaMemsetAsync(base, 0, kListWords * sizeof(uint32_t), s));
             p->list_ctl = base;
         } else {
@@ -1340,7 +1429,7 @@ int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, CountParams* p, RangesOf 
             ++q->list_turn;
         }
         p->list = reinterpret_cast<uint2*>(base + 2 * kListWords);
-        p->list_cap = kQueryListItems;
+        p->list_cap = q->list_items;
     }
     p->list_huge = split ? p->list_cap : p->list_cap / 2u;
     return SJCS_OK;
@@ -1359,19 +1448,19 @@ int launch_listed_images(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams&
 }
 
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
-                      const LaneScratch* given) {
+                      const LaneScratch* given, const Warps& warps) {
     // Packed rows need the slots of a box's planes within 2^24 of each other;
     // with more than 2^29 particles ordinary boxes would not be.
     bool pack = true;
     for (int i = 0; i < p.nidx; ++i) pack &= p.mn[i] <= (1u << 29);
-    return pack ? launch_ranges<RANGE_ROWS, true>(ctx, q, p, s, given, nullptr)
-                : launch_ranges<RANGE_ROWS, false>(ctx, q, p, s, given, nullptr);
+    return pack ? launch_ranges<RANGE_ROWS, true>(ctx, q, p, s, given, nullptr, warps)
+                : launch_ranges<RANGE_ROWS, false>(ctx, q, p, s, given, nullptr, warps);
 }
 
 int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
-                            const LaneModel* model) {
-    return model ? launch_ranges<RANGE_MODEL, false>(ctx, q, p, s, nullptr, model)
-                 : launch_ranges<RANGE_CELLS, false>(ctx, q, p, s, nullptr, nullptr);
+                            const LaneModel* model, const Warps& warps) {
+    return model ? launch_ranges<RANGE_MODEL, false>(ctx, q, p, s, nullptr, model, warps)
+                 : launch_ranges<RANGE_CELLS, false>(ctx, q, p, s, nullptr, nullptr, warps);
 }
 
 }  // namespace sjcs

@@ -250,7 +250,10 @@ template <int LOOK, int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(MC_THREADS, 8) k_morton_count(CountParams p, MortonParams m) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if constexpr (LIST) clear_next_list(p);
+    if constexpr (LIST) {
+        if (p.gate && *p.gate == 0u) return;
+        clear_next_list(p);
+    }
     const MView v = setup_m<LOOK, BIG>(p, m, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * MC_WARPS;
@@ -458,8 +461,7 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
     p.mn[0] = (uint32_t)idx->n;
     const bool lanes = lane_count_applies(q, p), learned = idx->kind == SJCS_INDEX_LEARNED;
     const LaneModel model{idx->leaves, idx->root, 63 - 3 * idx->level};
-    if (lanes && !warps_count_sooner(ctx, p))
-        return launch_lane_count_cells(ctx, q, p, s, learned ? &model : nullptr);
+    const Counter who = lanes ? who_counts(ctx, p, learned ? RangesOf::Model : RangesOf::Cells) : Counter::Warps;
     MortonParams m{};
     m.table = idx->cell_start;
     m.leaves = idx->leaves;
@@ -475,16 +477,20 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
                         (big ? 0 : (size_t)(q->pad + q->nlut + MC_WARPS * q->nrads) * sizeof(uint32_t));
     if (lanes) {
         // a warp to a halo, the heavy images left to the listed count
+        auto by_warps = [&](const CountParams& w) {
+            if (learned)
+                return bin == BIN_LUT ? launch_m<LOOK_MODEL, BIN_LUT, false, true>(ctx, w, m, smem, s)
+                                      : launch_m<LOOK_MODEL, BIN_BSEARCH, false, true>(ctx, w, m, smem, s);
+            return bin == BIN_LUT ? launch_m<LOOK_TABLE, BIN_LUT, false, true>(ctx, w, m, smem, s)
+                                  : launch_m<LOOK_TABLE, BIN_BSEARCH, false, true>(ctx, w, m, smem, s);
+        };
+        const LaneModel* lm = learned ? &model : nullptr;
+        if (who != Counter::Warps)
+            return launch_lane_count_cells(ctx, q, p, s, lm, who == Counter::Sampled ? Warps(by_warps) : Warps());
         StreamScratch scr(s);
         int rc = list_for_warps(ctx, q, &p, RangesOf::Cells, scr, s, nullptr);
-        if (rc) return rc;
-        if (learned)
-            rc = bin == BIN_LUT ? launch_m<LOOK_MODEL, BIN_LUT, false, true>(ctx, p, m, smem, s)
-                                : launch_m<LOOK_MODEL, BIN_BSEARCH, false, true>(ctx, p, m, smem, s);
-        else
-            rc = bin == BIN_LUT ? launch_m<LOOK_TABLE, BIN_LUT, false, true>(ctx, p, m, smem, s)
-                                : launch_m<LOOK_TABLE, BIN_BSEARCH, false, true>(ctx, p, m, smem, s);
-        return rc ? rc : launch_listed_images(ctx, q, p, RangesOf::Cells, s, nullptr, learned ? &model : nullptr);
+        if (!rc) rc = by_warps(p);
+        return rc ? rc : launch_listed_images(ctx, q, p, RangesOf::Cells, s, nullptr, lm);
     }
     // Learned kind: model lookups, unless the judge recorded a mismatch (the
     // kernel reads the record and then answers from the table).

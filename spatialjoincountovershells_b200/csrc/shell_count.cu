@@ -380,7 +380,10 @@ template <int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count(CountParams p) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if constexpr (LIST) clear_next_list(p);
+    if constexpr (LIST) {
+        if (p.gate && *p.gate == 0u) return;
+        clear_next_list(p);
+    }
     const SmemView v = setup_smem<BIG>(p, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * CT_WARPS;
@@ -398,7 +401,10 @@ template <int BIN, bool BIG, bool LIST>
 __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_multi(CountParams p) {
     extern __shared__ uint32_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if constexpr (LIST) clear_next_list(p);
+    if constexpr (LIST) {
+        if (p.gate && *p.gate == 0u) return;
+        clear_next_list(p);
+    }
     const SmemView v = setup_smem<BIG>(p, smem, tid, warp);
     __syncthreads();
     const uint64_t W = (uint64_t)gridDim.x * CT_WARPS;
@@ -616,14 +622,17 @@ int launch_static(sjcs_ctx* ctx, const CountParams& p, int bin, bool big, size_t
 namespace {
 int launch_lanes_or_warps(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,
                           const LaneScratch* given) {
-    if (!warps_count_sooner(ctx, p)) return launch_lane_count(ctx, q, p, s, given);
+    auto by_warps = [&](const CountParams& w) {
+        return bin_mode(q) == BIN_LUT ? launch_variant<BIN_LUT, false, true>(ctx, w, count_smem(q), s, w.nidx > 1)
+                                      : launch_variant<BIN_BSEARCH, false, true>(ctx, w, count_smem(q), s, w.nidx > 1);
+    };
+    const Counter who = who_counts(ctx, p, RangesOf::Rows);
+    if (who != Counter::Warps)
+        return launch_lane_count(ctx, q, p, s, given, who == Counter::Sampled ? Warps(by_warps) : Warps());
     CountParams w = p;
     StreamScratch scr(s);
     int rc = list_for_warps(ctx, q, &w, RangesOf::Rows, scr, s, given);
-    if (rc) return rc;
-    const bool multi = p.nidx > 1;
-    rc = bin_mode(q) == BIN_LUT ? launch_variant<BIN_LUT, false, true>(ctx, w, count_smem(q), s, multi)
-                                : launch_variant<BIN_BSEARCH, false, true>(ctx, w, count_smem(q), s, multi);
+    if (!rc) rc = by_warps(w);
     return rc ? rc : launch_listed_images(ctx, q, w, RangesOf::Rows, s, given, nullptr);
 }
 }  // namespace

@@ -317,8 +317,9 @@ int query_prepare(sjcs_ctx* ctx, const float* d_halo_xyz, size_t stride, uint64_
     q->lane.slots = reinterpret_cast<uint32_t*>(q->d_r2) + pad + lut.size();
     const uint64_t ncnt = nhalos * (uint64_t)nrads;
     const uint64_t padded = (ncnt + 3) & ~3ull;  // the list behind the counts starts aligned
-    SJCS_CUDA_TRY(cudaMallocAsync(&q->counts, padded * sizeof(uint32_t) + kQueryListBytes, s));
-    SJCS_CUDA_TRY(cudaMemsetAsync(q->counts, 0, padded * sizeof(uint32_t) + 2 * 8 * sizeof(uint32_t), s));
+    q->list_items = count_by_warps_items(ctx, nhalos);
+    SJCS_CUDA_TRY(cudaMallocAsync(&q->counts, padded * sizeof(uint32_t) + count_by_warps_bytes(q->list_items), s));
+    SJCS_CUDA_TRY(cudaMemsetAsync(q->counts, 0, padded * sizeof(uint32_t) + count_by_warps_bytes(0), s));
     q->list_ctl = q->counts + padded;
     q->list_turn = 0;
     SJCS_CUDA_TRY(cudaMallocAsync(&q->halos, (nhalos ? nhalos : 1) * sizeof(float4), s));

@@ -166,11 +166,6 @@ struct sjcs_index {
     bool had_h2d;
 };
 
-namespace sjcs {
-constexpr uint32_t kQueryListItems = 16384;
-constexpr size_t kQueryListBytes = 2 * 8 * sizeof(uint32_t) + kQueryListItems * sizeof(uint2);
-}  // namespace sjcs
-
 struct sjcs_query {
     uint32_t magic;
     sjcs_ctx* ctx;
@@ -188,6 +183,7 @@ struct sjcs_query {
     // that give a warp to each halo (shell_count.cu, morton_count.cu).  A count
     // takes the sets in turn and clears the other one.
     uint32_t* list_ctl;
+    uint32_t list_items;  // even; 0: such counts do not occur
     mutable uint32_t list_turn;
     float* d_r2;        // [pad], entries past nrads = +inf
     // Shell lookup on the bit pattern of dist (non-negative floats order like
@@ -262,6 +258,10 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
 // zeroed accumulators, Morton-sorted halos) and schedule resolution
 int query_prepare(sjcs_ctx* ctx, const float* d_halo_xyz, size_t stride, uint64_t nhalos, const float* r2,
                   int nrads, int flags, sjcs_query* q, cudaStream_t s);
+// Counts that give a warp to each halo (lane_count.cu): items of a query's list,
+// and the bytes that the list takes with its control words.
+uint32_t count_by_warps_items(const sjcs_ctx* ctx, uint64_t nhalos);
+constexpr size_t count_by_warps_bytes(uint32_t items) { return 2 * 8 * sizeof(uint32_t) + items * sizeof(uint2); }
 // Slots of the lane-per-halo count for a non-decreasing table (sjcs_abi.cu);
 // leaves t->nslots 0 when the table does not fit the form.
 void build_lane_table(const float* r2, int nrads, float half, std::vector<uint32_t>* slots, sjcs_query::LaneTable* t);

@@ -99,11 +99,11 @@ def test_many_halos_on_cells_of_any_level(ctx, kind, level):
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("data", ["uniform", "clumps", "few clumps"])
 @pytest.mark.parametrize("files", [1, 3])
-@pytest.mark.parametrize("m", [3000])
+@pytest.mark.parametrize("m", [3000, 24100])
 def test_full_boxes(ctx, kind, data, files, m):
-    """Boxes of many rows of many candidates, clumps around most halos or around
-    3 % of them: images listed from a later part of their box on, in short rows
-    and long ones."""
+    """More candidates to an ordinary box than a lane walks: of many halos a
+    sample tells whether lanes or warps count them (clumps around most halos, or
+    around 3 % of them).  Images listed from a later part of their box on."""
     rng = np.random.default_rng(1550)
     n, radius = 40000, 120.0
     ps = [rng.uniform(0, 1000, (n, 3)) for _ in range(files)]
