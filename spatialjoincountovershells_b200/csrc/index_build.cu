@@ -184,6 +184,20 @@ __device__ __forceinline__ uint32_t pb_block_scan(uint32_t v, uint32_t* ws, uint
 
 __device__ __forceinline__ uint32_t pb_key(const float4& r) { return __float_as_uint(r.w); }
 
+// One from counter lk of a group's cells for every lane (none, ~0: lk out of
+// range); a warp whose lanes all want the same counter asks for it once.
+__device__ __forceinline__ uint32_t pb_take(uint32_t* __restrict__ hist, uint32_t lk) {
+    const uint32_t first = __shfl_sync(0xffffffffu, lk, 0);
+    if (__all_sync(0xffffffffu, lk == first)) {
+        if (first >= PB_GROUP_CELLS) return 0xffffffffu;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&hist[first], 32u);
+        return __shfl_sync(0xffffffffu, at, 0) + lane;
+    }
+    return lk < PB_GROUP_CELLS ? atomicAdd(&hist[lk], 1u) : 0xffffffffu;
+}
+
 // Cell key of a particle: the grid's cell number, or the level-L Morton code.
 struct GridKey {
     GridGeom g;
@@ -419,14 +433,42 @@ k_pb_partition(const float* __restrict__ xyz, int xyz_aligned, const float4* __r
     }
 }
 
+// Groups of the last pass with so many records that one block would be busy
+// with them long after the others are listed and shared by all blocks.  A block
+// moves about one record a nanosecond and all of them 130 (5e6 equal particles
+// took 5.2 ms and take 0.19; 2e7, half of them in a clump of sigma 2, 9.6 and
+// 0.71 ms by Morton cells), so a group counts as dense from n / 128 on; listing
+// from 32768 on cost 5e7 clustered particles 12 %.
+struct PbDense {
+    uint32_t* n;      // groups listed (zeroed)
+    uint32_t* group;  // [pb_dense_slots]
+    uint32_t* done;   // [pb_dense_slots] pieces counted
+    uint32_t* cur;    // [pb_dense_slots][PB_GROUP_CELLS] counts, then where the next record goes
+};
+constexpr uint32_t kPbPiece = 4 * PB_TILE;  // records of a piece
+
+// Records from which on a group is dense, and how many groups can be.
+__host__ __device__ constexpr uint32_t pb_dense(uint64_t n) {
+    return n / 128 > 8 * PB_TILE ? (uint32_t)(n / 128) : 8 * PB_TILE;
+}
+__host__ __device__ constexpr uint32_t pb_dense_slots(uint64_t n) { return (uint32_t)(n / pb_dense(n)); }
+// Words of PbDense for n particles, without the count.
+constexpr uint64_t pb_dense_words(uint64_t n) { return (uint64_t)pb_dense_slots(n) * (PB_GROUP_CELLS + 2); }
+PbDense pb_dense_at(uint32_t* n, uint32_t* words, uint64_t particles) {
+    const uint32_t k = pb_dense_slots(particles);
+    return {n, words, words + k, words + 2 * (uint64_t)k};
+}
+
 // Last pass: block b counting-sorts the records of cells [4096 b, 4096 b +
 // 4096) (whole segments of 2^sb cells, contiguous after the partition passes)
 // and writes cell_start for those of its cells that are <= ncells.  A group
 // of at most PB_TILE records goes through shared memory; a larger one is read
-// twice (counts, then placement) and written in place.
+// twice (counts, then placement) and written in place, or left to the passes
+// over dense groups.
 __global__ void __launch_bounds__(PB_THREADS, 2)
 k_pb_cells(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start, uint64_t nseg, int sb,
-           uint64_t ncells, uint32_t* __restrict__ cs, float4* __restrict__ out) {
+           uint64_t ncells, uint32_t* __restrict__ cs, float4* __restrict__ out, PbDense dense, uint32_t slots,
+           uint32_t limit) {
     __shared__ __align__(16) uint32_t hist[PB_GROUP_CELLS];
     __shared__ uint32_t ws[PB_THREADS / 32 + 1];
     extern __shared__ float4 xch[];
@@ -437,6 +479,20 @@ k_pb_cells(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start
     const uint64_t seg1 = min(seg0 + (PB_GROUP_CELLS >> sb), nseg);
     const uint32_t lo = seg_start[seg0], cnt = seg_start[seg1] - lo;
     const uint32_t c0 = (uint32_t)cell0;
+    if (cnt > limit && slots) {
+        if (tid == 0) ws[0] = atomicAdd(dense.n, 1u);
+        __syncthreads();
+        const uint32_t slot = ws[0];
+        if (slot < slots) {
+            if (tid == 0) {
+                dense.group[slot] = blockIdx.x;
+                dense.done[slot] = 0u;
+            }
+            for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS)
+                dense.cur[(uint64_t)slot * PB_GROUP_CELLS + c] = 0u;
+            return;
+        }
+    }
     uint4* h4 = reinterpret_cast<uint4*>(hist);
     h4[2 * tid] = make_uint4(0u, 0u, 0u, 0u);
     h4[2 * tid + 1] = make_uint4(0u, 0u, 0u, 0u);
@@ -518,6 +574,149 @@ k_pb_cells(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start
     }
 }
 
+// A piece of a dense group: its place in the list, records and first cell.
+struct PbPiece {
+    uint32_t slot, lo, cnt, c0, pieces, start, len;
+};
+// Piece `at` of all listed groups; false: there are fewer.
+__device__ __forceinline__ bool pb_piece(const PbDense& dense, uint32_t nd, const uint32_t* __restrict__ seg_start,
+                                         uint64_t nseg, int sb, uint32_t at, PbPiece* p) {
+    for (uint32_t k = 0; k < nd; ++k) {
+        const uint64_t cell0 = (uint64_t)dense.group[k] * PB_GROUP_CELLS, seg0 = cell0 >> sb;
+        const uint32_t lo = seg_start[seg0];
+        const uint32_t cnt = seg_start[min(seg0 + (PB_GROUP_CELLS >> sb), nseg)] - lo;
+        const uint32_t pieces = (cnt + kPbPiece - 1u) / kPbPiece;
+        if (at < pieces) {
+            *p = {k, lo, cnt, (uint32_t)cell0, pieces, at * kPbPiece, min(kPbPiece, cnt - at * kPbPiece)};
+            return true;
+        }
+        at -= pieces;
+    }
+    return false;
+}
+
+// Counts per cell of the dense groups, a piece to a block; the last block of a
+// group turns them into cell_start and the cursors that begin there.
+__global__ void __launch_bounds__(PB_THREADS, 2)
+k_pb_dense_count(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start, uint64_t nseg, int sb,
+                 uint64_t ncells, uint32_t* __restrict__ cs, PbDense dense, uint32_t slots) {
+    __shared__ uint32_t hist[PB_GROUP_CELLS];
+    __shared__ uint32_t ws[PB_THREADS / 32 + 1];
+    __shared__ uint32_t last;
+    const int tid = threadIdx.x;
+    cudaGridDependencySynchronize();
+    const uint32_t nd = min(*dense.n, slots);
+    PbPiece p;
+    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, at, &p); at += gridDim.x) {
+        uint32_t* cur = dense.cur + (uint64_t)p.slot * PB_GROUP_CELLS;
+        for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS) hist[c] = 0u;
+        __syncthreads();
+        for (uint32_t j0 = 0; j0 < p.len; j0 += PB_TILE) {
+            uint32_t lk[PB_ITEMS];
+#pragma unroll
+            for (int i = 0; i < PB_ITEMS; ++i) {
+                const uint32_t j = j0 + (uint32_t)i * PB_THREADS + (uint32_t)tid;
+                lk[i] = j < p.len ? pb_key(in[p.lo + p.start + j]) - p.c0 : 0xffffffffu;
+            }
+#pragma unroll
+            for (int i = 0; i < PB_ITEMS; ++i) pb_take(hist, lk[i]);
+        }
+        __syncthreads();
+        for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS)
+            if (hist[c]) atomicAdd(cur + c, hist[c]);
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last = atomicAdd(dense.done + p.slot, 1u) == p.pieces - 1u ? 1u : 0u;
+        __syncthreads();
+        if (!last) continue;  // the whole block
+        __threadfence();
+        uint32_t e[8], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            e[k] = sum;
+            sum += __ldcg(cur + 8u * (uint32_t)tid + k);
+        }
+        uint32_t total;
+        const uint32_t base = pb_block_scan(sum, ws, &total) + p.lo;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t c = 8u * (uint32_t)tid + k;
+            cur[c] = base + e[k];
+            if ((uint64_t)p.c0 + c <= ncells) cs[p.c0 + c] = base + e[k];
+        }
+        __syncthreads();
+    }
+}
+
+// The records of the dense groups to their cells: a tile's ranks from counters
+// in shared memory, room for each of its cells from the group's cursors.
+__global__ void __launch_bounds__(PB_THREADS, 2)
+k_pb_dense_place(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start, uint64_t nseg, int sb,
+                 float4* __restrict__ out, PbDense dense, uint32_t slots) {
+    __shared__ uint32_t hist[PB_GROUP_CELLS];
+    const int tid = threadIdx.x;
+    cudaGridDependencySynchronize();
+    const uint32_t nd = min(*dense.n, slots);
+    PbPiece p;
+    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, at, &p); at += gridDim.x) {
+        uint32_t* cur = dense.cur + (uint64_t)p.slot * PB_GROUP_CELLS;
+        for (uint32_t j0 = 0; j0 < p.len; j0 += PB_TILE) {
+            for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS) hist[c] = 0u;
+            __syncthreads();
+            float4 v[PB_ITEMS];
+            uint32_t lk[PB_ITEMS], r[PB_ITEMS];
+#pragma unroll
+            for (int i = 0; i < PB_ITEMS; ++i) {
+                const uint32_t j = j0 + (uint32_t)i * PB_THREADS + (uint32_t)tid;
+                if (j < p.len) v[i] = in[p.lo + p.start + j];
+                lk[i] = j < p.len ? pb_key(v[i]) - p.c0 : 0xffffffffu;
+            }
+#pragma unroll
+            for (int i = 0; i < PB_ITEMS; ++i) r[i] = pb_take(hist, lk[i]);
+            __syncthreads();
+            for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS) {
+                const uint32_t k = hist[c];
+                if (k) hist[c] = atomicAdd(cur + c, k);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < PB_ITEMS; ++i) {
+                if (r[i] == 0xffffffffu) continue;
+                const uint32_t o = hist[lk[i]] + r[i];
+                if (o - p.lo < p.cnt) out[o] = v[i];  // in range unless the input changed after the histogram
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// The last pass and, where a group may be dense, the passes over those.
+int launch_cells(const float4* tmp, const uint32_t* seg, uint64_t nseg, int sb, uint64_t n, uint64_t ncells, uint32_t* cs,
+                 float4* pts, const PbDense& dense, int num_sms, cudaStream_t s) {
+    const unsigned ngroups = (unsigned)(ncells / PB_GROUP_CELLS + 1);  // the last one holds cell_start[ncells]
+    const uint32_t slots = pb_dense_slots(n);
+    k_pb_cells<<<ngroups, PB_THREADS, PB_SMEM, s>>>(tmp, seg, nseg, sb, ncells, cs, pts, dense, slots,
+                                                    pb_dense(n));
+    SJCS_LAUNCH_CHECK();
+    if (!slots) return SJCS_OK;
+    const unsigned blocks = (unsigned)std::min<uint64_t>(2 * (uint64_t)num_sms, (n + kPbPiece - 1) / kPbPiece);
+    // launched while the kernel before drains: idle, they cost 3 us each without
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(PB_THREADS);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_count, tmp, seg, nseg, sb, ncells, cs, dense, slots));
+    SJCS_LAUNCH_CHECK();
+    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_place, tmp, seg, nseg, sb, pts, dense, slots));
+    SJCS_LAUNCH_CHECK();
+    return SJCS_OK;
+}
+
 // Segment bits of a key, <= PB_GROUP_BITS.  Keys of up to 21 bits take
 // segments wide enough for one digit above them: one partition pass instead
 // of two.
@@ -540,8 +739,8 @@ int set_partition_smem() {
 // The partition build into pts (n records) and cs (ncells + 1 entries) by a
 // cell key of kb <= 30 bits.
 template <class Key>
-int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t ncells, float4* pts, uint32_t* cs,
-                      cudaStream_t s) {
+int build_partitioned(int num_sms, const float* d_xyz, uint64_t n, Key key, int kb, uint64_t ncells, float4* pts,
+                      uint32_t* cs, cudaStream_t s) {
     if (n == 0) {
         SJCS_CUDA_TRY(cudaMemsetAsync(cs, 0, (ncells + 1) * sizeof(uint32_t), s));
         return SJCS_OK;
@@ -554,7 +753,6 @@ int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t 
     const uint32_t ntop = (uint32_t)((nseg + (1ull << bits_mid) - 1) >> bits_mid);
     const uint64_t ntiles_in = (n + PB_TILE - 1) / PB_TILE;
     const uint64_t ntiles_mid = ntiles_in + ntop;  // bound on the middle pass's tiles
-    const uint64_t ngroups = ncells / PB_GROUP_CELLS + 1;  // the last one holds cell_start[ncells]
     const int aligned = (reinterpret_cast<uintptr_t>(d_xyz) & 15u) == 0;
 
     StreamScratch scr(s);
@@ -563,8 +761,9 @@ int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t 
     PbTile* tiles = nullptr;
     uint16_t* mid = nullptr;
     // top digit counts and starts (ntop + 1 entries); without a middle pass
-    // the top digit is the segment and these are the segment starts too
-    SJCS_CUDA_TRY(scr.alloc(&top, ((uint64_t)ntop + 1) * sizeof(uint32_t)));
+    // the top digit is the segment and these are the segment starts too.  The
+    // word behind them counts the dense groups, whose room follows.
+    SJCS_CUDA_TRY(scr.alloc(&top, ((uint64_t)ntop + 2 + pb_dense_words(n)) * sizeof(uint32_t)));
     SJCS_CUDA_TRY(scr.alloc(&cur_top, ((uint64_t)ntop + 1) * sizeof(uint32_t)));
     SJCS_CUDA_TRY(scr.alloc(&tmp, n * sizeof(float4)));
     if (bits_mid) {
@@ -580,9 +779,9 @@ int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t 
     const int top_shift = sb + bits_mid;
     int rc = set_partition_smem<Key>();
     if (rc) return rc;
-    SJCS_CUDA_TRY(cudaMemsetAsync(top, 0, ((uint64_t)ntop + 1) * sizeof(uint32_t), s));
+    SJCS_CUDA_TRY(cudaMemsetAsync(top, 0, ((uint64_t)ntop + 2) * sizeof(uint32_t), s));
     // four tiles a block once every SM has blocks enough
-    const uint32_t per = ntiles_in >= 148ull * 4 * PB_TOP_TILES ? PB_TOP_TILES : 1u;
+    const uint32_t per = ntiles_in >= (uint64_t)num_sms * 4 * PB_TOP_TILES ? PB_TOP_TILES : 1u;
     k_pb_top_hist<Key><<<(unsigned)((ntiles_in + per - 1) / per), PB_THREADS, PB_STAGE_SMEM, s>>>(d_xyz, aligned, n, key,
                                                                                           top_shift, top, per);
     SJCS_LAUNCH_CHECK();
@@ -608,14 +807,16 @@ int build_partitioned(const float* d_xyz, uint64_t n, Key key, int kb, uint64_t 
             nullptr, 0, pts, tiles, ntiles, n, key, sb, bits_mid, bits_mid, cur_seg, tmp, nullptr, sb, 0u);
         SJCS_LAUNCH_CHECK();
     }
-    k_pb_cells<<<(unsigned)ngroups, PB_THREADS, PB_SMEM, s>>>(tmp, seg, nseg, sb, ncells, cs, pts);
-    SJCS_LAUNCH_CHECK();
-    return SJCS_OK;
+    return launch_cells(tmp, seg, nseg, sb, n, ncells, cs, pts, pb_dense_at(top + ntop + 1, top + ntop + 2, n), num_sms,
+                        s);
 }
 
 }  // namespace
 
-int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s) {
+int build_grid_into(int num_sms, const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b,
+                    cudaStream_t s) {
+    static_assert(pb_dense_words(SJCS_NOALLOC_MAX_PARTICLES) <= kGridDenseWords, "room for the dense groups");
+    if (pb_dense_words(n) > kGridDenseWords) return fail(SJCS_ERR_INVALID, "too many particles for the fixed buffers");
     if (n == 0) {
         SJCS_CUDA_TRY(cudaMemsetAsync(b.cell_start, 0, (g.ncells + 1) * sizeof(uint32_t), s));
         return SJCS_OK;
@@ -638,10 +839,8 @@ int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const Gri
                                                                         sb, bits_top, 0, b.cursors, b.tmp, nullptr, sb,
                                                                         0u);
     SJCS_LAUNCH_CHECK();
-    k_pb_cells<<<(unsigned)(g.ncells / PB_GROUP_CELLS + 1), PB_THREADS, PB_SMEM, s>>>(b.tmp, b.top, nseg, sb, g.ncells,
-                                                                                      b.cell_start, b.pts);
-    SJCS_LAUNCH_CHECK();
-    return SJCS_OK;
+    return launch_cells(b.tmp, b.top, nseg, sb, n, g.ncells, b.cell_start, b.pts, pb_dense_at(b.top + 513, b.dense, n),
+                        num_sms, s);
 }
 
 GridGeom auto_grid(uint64_t n, float radius_hint, const uint32_t* grid_req) {
@@ -722,21 +921,21 @@ int fill_cell_table(const uint32_t* sorted_cells, uint64_t n, uint64_t ncells, u
     return SJCS_OK;
 }
 
-int build_morton_table(const float* d_xyz, uint64_t n, int level, float4* pts, uint32_t* table, cudaStream_t s) {
+int build_morton_table(int num_sms, const float* d_xyz, uint64_t n, int level, float4* pts, uint32_t* table,
+                       cudaStream_t s) {
     const int G = 1 << level;
-    return build_partitioned(d_xyz, n, MortonKey{(float)G / 1000.0f, G}, std::max(1, 3 * level), 1ull << (3 * level),
+    return build_partitioned(num_sms, d_xyz, n, MortonKey{(float)G / 1000.0f, G}, std::max(1, 3 * level), 1ull << (3 * level),
                              pts, table, s);
 }
 
 int build_grid_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, const GridGeom& g,
                      sjcs_index* idx, cudaStream_t s) {
-    (void)ctx;
     idx->geom = g;
     const uint64_t nalloc = n ? n : 1;
     SJCS_CUDA_TRY(cudaMallocAsync(&idx->pts, nalloc * sizeof(float4), s));
     SJCS_CUDA_TRY(cudaMallocAsync(&idx->cell_start, (g.ncells + 1) * sizeof(uint32_t), s));
     if (grid_key_bits(g) <= PB_MAX_KEY_BITS)
-        return build_partitioned(d_xyz, n, GridKey{g}, grid_key_bits(g), g.ncells, idx->pts, idx->cell_start, s);
+        return build_partitioned(ctx->num_sms, d_xyz, n, GridKey{g}, grid_key_bits(g), g.ncells, idx->pts, idx->cell_start, s);
 
     LsdBuffers b{};
     b.pts = idx->pts;

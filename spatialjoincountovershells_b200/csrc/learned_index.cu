@@ -266,7 +266,6 @@ int morton_auto_level(uint64_t n, float radius_hint, bool learned) {
 
 int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level, bool learned, bool verify,
                        sjcs_index* idx, cudaStream_t s) {
-    (void)ctx;
     idx->level = level;
     idx->verify = learned && verify;
     for (int a = 0; a < 3; ++a) {
@@ -294,7 +293,7 @@ int build_morton_index(sjcs_ctx* ctx, const float* d_xyz, uint64_t n, int level,
     // level-L code (three streaming passes or fewer) instead of eight sort
     // passes (2e7 particles: 2.3 -> 0.4 ms).
     if (!learned) {
-        const int rc = build_morton_table(d_xyz, n, level, idx->pts, idx->cell_start, s);
+        const int rc = build_morton_table(ctx->num_sms, d_xyz, n, level, idx->pts, idx->cell_start, s);
         if (rc) return rc;
         cudaEventRecord(idx->ev_train0, s);
         return SJCS_OK;

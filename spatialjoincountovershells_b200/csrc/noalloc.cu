@@ -46,13 +46,14 @@ constexpr uint64_t kOffPts = 0;
 constexpr uint64_t kOffCells = align256(kOffPts + kNP * 16);
 constexpr uint64_t kOffTmp = align256(kOffCells + (kNC + 1) * 4);
 constexpr uint64_t kOffTop = align256(kOffTmp + kNP * 16);
-constexpr uint64_t kOffCursors = align256(kOffTop + 513 * 4);
+constexpr uint64_t kOffCursors = align256(kOffTop + 514 * 4);
 constexpr uint64_t kOffHalos = align256(kOffCursors + 513 * 4);
 constexpr uint64_t kOffR2 = align256(kOffHalos + kNH * 16);
 constexpr uint64_t kOffSlots = align256(kOffR2 + (uint64_t)kNR * 4);
 constexpr uint64_t kOffCtl = align256(kOffSlots + (uint64_t)kMaxTable * 4);
 constexpr uint64_t kOffList = align256(kOffCtl + (uint64_t)kLaneCtlWords * 4);
-constexpr uint64_t kScratchBytes = align256(kOffList + (uint64_t)kListItems * 8);
+constexpr uint64_t kOffDense = align256(kOffList + (uint64_t)kListItems * 8);
+constexpr uint64_t kScratchBytes = align256(kOffDense + kGridDenseWords * 4);
 static_assert(kScratchBytes <= SJCS_NOALLOC_SCRATCH_BYTES, "the scratch array holds every buffer");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[SJCS_NOALLOC_SCRATCH_BYTES];
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(256) k_noalloc_prep(const __grid_constant__ Ta
     if (blockIdx.x == 0) {
         for (int k = threadIdx.x; k < pad; k += blockDim.x) r2[k] = t.r2.v[k];
         for (int k = threadIdx.x; k < nslots; k += blockDim.x) slots[k] = t.slots[k];
-        for (int k = threadIdx.x; k < 513; k += blockDim.x) top[k] = 0u;
+        for (int k = threadIdx.x; k < 514; k += blockDim.x) top[k] = 0u;
         if (threadIdx.x < kLaneCtlWords) ctl[threadIdx.x] = 0u;
     }
     if (i < nh) {
@@ -301,11 +302,12 @@ extern "C" int sjcs_count_noalloc(const float* d_xyz, uint64_t n, const float* d
     b.tmp = reinterpret_cast<float4*>(base + kOffTmp);
     b.top = reinterpret_cast<uint32_t*>(base + kOffTop);
     b.cursors = reinterpret_cast<uint32_t*>(base + kOffCursors);
+    b.dense = reinterpret_cast<uint32_t*>(base + kOffDense);
     k_noalloc_prep<<<(unsigned)((nhalos + 255) / 256), 256, 0, s>>>(
         tab, pad, q.lane.nslots, reinterpret_cast<const char*>(d_halo_xyz), stride_bytes, nhalos, q.d_r2, q.lane.slots,
         b.top, list.ctl, q.halos);
     SJCS_LAUNCH_CHECK();
-    rc = build_grid_into(d_xyz, n, g, b, s);
+    rc = build_grid_into(c.num_sms, d_xyz, n, g, b, s);
     if (rc) return rc;
 
     sjcs_index idx{};

@@ -319,14 +319,18 @@ struct GridBuildBuffers {
     float4* pts;           // n particles grouped by cell (output)
     uint32_t* cell_start;  // ncells + 1 (output)
     float4* tmp;           // n records
-    uint32_t* top;         // 513, zeroed
+    uint32_t* top;         // 514, zeroed
     uint32_t* cursors;     // 513
+    uint32_t* dense;       // kGridDenseWords
 };
+constexpr uint64_t kGridDenseWords = 4 * (4096 + 2);
 constexpr int kGridMaxDirectBits = 21;
-int build_grid_into(const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b, cudaStream_t s);
+int build_grid_into(int num_sms, const float* d_xyz, uint64_t n, const GridGeom& g, const GridBuildBuffers& b,
+                    cudaStream_t s);
 // Particles grouped by level-L Morton cell (in code order, any order inside a
 // cell; 4th word = the code) and the offset table of 8^L + 1 entries.
-int build_morton_table(const float* d_xyz, uint64_t n, int level, float4* pts, uint32_t* table, cudaStream_t s);
+int build_morton_table(int num_sms, const float* d_xyz, uint64_t n, int level, float4* pts, uint32_t* table,
+                       cudaStream_t s);
 constexpr uint32_t kGridGaps = 1u << 16;
 int grid_key_bits(const GridGeom& g);
 // cell_start[c] = first slot of cell c, from the cell ids of the sorted particles.
