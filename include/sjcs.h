@@ -445,7 +445,9 @@ int sjcs_query_get_schedule(const sjcs_query *q, sjcs_schedule *out);
  * two, largest radius, shells, periodicity), where SJCS_SCHED_AUTO finds it.
  * The query's counts are left as they were.  Blocks; trial_ms[i] (up to
  * max_trials entries, may be NULL) receives each trial's kernel time in the
- * order above and *ntrials their number. */
+ * order above and *ntrials their number.  Tables for which every schedule runs
+ * the same kernels (above) are timed once: every entry is that time, and the
+ * static schedule is kept. */
 int sjcs_autotune(sjcs_ctx *ctx, sjcs_query *q, const sjcs_index *idx, sjcs_schedule *chosen,
                   float *trial_ms, int max_trials, int *ntrials);
 

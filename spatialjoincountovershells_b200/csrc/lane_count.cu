@@ -1178,6 +1178,15 @@ bool lane_count_applies(const sjcs_query* q, const CountParams& p) {
     return true;
 }
 
+bool ignores_schedule(const sjcs_query* q, const sjcs_index* idx) {
+    CountParams p{};
+    p.prune = q->monotone && std::isfinite(q->r2max) ? 1 : 0;
+    p.nhalos = q->nhalos;
+    p.nidx = 1;
+    p.mn[0] = (uint32_t)idx->n;
+    return lane_count_applies(q, p);
+}
+
 namespace {
 // The list takes 1.5 items per halo and index.  An image is one item at most:
 // lists of up to kExactItems (16 MB), and those of counts without images, have

@@ -1454,7 +1454,16 @@ int sjcs_autotune(sjcs_ctx* ctx, sjcs_query* q, const sjcs_index* idx, sjcs_sche
     float warm = 0.0f;
     rc = run(cand[0], &warm);  // warm-up (caches, clocks, lazy module loading)
     const int reps = warm < 5.0f ? 3 : 1;
+    // tables that lanes can count: every schedule runs the same kernels, so the
+    // candidates share the static one's trial and the choice
+    const bool same = ignores_schedule(q, idx);
     for (size_t i = 0; i < cand.size() && !rc; ++i) {
+        if (same && i > 0) {
+            ms[i] = ms[0];
+            if (q->nhalos * (uint64_t)cand[i].max_pieces >= (1ull << 32))
+                rc = fail(SJCS_ERR_INVALID, "queue schedule: nhalos * max_pieces must stay below 2^32");
+            continue;
+        }
         float best = 0.0f;
         for (int r = 0; r < reps && !rc; ++r) {
             float t = 0.0f;

@@ -305,6 +305,8 @@ int launch_shell_count_multi(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_inde
 // indexes: the static schedule, or a query counted by lanes (lane_count.cu),
 // which the queue would count index by index for nothing.
 bool may_fuse(const sjcs_query* q, const sjcs_index* idx, const Schedule& sc);
+// Whether every schedule counts q on idx with the same kernels (lane_count.cu).
+bool ignores_schedule(const sjcs_query* q, const sjcs_index* idx);
 
 // scan.cu: exclusive prefix sum of m u32 values, in place.  `partials`
 // (scan_partials_needed(m) u32) may be given; otherwise it is allocated when
