@@ -1061,19 +1061,24 @@ __device__ __forceinline__ void count_items(const CountParams& p, const LanePara
 // Two neighbouring items of the list are counted together when they are two
 // centres of one index no further apart than a radius: most candidates then
 // serve both.
+template <bool BY_WARPS>
 __device__ __forceinline__ bool paired(const CountParams& p, const uint2* it, uint32_t n) {
-    constexpr uint32_t kAlone = kItemZone | kItemFar | kItemShort | ~((1u << kItemFrom) - 1u);
+    constexpr uint32_t kLater = ~((1u << kItemFrom) - 1u);  // an image's later part
+    constexpr uint32_t kAlone = kItemZone | kItemFar | kItemShort | (BY_WARPS ? kLater : 0u);
     if (n < 2u || ((it[0].y | it[1].y) & kAlone) || (((it[0].y ^ it[1].y) >> 3) & 3u)) return false;
     const float4 a = item_centre(p, it[0]), b = item_centre(p, it[1]);
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     return dx * dx + dy * dy + dz * dz <= p.r2max;
 }
 
-template <int R, int BLOCKS>
+// BY_WARPS: (also) the list of a count that gives a warp to each halo, whose
+// items may begin in a later part of their box.
+template <int R, int BLOCKS, bool BY_WARPS>
 __global__ void __launch_bounds__(HV_THREADS, BLOCKS)
 k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
-    const bool whole = q.gate && *q.gate == 0u;  // lanes counted: all room was for either kind
+    auto from = [](const uint2& it) { return BY_WARPS ? 32u * (it.y >> kItemFrom) : 0u; };
+    const bool whole = !BY_WARPS || (q.gate && *q.gate == 0u);  // lanes counted: all room was for either kind
     const uint32_t nhuge = min(q.ctl[1], whole ? q.cap : q.cap_huge);
     const uint32_t nother = min(q.ctl[2], whole ? q.cap : q.cap_other);
     if (nhuge + nother == 0u) return;
@@ -1110,14 +1115,14 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
 #pragma unroll
             for (uint32_t j = 0; j < 2u; ++j)
                 it[j] = j < n ? q.list[huge ? per * k + j : q.cap - 1u - (per * k + j)] : make_uint2(0u, 0u);
-            if (paired(p, it, n)) {
+            if (paired<BY_WARPS>(p, it, n)) {
                 if (phase == 0) count_items<R, 2, false>(p, q, it, part, nparts, cols, slots, lane);
             } else if (phase == 1) {
 #pragma unroll 1
                 for (uint32_t j = 0; j < n; ++j) {
                     const uint2 one = j ? it[1] : it[0];
                     if (!(one.y & (kItemZone | kItemFar | kItemShort)))
-                        count_items<R, 1, false>(p, q, &one, part, nparts, cols, slots, lane, 32u * (one.y >> kItemFrom));
+                        count_items<R, 1, false>(p, q, &one, part, nparts, cols, slots, lane, from(one));
                 }
             } else if (phase == 2) {
 #pragma unroll 1
@@ -1125,7 +1130,7 @@ k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ La
                     const uint2 one = j ? it[1] : it[0];
                     if (one.y & (kItemZone | kItemFar)) count_literal<R>(p, q, one, part, nparts, lane);
                     else if (one.y & kItemShort)
-                        count_items<R, 1, true>(p, q, &one, part, nparts, cols, slots, lane, 32u * (one.y >> kItemFrom));
+                        count_items<R, 1, true>(p, q, &one, part, nparts, cols, slots, lane, from(one));
                 }
             }
         }
@@ -1189,10 +1194,10 @@ bool ignores_schedule(const sjcs_query* q, const sjcs_index* idx) {
 
 namespace {
 // The list takes 1.5 items per halo and index.  An image is one item at most:
-// lists of up to kExactItems (16 MB), and those of counts without images, have
+// lists of up to kExactItems (64 MB), and those of counts without images, have
 // room for all of them and nothing is ever left (marks and an idle k_left_count
 // cost about 5 us).
-constexpr uint64_t kExactItems = 1u << 21;
+constexpr uint64_t kExactItems = 1u << 23;
 
 // List, control words and marks of a count on stream s.  A pool that cannot
 // give the whole list gives a shorter one, down to none.
@@ -1280,13 +1285,13 @@ LaneParams lane_params(const sjcs_query* qq, const CountParams& p, const LaneMod
 size_t listed_smem(const LaneParams& q) { return HV_WARPS * 2 * (size_t)(q.ncol + 1) * 64 + (size_t)q.nslots * 4; }
 
 // The items of q's list (front and end), and what was marked beside it.
-template <int R>
+template <int R, bool BY_WARPS>
 int launch_listed(sjcs_ctx* ctx, const CountParams& p, const LaneParams& q, bool noalloc, cudaStream_t s) {
     const size_t smem = listed_smem(q);
     int per_sm = 0;
-    auto listed = k_listed_count<R, HV_BLOCKS>;
+    auto listed = k_listed_count<R, HV_BLOCKS, BY_WARPS>;
     if constexpr (R == RANGE_ROWS)
-        if (noalloc) listed = k_listed_count<R, HV_BLOCKS_NOALLOC>;
+        if (noalloc) listed = k_listed_count<R, HV_BLOCKS_NOALLOC, BY_WARPS>;
     SJCS_CUDA_TRY(allow_block_smem(listed));
     SJCS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, listed, HV_THREADS, smem));
     if (per_sm < 1) per_sm = 1;
@@ -1374,7 +1379,8 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     SJCS_CUDA_TRY(allow_block_smem(k_lane_count<R, PACK>));
     k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, nw * warp_a + table, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
-    return launch_listed<R>(ctx, p, q, given != nullptr, s);
+    return warps ? launch_listed<R, true>(ctx, p, q, given != nullptr, s)
+                 : launch_listed<R, false>(ctx, p, q, given != nullptr, s);
 }
 }  // namespace
 
@@ -1397,7 +1403,11 @@ uint32_t count_by_warps_items(const sjcs_ctx* ctx, uint64_t nhalos) {
 // pays for a sample, and rows are better off with warps (1000 on 2e7, R = 20:
 // clustered 151 and 153, uniform 73 and 54), quads of the table with lanes (124
 // and 212, 107 and 75), those of the model with warps (473 and 262, 350 and 91).
-Counter who_counts(sjcs_ctx* ctx, const CountParams& p, RangesOf of) {
+// Halos in no order (sorted false, the allocation-free call's): warps that take
+// neighbours share no particle lines, so lanes from a batch per SM on (20000 on
+// 131072 at R = 40 75 us a call, 81 by warps; 130 on them 69 and 61).
+Counter who_counts(sjcs_ctx* ctx, const CountParams& p, RangesOf of, bool sorted) {
+    if (!sorted) return (p.nhalos + 31) / 32 <= (uint64_t)ctx->num_sms ? Counter::Warps : Counter::Lanes;
     const bool rows = of == RangesOf::Rows, few = few_batches(ctx, p.nhalos);
     const UniformBox b = uniform_box(p, rows);
     if (b.candidates <= (double)walk_limit(ctx, p, rows)) return few ? Counter::Warps : Counter::Lanes;
@@ -1452,8 +1462,9 @@ int launch_listed_images(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams&
     q.cap = p.list_cap;
     q.cap_huge = p.list_huge;
     q.cap_other = p.list_cap - p.list_huge;
-    if (ranges == RangesOf::Rows) return launch_listed<RANGE_ROWS>(ctx, p, q, given != nullptr, s);
-    return model ? launch_listed<RANGE_MODEL>(ctx, p, q, false, s) : launch_listed<RANGE_CELLS>(ctx, p, q, false, s);
+    if (ranges == RangesOf::Rows) return launch_listed<RANGE_ROWS, true>(ctx, p, q, given != nullptr, s);
+    return model ? launch_listed<RANGE_MODEL, true>(ctx, p, q, false, s)
+                 : launch_listed<RANGE_CELLS, true>(ctx, p, q, false, s);
 }
 
 int launch_lane_count(sjcs_ctx* ctx, const sjcs_query* q, const CountParams& p, cudaStream_t s,

@@ -49,7 +49,7 @@ int launch_lane_count_cells(sjcs_ctx* ctx, const sjcs_query* q, const count::Cou
 // `given`; under capture memory of the stream); and the count of what was listed.
 enum class RangesOf { Rows, Cells, Model };
 enum class Counter { Lanes, Warps, Sampled };
-Counter who_counts(sjcs_ctx* ctx, const count::CountParams& p, RangesOf ranges);
+Counter who_counts(sjcs_ctx* ctx, const count::CountParams& p, RangesOf ranges, bool sorted = true);
 int list_for_warps(sjcs_ctx* ctx, const sjcs_query* q, count::CountParams* p, RangesOf ranges, StreamScratch& scr,
                    cudaStream_t s, const LaneScratch* given);
 int launch_listed_images(sjcs_ctx* ctx, const sjcs_query* q, const count::CountParams& p, RangesOf ranges,

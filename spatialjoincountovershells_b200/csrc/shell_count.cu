@@ -626,7 +626,7 @@ int launch_lanes_or_warps(sjcs_ctx* ctx, const sjcs_query* q, const CountParams&
         return bin_mode(q) == BIN_LUT ? launch_variant<BIN_LUT, false, true>(ctx, w, count_smem(q), s, w.nidx > 1)
                                       : launch_variant<BIN_BSEARCH, false, true>(ctx, w, count_smem(q), s, w.nidx > 1);
     };
-    const Counter who = who_counts(ctx, p, RangesOf::Rows);
+    const Counter who = who_counts(ctx, p, RangesOf::Rows, !given);
     if (who != Counter::Warps)
         return launch_lane_count(ctx, q, p, s, given, who == Counter::Sampled ? Warps(by_warps) : Warps());
     CountParams w = p;
