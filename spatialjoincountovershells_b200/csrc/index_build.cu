@@ -437,19 +437,23 @@ k_pb_partition(const float* __restrict__ xyz, int xyz_aligned, const float4* __r
 // with them long after the others are listed and shared by all blocks.  A block
 // moves about one record a nanosecond and all of them 130 (5e6 equal particles
 // took 5.2 ms and take 0.19; 2e7, half of them in a clump of sigma 2, 9.6 and
-// 0.71 ms by Morton cells), so a group counts as dense from n / 128 on; listing
-// from 32768 on cost 5e7 clustered particles 12 %.
+// 0.71 ms by Morton cells), so a group counts as dense from about n / 100 on,
+// and 32768 more for the two passes (20 to 50 us; 2e6 clustered by Morton cells:
+// 101 us, 148 with groups from n / 128 on).
 struct PbDense {
     uint32_t* n;      // groups listed (zeroed)
     uint32_t* group;  // [pb_dense_slots]
     uint32_t* done;   // [pb_dense_slots] pieces counted
     uint32_t* cur;    // [pb_dense_slots][PB_GROUP_CELLS] counts, then where the next record goes
 };
-constexpr uint32_t kPbPiece = 4 * PB_TILE;  // records of a piece
+// Records of a piece.  Small sets need the pieces (a clump of 131072 87 us by
+// four tiles, 56 by one), a large one with many dense groups fewer counters to
+// clear and add up (5e7 clustered, R = 20 by Morton cells: 1.32 ms, 2.0 by one).
+__host__ __device__ constexpr uint32_t pb_piece_len(uint64_t n) { return n < (1u << 22) ? PB_TILE : 4 * PB_TILE; }
 
 // Records from which on a group is dense, and how many groups can be.
 __host__ __device__ constexpr uint32_t pb_dense(uint64_t n) {
-    return n / 128 > 8 * PB_TILE ? (uint32_t)(n / 128) : 8 * PB_TILE;
+    return 8 * PB_TILE + (uint32_t)(n / 100);
 }
 __host__ __device__ constexpr uint32_t pb_dense_slots(uint64_t n) { return (uint32_t)(n / pb_dense(n)); }
 // Words of PbDense for n particles, without the count.
@@ -580,14 +584,15 @@ struct PbPiece {
 };
 // Piece `at` of all listed groups; false: there are fewer.
 __device__ __forceinline__ bool pb_piece(const PbDense& dense, uint32_t nd, const uint32_t* __restrict__ seg_start,
-                                         uint64_t nseg, int sb, uint32_t at, PbPiece* p) {
+                                         uint64_t nseg, int sb, uint32_t piece, uint32_t at,
+                                         PbPiece* p) {
     for (uint32_t k = 0; k < nd; ++k) {
         const uint64_t cell0 = (uint64_t)dense.group[k] * PB_GROUP_CELLS, seg0 = cell0 >> sb;
         const uint32_t lo = seg_start[seg0];
         const uint32_t cnt = seg_start[min(seg0 + (PB_GROUP_CELLS >> sb), nseg)] - lo;
-        const uint32_t pieces = (cnt + kPbPiece - 1u) / kPbPiece;
+        const uint32_t pieces = (cnt + piece - 1u) / piece;
         if (at < pieces) {
-            *p = {k, lo, cnt, (uint32_t)cell0, pieces, at * kPbPiece, min(kPbPiece, cnt - at * kPbPiece)};
+            *p = {k, lo, cnt, (uint32_t)cell0, pieces, at * piece, min(piece, cnt - at * piece)};
             return true;
         }
         at -= pieces;
@@ -599,7 +604,8 @@ __device__ __forceinline__ bool pb_piece(const PbDense& dense, uint32_t nd, cons
 // group turns them into cell_start and the cursors that begin there.
 __global__ void __launch_bounds__(PB_THREADS, 2)
 k_pb_dense_count(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start, uint64_t nseg, int sb,
-                 uint64_t ncells, uint32_t* __restrict__ cs, PbDense dense, uint32_t slots) {
+                 uint64_t ncells, uint32_t* __restrict__ cs, PbDense dense, uint32_t slots,
+                 uint32_t piece) {
     __shared__ uint32_t hist[PB_GROUP_CELLS];
     __shared__ uint32_t ws[PB_THREADS / 32 + 1];
     __shared__ uint32_t last;
@@ -607,7 +613,7 @@ k_pb_dense_count(const float4* __restrict__ in, const uint32_t* __restrict__ seg
     cudaGridDependencySynchronize();
     const uint32_t nd = min(*dense.n, slots);
     PbPiece p;
-    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, at, &p); at += gridDim.x) {
+    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, piece, at, &p); at += gridDim.x) {
         uint32_t* cur = dense.cur + (uint64_t)p.slot * PB_GROUP_CELLS;
         for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS) hist[c] = 0u;
         __syncthreads();
@@ -652,13 +658,13 @@ k_pb_dense_count(const float4* __restrict__ in, const uint32_t* __restrict__ seg
 // in shared memory, room for each of its cells from the group's cursors.
 __global__ void __launch_bounds__(PB_THREADS, 2)
 k_pb_dense_place(const float4* __restrict__ in, const uint32_t* __restrict__ seg_start, uint64_t nseg, int sb,
-                 float4* __restrict__ out, PbDense dense, uint32_t slots) {
+                 float4* __restrict__ out, PbDense dense, uint32_t slots, uint32_t piece) {
     __shared__ uint32_t hist[PB_GROUP_CELLS];
     const int tid = threadIdx.x;
     cudaGridDependencySynchronize();
     const uint32_t nd = min(*dense.n, slots);
     PbPiece p;
-    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, at, &p); at += gridDim.x) {
+    for (uint32_t at = blockIdx.x; nd && pb_piece(dense, nd, seg_start, nseg, sb, piece, at, &p); at += gridDim.x) {
         uint32_t* cur = dense.cur + (uint64_t)p.slot * PB_GROUP_CELLS;
         for (uint32_t j0 = 0; j0 < p.len; j0 += PB_TILE) {
             for (uint32_t c = (uint32_t)tid; c < PB_GROUP_CELLS; c += PB_THREADS) hist[c] = 0u;
@@ -699,7 +705,8 @@ int launch_cells(const float4* tmp, const uint32_t* seg, uint64_t nseg, int sb, 
                                                     pb_dense(n));
     SJCS_LAUNCH_CHECK();
     if (!slots) return SJCS_OK;
-    const unsigned blocks = (unsigned)std::min<uint64_t>(2 * (uint64_t)num_sms, (n + kPbPiece - 1) / kPbPiece);
+    const uint32_t piece = pb_piece_len(n);
+    const unsigned blocks = (unsigned)std::min<uint64_t>(2 * (uint64_t)num_sms, (n + piece - 1) / piece);
     // launched while the kernel before drains: idle, they cost 3 us each without
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -710,9 +717,9 @@ int launch_cells(const float4* tmp, const uint32_t* seg, uint64_t nseg, int sb, 
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_count, tmp, seg, nseg, sb, ncells, cs, dense, slots));
+    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_count, tmp, seg, nseg, sb, ncells, cs, dense, slots, piece));
     SJCS_LAUNCH_CHECK();
-    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_place, tmp, seg, nseg, sb, pts, dense, slots));
+    SJCS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pb_dense_place, tmp, seg, nseg, sb, pts, dense, slots, piece));
     SJCS_LAUNCH_CHECK();
     return SJCS_OK;
 }

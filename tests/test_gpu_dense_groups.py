@@ -1,6 +1,6 @@
 """Index builds whose particles crowd into few cells: groups of 4096 cells with
-more records than one block takes (32768 or a 128th of all, the edge; several
-groups; all in one cell), grid and Morton table, and the allocation-free call.  Counts are integers and must equal
+more records than one block takes (32768 and a 100th of all, the edge; several
+groups; all in one cell; pieces of one and of four tiles), grid and Morton table, and the allocation-free call.  Counts are integers and must equal
 the oracle's."""
 from __future__ import annotations
 
@@ -31,8 +31,8 @@ def _crowd(rng, data, n):
 
 
 @pytest.mark.parametrize("kind", [nat.INDEX_GRID, nat.INDEX_MORTON])
-@pytest.mark.parametrize("data,n", [("equal", 32767), ("equal", 32768), ("equal", 32769), ("equal", 1000003), ("cells", 400001),
-                                    ("half", 300007), ("half", 3000001), ("many groups", 4000000)])
+@pytest.mark.parametrize("data,n", [("equal", 32767), ("equal", 32768), ("equal", 33099), ("equal", 33100), ("equal", 1000003), ("cells", 400001),
+                                    ("half", 300007), ("half", 3000001), ("many groups", 4000000), ("half", 4500001)])
 def test_crowded_particles(ctx, kind, data, n):
     rng = np.random.default_rng(1600)
     p = _crowd(rng, data, n).astype(np.float32)
