@@ -1071,16 +1071,17 @@ __device__ __forceinline__ bool paired(const CountParams& p, const uint2* it, ui
     return dx * dx + dy * dy + dz * dz <= p.r2max;
 }
 
-// BY_WARPS: (also) the list of a count that gives a warp to each halo, whose
-// items may begin in a later part of their box.
+// BY_WARPS: the list of a count that gives a warp to each halo, whose items may
+// begin in a later part of their box (1 % of the time of heavy lists of lanes,
+// hence two kernels).
 template <int R, int BLOCKS, bool BY_WARPS>
 __global__ void __launch_bounds__(HV_THREADS, BLOCKS)
 k_listed_count(const __grid_constant__ CountParams p, const __grid_constant__ LaneParams q) {
     extern __shared__ uint32_t smem[];
     auto from = [](const uint2& it) { return BY_WARPS ? 32u * (it.y >> kItemFrom) : 0u; };
-    const bool whole = !BY_WARPS || (q.gate && *q.gate == 0u);  // lanes counted: all room was for either kind
-    const uint32_t nhuge = min(q.ctl[1], whole ? q.cap : q.cap_huge);
-    const uint32_t nother = min(q.ctl[2], whole ? q.cap : q.cap_other);
+    if (q.gate && (*q.gate != 0u) != BY_WARPS) return;
+    const uint32_t nhuge = min(q.ctl[1], BY_WARPS ? q.cap_huge : q.cap);
+    const uint32_t nother = min(q.ctl[2], BY_WARPS ? q.cap_other : q.cap);
     if (nhuge + nother == 0u) return;
     // Warps claim (two items, part); only huge items have several parts.  With
     // fewer items than warps each is claimed alone, and blocks beyond the last
@@ -1379,8 +1380,13 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
     SJCS_CUDA_TRY(allow_block_smem(k_lane_count<R, PACK>));
     k_lane_count<R, PACK><<<(unsigned)blocks, nw * 32, nw * warp_a + table, s>>>(p, q);
     SJCS_LAUNCH_CHECK();
-    return warps ? launch_listed<R, true>(ctx, p, q, given != nullptr, s)
-                 : launch_listed<R, false>(ctx, p, q, given != nullptr, s);
+    if (warps) {
+        LaneParams w = q;
+        w.left = nullptr;  // only lanes mark
+        const int rc = launch_listed<R, true>(ctx, p, w, given != nullptr, s);
+        if (rc) return rc;
+    }
+    return launch_listed<R, false>(ctx, p, q, given != nullptr, s);
 }
 }  // namespace
 
