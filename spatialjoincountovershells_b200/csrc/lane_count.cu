@@ -48,7 +48,9 @@
 // slots, measured), so staging the candidates would not pay.  What bounds it:
 // the L1/shared data pipe (75 % of its peak, 51 % issue active).
 //
-// k_listed_count runs at 68 % of both the data pipe and issue.
+// k_listed_count runs at 54 % of the data pipe's and 56 % of issue's peak (1e6
+// clustered halos on 2e7 particles, R = 20; 53 and 54 on 5e7): between them a
+// warp waits for its rows' loads.
 //
 // Measured (B200, count kernels of one call, warp-per-halo kernel -> this one):
 // 1e7 uniform halos on 1e8 particles, R = 5, 40 shells 6.66 -> 4.00 ms; 1e6 on
@@ -1310,7 +1312,8 @@ int launch_listed(sjcs_ctx* ctx, const CountParams& p, const LaneParams& q, bool
 // Most candidates of a lane's walk: a batch lasts as long as its longest lane,
 // so with few batches per SM long walks are left to the list (1e5 clustered
 // halos on 2e7 particles at R = 10, 1.3 waves: 1.06 ms without this, 0.78 with
-// it).  Quads of Morton cells hold a quarter more candidates than rows (1e6 x
+// it), but not below 160 (131072 x 20000, R = 40: 98 us a call with 96, 78 with
+// 160).  Quads of Morton cells hold a quarter more candidates than rows (1e6 x
 // 2e5 uniform at R = 20: 0.50 ms with 8, 0.35 with 10, 0.42 with 13).
 uint32_t walk_limit(sjcs_ctx* ctx, const CountParams& p, bool rows) {
     const uint64_t nbatch = (p.nhalos + 31) / 32, per = rows ? 8 : 10;

@@ -1,10 +1,10 @@
 // Persistent work-queue schedule, shared by the grid and Morton count kernels.
 //
-// A count kernel's estimate kernel gives every halo (Morton order) a size
+// A count kernel's estimate kernel gives every halo (in the query's order) a size
 // bucket (est_bucket of its estimated candidates) and a histogram of the
 // buckets; order_and_plan then
-//   sorts    one 8-bit radix pass by descending bucket (stable: Morton order
-//            within a bucket) -> ord[i] = Morton index
+//   sorts    one 8-bit radix pass by descending bucket (stable: the query's
+//            order within a bucket) -> ord[i] = place in the query
 //   plans    k_plan_items, per bucket (lower bound e of its estimates): halos
 //            with e >= piece are split into min(max_pieces, ceil(e/piece))
 //            pieces that separate warps count (every candidate set split

@@ -420,11 +420,11 @@ __global__ void __launch_bounds__(CT_THREADS, 8) k_shell_count_multi(CountParams
 
 // ---- persistent work-queue schedule -----------------------------------------
 //
-// k_estimate    per halo (Morton order): the number of candidates of its
+// k_estimate    per halo (in the query's order): the number of candidates of its
 //               clipped rows (times 2^k for k flagged periodic axes) and its
 //               size bucket (est_bucket, 8 bits); a histogram of the buckets
-// sort          one 8-bit radix pass by descending bucket (stable: Morton
-//               order within a bucket) -> ord[i] = Morton index
+// sort          one 8-bit radix pass by descending bucket (stable: the
+//               query's order within a bucket) -> ord[i] = place in the query
 // k_plan_items  per bucket (lower bound e of its estimates): halos with
 //               e >= piece are split into min(max_pieces, ceil(e/piece))
 //               pieces that separate warps count (every row set split

@@ -177,7 +177,7 @@ struct sjcs_query {
     float R;            // (float)sqrt((double)r2[nrads-1]), as MultiRangeCount.c:19
     float half;         // query half-width: R (periodic) or r2[nrads-1] (non-periodic, MultiRangeCount.c:81)
     float r2max;
-    float4* halos;      // Morton-sorted halos, .w = original index bits
+    float4* halos;      // grouped by Morton bucket (up to 4096: as given), .w = original index bits
     uint32_t* counts;   // [nhalos][nrads], caller's halo order
     // Behind them: two sets of control words and a list of images for counts
     // that give a warp to each halo (shell_count.cu, morton_count.cu).  A count
@@ -255,7 +255,7 @@ int launch_morton_count(sjcs_ctx* ctx, const sjcs_query* q, const sjcs_index* id
                         const Schedule* sc = nullptr);
 
 // sjcs_abi.cu: query preparation on stream s (radius table, shell lookup,
-// zeroed accumulators, Morton-sorted halos) and schedule resolution
+// zeroed accumulators, halos in Morton buckets) and schedule resolution
 int query_prepare(sjcs_ctx* ctx, const float* d_halo_xyz, size_t stride, uint64_t nhalos, const float* r2,
                   int nrads, int flags, sjcs_query* q, cudaStream_t s);
 // Counts that give a warp to each halo (lane_count.cu): items of a query's list,
