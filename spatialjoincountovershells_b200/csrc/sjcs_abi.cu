@@ -204,7 +204,10 @@ void build_shell_lut(const float* r2, int nrads, std::vector<uint32_t>* lut, uin
 // safe2: with d = p - c rounded per axis and the box bounds rounded from c -+
 // half, a particle outside the box on some axis has |d| >= (half - 2^-24 (|c|
 // + half)) (1 - 2^-24), so its fp32 distance is at least safe2 as computed
-// here for |c| <= cmax.  Slot j covers the keys [kbase + (j << shift), ... +
+// here for |c| <= cmax.  (It holds for any centre: rounding is monotone, so a
+// particle beyond the rounded bound is no nearer than half, and its distance no
+// less than half * half rounded.  Lanes test centres beyond cmax literally all
+// the same; images that warps list need no mark for it.)  Slot j covers the keys [kbase + (j << shift), ... +
 // (1 << shift)) and holds at most one of the thresholds (r2 below safe2, then
 // safe2); word j is (thresholds before the slot << shift) + (1 << shift) - low
 // bits of its threshold - (j << shift), so adding key - kbase leaves the slot's
