@@ -1204,14 +1204,16 @@ constexpr uint64_t kExactItems = 1u << 23;
 
 // List, control words and marks of a count on stream s.  A pool that cannot
 // give the whole list gives a shorter one, down to none.
-int alloc_list(StreamScratch& scr, const CountParams& p, LaneParams* q, cudaStream_t s) {
+int alloc_list(StreamScratch& scr, const CountParams& p, bool lean, LaneParams* q, cudaStream_t s) {
     const uint64_t n = p.nhalos * (uint64_t)p.nidx;
+    // a lean query's list stays within what a server admits a request with
+    const uint64_t part = n + (lean ? n / 4 : n / 2) + 1024;
     uint64_t cap = n * (p.periodic ? 8u : 1u), marks = 0;
     auto not_all = [&] {
-        cap = std::min<uint64_t>(n + n / 2 + 1024, 0xf0000000ull);
+        cap = std::min<uint64_t>(part, 0xf0000000ull);
         marks = (n + 1) / 2;
     };
-    if (cap > std::max(kExactItems, n + n / 2 + 1024) || cap > 0xf0000000ull) not_all();
+    if (cap > std::max(lean ? 0 : kExactItems, part) || cap > 0xf0000000ull) not_all();
     uint32_t* ctl = nullptr;
     for (;;) {
         const cudaError_t e =
@@ -1353,7 +1355,7 @@ int launch_ranges(sjcs_ctx* ctx, const sjcs_query* qq, const CountParams& p, cud
         q.list = given->list;
         q.cap = q.cap_huge = q.cap_other = given->cap;
     } else {
-        const int rc = alloc_list(scr, p, &q, s);
+        const int rc = alloc_list(scr, p, qq->lean, &q, s);
         if (rc) return rc;
     }
     q.huge = few_halos(ctx, p) ? kHugeFew : kHuge;
@@ -1399,9 +1401,9 @@ bool few_batches(const sjcs_ctx* ctx, uint64_t nhalos) {
 }
 }  // namespace
 
-// Most halos have an image or two that is listed, on one to three indexes.
+// An image or two of every halo on one to three indexes.
 uint32_t count_by_warps_items(const sjcs_ctx* ctx, uint64_t nhalos) {
-    return few_batches(ctx, nhalos) ? (uint32_t)std::min<uint64_t>(8 * nhalos, 131072) : 0u;
+    return few_batches(ctx, nhalos) ? (uint32_t)(4 * nhalos) : 0u;
 }
 
 // Boxes that lanes would walk: by the number of batches.  Fuller ones are all

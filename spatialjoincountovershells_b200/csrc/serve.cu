@@ -104,7 +104,7 @@ bool valid_server(const sjcs_server* s) { return s && s->magic == kServerMagic; 
 uint64_t request_bytes(uint64_t nhalos, size_t stride, int nrads) {
     // per halo: raw halo + ordered halo + counts, and 53 bytes of scratch: its
     // rank and share of the bucket counters (6 B) and the count's item list
-    // (14 B per index of a fused pass, up to 4; small ones up to 16 MB), or the queue schedule's keys
+    // (12 B per index of a fused pass, up to 4; 32 B if there are few), or the queue schedule's keys
     // and order (13 B); fixed: radius and lookup tables, scan partials
     return nhalos * (uint64_t)(stride + 16 + 40 + 4 * (uint64_t)nrads + 13) + 65536 + 8 * (uint64_t)nrads;
 }
@@ -122,6 +122,7 @@ int enqueue(sjcs_server* srv, Slot& sl) {
     const size_t raw_bytes = n ? (size_t)((n - 1) * r->stride + 12) : 16;
     SJCS_CUDA_TRY(cudaMallocAsync(&sl.d_raw, raw_bytes, s));
     if (n) SJCS_CUDA_TRY(cudaMemcpyAsync(sl.d_raw, r->halo_xyz, raw_bytes, cudaMemcpyHostToDevice, s));
+    sl.q.lean = true;
     int rc = query_prepare(srv->ctx, sl.d_raw, r->stride, n, r->r2.data(), nrads, r->flags, &sl.q, s);
     if (rc) return rc;
     if (n) {

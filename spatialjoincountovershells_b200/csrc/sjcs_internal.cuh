@@ -183,7 +183,8 @@ struct sjcs_query {
     // that give a warp to each halo (shell_count.cu, morton_count.cu).  A count
     // takes the sets in turn and clears the other one.
     uint32_t* list_ctl;
-    uint32_t list_items;  // even; 0: such counts do not occur
+    uint32_t list_items;  // 0: such counts do not occur
+    bool lean = false;    // the lane count's list takes 12 bytes per halo and index, however small
     mutable uint32_t list_turn;
     float* d_r2;        // [pad], entries past nrads = +inf
     // Shell lookup on the bit pattern of dist (non-negative floats order like
